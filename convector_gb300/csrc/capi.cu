@@ -116,6 +116,7 @@ struct cvx_scene {
     // read the caller's ray arrays in place. host_access: CVX_HOST_ACCESS_*.
     bool host_page_tables = false;
     bool slab_sel = false;  // DeviceScene::slab_sel
+    bool nested = false;    // DeviceScene::nested
     uint32_t host_access = CVX_HOST_ACCESS_AUTO;
     bool reads_host_in_place() const { return host_page_tables && host_access == CVX_HOST_ACCESS_AUTO; }
     // scratch for the host-buffer query
@@ -142,6 +143,7 @@ struct cvx_scene {
         s.general_pick = general_pick;
         s.depth = depth;
         s.slab_sel = slab_sel ? 1u : 0u;
+        s.nested = nested ? 1u : 0u;
         return s;
     }
     ~cvx_scene() {
@@ -323,6 +325,15 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
                 (hi == 0.0f && std::signbit(hi)))
                 s->slab_sel = false;
         }
+    s->nested = s->slab_sel;
+    for (uint32_t i = 0; i < n_nodes && s->nested; i++) {
+        if (nodes[i].len != 0) continue;
+        for (uint32_t k = 0; k < 2; k++) {
+            const cvx_bvh_node& child = nodes[nodes[i].index + k];
+            for (int c = 0; c < 3; c++)
+                if (child.origin[c] < nodes[i].origin[c] || child.far_[c] > nodes[i].far_[c]) s->nested = false;
+        }
+    }
     // Node pairs: q0 = lo0 hi0.x | q1 = hi0.yz lo1.xy | q2 = lo1.z hi1 | q3 = index/len x2
     // q3 holds the two children's stack references, the form the traversal
     // pushes (traverse.cuh): (index << 5) | len for internal nodes (len 0, index =

@@ -235,23 +235,27 @@ struct StagedSoaClaim {
 // shared, 0.890 with 4, 0.878 with 8, 0.883 with 12. (The wavefront and the
 // path-refill traversals, whose larger working sets need the L1 that the
 // carve-out takes, measured no gain or a loss.)
-// Traversal steps a lane takes per round of the warp's claim votes: 1, 3, 4
-// -> 0.798, 0.784, 0.777 ms per 4M rays of the 28-level icosphere (12 shared
-// stack entries) and 1.538, 1.503, 1.499 ms on the 70-level tube (medians of
-// three runs each; six steps: 0.774-0.778 and 1.474-1.482, within noise). The
-// claim thresholds, swept again at four steps, stay at 16 (12, 16, 20 on the
-// icosphere: 0.774-0.780, 0.776-0.778, 0.792-0.796 ms) and 8 for trees deeper
-// than 40 levels (6, 8, 12 on the tube: 1.499, 1.489-1.513, 1.493 ms). A leaf
-// reached from a pair tested in the same step (the frame kernels' form) is
-// slower here at 2, 3 and 4 steps: 0.84, 0.82-0.84, 0.82 ms on the icosphere.
-constexpr int kQuerySteps = 4;
+// Node pairs a lane walks per round of the warp's claim votes, before the
+// round's leaf test (RefillRay::walk; traversal steps, leaves included, in the
+// x86 form). The kernel is bound by instruction issue, and with a leaf tested
+// wherever a lane met one, the triangle code ran at nearly every step for one
+// or two lanes; once per round it runs for about eight. 3, 4, 5, 6, 8 pairs
+// per round: 4M rays of the 28-level icosphere 750, 724, 696, 717, 786 us (806
+// with leaves tested at once, four steps), 1M rays of the 70-level tube 531,
+// 539, 541, 557, 585 us (580), of the 19-level room 183, 175, 180, 182, 189 us
+// (198). The five walks unrolled: 696 -> 684, 543 -> 536, 181 -> 179 us. Ending
+// a round early when fewer than 8 to 20 lanes can walk on costs more in votes
+// than it saves: 748-794 us on the icosphere. The claim thresholds, swept again,
+// stay at 16 (12, 20, 24: 692, 733, 829 us) and 8 for trees deeper than 40
+// levels (6, 12, 16: 543, 542, 547 us).
+constexpr int kQuerySteps = 5;
 // The default; a scene may choose 0, 4 or 12 instead (cvx_scene_set_query_stack,
 // which the query autotuner sets per scene).
 constexpr int kQueryStackShared = 8;
 
-// SELECT: the select-form slab test for the rays that meet its conditions
-// (on scenes that do); the others are marked kDeferredRay and traced by
-// k_intersect_deferred. Measured on 4M rays: 0.844 against 0.877 ms.
+// SELECT: the select-form slab test and postponed leaves for the rays that
+// meet the conditions (on scenes that do); the others are marked kDeferredRay
+// and traced by k_intersect_deferred.
 // SHARED: stack entries of each lane in shared memory (the rest in local).
 template <int MINB, bool COUNT, int CLAIM, bool SELECT, int SHARED = kQueryStackShared>
 __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uint32_t* __restrict__ next_ray,
@@ -519,13 +523,15 @@ struct FramePaths {
 // room (5k triangles), the 82k-triangle icosphere and the 870k-triangle tube at
 // 1280x736: 7 resident blocks per SM (72 registers, no spill; 8 blocks spill
 // and lose 2-7 %), and a leaf reached from a pair tested in the same step.
-// Trees up to 40 levels: claim threshold 16 and three traversal steps per
-// round of votes, swept with the select-form rounds in place (room 0.711 ->
-// 0.701-0.704 ms, icosphere 1.42 -> 1.40-1.41 ms against two steps; four
-// steps 0.733 and 1.46; claim 12 or 20 at three steps: room 0.751 or 0.694,
-// icosphere 1.412 or 1.432). Deeper trees: below (kDeepFrame*).
+// Trees up to 40 levels: claim threshold 16 and five node pairs per round with
+// the leaves they lead to tested once, at its end (RefillRay::walk). 2, 3, 4,
+// 5, 6 pairs per round: 82k icosphere at 1920x1080 2.53, 2.40, 2.32, 2.31,
+// 2.32 ms (2.79 with leaves tested at once, three steps); room 1280x736 0.61 ms
+// at five (0.70). At five: claim 12, 20, 24 icosphere 2.31, 2.41, 2.58 ms, room
+// 0.63, 0.60, 0.61; 6 and 8 blocks per SM 2.44, 2.36 and 0.61, 0.65; the walks
+// unrolled 2.44 and 0.65 (instruction fetch). Deeper trees: below (kDeepFrame*).
 constexpr int kRefillFrameBlocksPerSm = 7;
-constexpr int kRefillFrameSteps = 3;
+constexpr int kRefillFrameSteps = 5;
 
 // COUNT: the same frame, also counting its work (FrameArgs::work); the
 // counters cost registers, so frames are rendered without them.
@@ -539,13 +545,13 @@ constexpr int kRefillFrameSteps = 3;
 // the same entries cost 3-4 %.
 constexpr int kDeepFrameStackShared = 16;
 
-// Deep trees: claim threshold 8 and three traversal steps per round of votes
-// (tube, ms per sample: claim 6, 8, 10, 12 -> 3.01, 2.98, 2.97, 2.99 at two
-// steps; steps 1, 2, 3, 4 -> 3.15, 2.98, 2.93, 3.07 at claim 8; 6 and 8
-// resident blocks per SM instead of 7 -> 3.07 and 2.97, the latter with 64
-// registers and a 76-byte spill).
+// Deep trees: claim threshold 8 and four node pairs per round. 870k tube,
+// 1280x736, 16 samples in one launch: 2, 3, 4, 5, 6 pairs per round -> 30.6,
+// 29.4, 28.7, 29.1, 29.9 ms (35.7 with leaves tested at once, three steps);
+// at five, claim 6, 12, 16 -> 29.7, 29.2, 30.5 ms; 6 and 8 resident blocks
+// per SM 30.6 and 30.3 ms.
 constexpr int kDeepFrameClaim = 8;
-constexpr int kDeepFrameSteps = 3;
+constexpr int kDeepFrameSteps = 4;
 // DEEP: a tree deeper than 40 levels (shared stack entries, the constants above).
 // MULTI: a.samples samples in one launch (FramePaths<true>).
 template <bool DEEP, bool COUNT, bool MULTI = false>
@@ -746,7 +752,7 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
         if (blocks > need) blocks = need;
         SoaRays src{s.nodes, s.geom, rays, n, far_dist, t_out, tri_out, counters};
         bool deep = s.depth > 40;
-        const bool sel = s.slab_sel != 0u && !counters;
+        const bool sel = s.slab_sel != 0u && s.nested != 0u && !counters;
         if (counters) k_intersect_refill<8, true, 16, false><<<blocks, 128, 0, st>>>(src, err + 1, err);
         else if (!sel) {  // x86-form slab test throughout
             if (deep) k_intersect_refill<8, false, 8, false><<<blocks, 128, 0, st>>>(src, err + 1, err);

@@ -37,6 +37,9 @@ struct DeviceScene {
     // Every node bound is finite, lo <= hi on each axis and none is -0: the
     // ray-cast kernel may take the select-form slab test (box_test_sel).
     uint32_t slab_sel;
+    // Every node's bounds lie inside its parent's (true of every built tree):
+    // with slab_sel, rays may be traced with postponed leaves (RefillRay::walk).
+    uint32_t nested;
 };
 
 struct DeviceCamera {

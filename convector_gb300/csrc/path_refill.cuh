@@ -5,8 +5,7 @@
 //
 // Each lane takes one path at a time from a counter (path p is lane p & 7 of
 // group p >> 3) and carries it through its bounces; every round a lane tracing
-// a ray processes up to STEPS node pairs or leaves of it (RefillRay). A lane
-// whose ray is finished waits until CLAIM_MIN lanes of its warp are in that
+// a ray processes up to STEPS node pairs of it (RefillRay). A lane whose ray is finished waits until CLAIM_MIN lanes of its warp are in that
 // state (or none is tracing); those lanes then shade together: the hit record,
 // continue_path, and either the next bounce's ray or the pixel's store and a
 // new path with its camera ray. Warps thus stay busy while paths of 1 to 5
@@ -43,12 +42,11 @@
 
 namespace cvx {
 
-// SELECT_ROUNDS: each round's traversal steps take the select-form slab test
-// when every tracing lane's ray allows it (a warp-uniform choice, so neither
-// form's code runs for the other's lanes), the x86 form otherwise. Measured
-// for the frame kernel: 1280x736 tube 3.11 -> 3.08 ms, room 0.714 -> 0.704 ms,
-// icosphere 1.44 -> 1.42 ms (the wave kernel, whose scene table costs
-// registers, would spill 10 bytes more).
+// SELECT_ROUNDS: a round walks STEPS node pairs with the select-form slab test
+// and tests the leaves they led to once, at its end (RefillRay::walk), when
+// every tracing lane's ray allows it (a warp-uniform choice, so neither form's
+// code runs for the other's lanes); otherwise it takes STEPS steps in the x86
+// form. Each lane's results are the same either way.
 template <int CLAIM_MIN, int STEPS, bool COUNT = false, bool SELECT_ROUNDS = false, int SHARED_STACK = 0,
           class Paths>
 __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, uint2* shared_stack = nullptr) {
@@ -62,6 +60,8 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
     ray.top = make_uint2(0u, 0u);
     ray.sp = 0;
     ray.cur = RefillRay::kNone;
+    ray.leaf = 0u;
+    ray.cur_t = 0.0f;
     ray.na = ray.nt = 0;
     ray.nodes = ray.geom = nullptr;
     ray.o = ray.d = ray.inv = f3(0, 0, 0);
@@ -120,7 +120,7 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
             } else {
                 bounce++;
                 ray.start(n.o, n.d, 1.0e5f, s.nodes, s.geom, tab);
-                ray_sel = SELECT_ROUNDS && s.slab_sel && select_form_ray(ray.inv);
+                ray_sel = SELECT_ROUNDS && s.slab_sel && s.nested && select_form_ray(ray.inv);
                 tracing = true;
                 P.count_ray(ref);
             }
@@ -142,7 +142,7 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
                     if (P.begin(p, ref, o, d, rng, tab)) {  // else: a group outside its image; take another path
                         const DeviceScene s = P.scene(ref);
                         ray.start(o, d, 1.0e5f, s.nodes, s.geom, tab);
-                        ray_sel = SELECT_ROUNDS && s.slab_sel && select_form_ray(ray.inv);
+                        ray_sel = SELECT_ROUNDS && s.slab_sel && s.nested && select_form_ray(ray.inv);
                         color = f3(1.0f, 1.0f, 1.0f);
                         bounce = 0u;
                         has_path = true;
@@ -153,10 +153,14 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
             }
         }
         if (__all_sync(0xffffffffu, done)) break;
-        if (SELECT_ROUNDS && __all_sync(0xffffffffu, !tracing || ray_sel)) {
-            for (int st = 0; st < STEPS && tracing; st++)
-                if (ray.step<COUNT, true, SELECT_ROUNDS>(stack, overflow)) tracing = false;
+        if (SELECT_ROUNDS && !COUNT && __all_sync(0xffffffffu, !tracing || ray_sel)) {
+            if (tracing) {
+#pragma unroll 1
+                for (int st = 0; st < STEPS; st++) ray.walk(stack, overflow);
+                if (ray.test_leaf()) tracing = false;
+            }
         } else {
+            if (SELECT_ROUNDS && !COUNT) ray.settle();
             for (int st = 0; st < STEPS && tracing; st++)
                 if (ray.step<COUNT, true>(stack, overflow)) tracing = false;
         }

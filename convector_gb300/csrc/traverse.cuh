@@ -263,6 +263,8 @@ struct RefillRay {
     uint2 top;
     int sp;
     uint32_t cur;  // ref of the node to process; kNone: pop
+    uint32_t leaf;  // walk(): ref of the leaf to test; 0: none
+    float cur_t;    // entry distance of cur
     uint32_t na, nt;
 
     __device__ __forceinline__ void start(F3 o_, F3 d_, float far, const float4* nodes_, const float4* geom_,
@@ -277,6 +279,8 @@ struct RefillRay {
         na = 2;
         nt = 0;
         cur = 0;  // the root pair: internal ref with index 0
+        leaf = 0u;
+        cur_t = __int_as_float(0xff800000);  // the roots are never culled (bvh.rs:604-634)
     }
 
     // The leaf loops are not unrolled: len is bounded by its 5 bits, and the
@@ -285,9 +289,8 @@ struct RefillRay {
     //
     // Returns true when the ray is finished (its stack is empty): h is then
     // its nearest hit. Sets `overflow` (and finishes the ray) when the stack
-    // would overflow. SELECT: the slab test in select form (box_test_sel; the
-    // scene and the ray must meet its conditions).
-    template <bool COUNT, bool LEAF_AFTER_PAIR, bool SELECT = false, class Stack>
+    // would overflow.
+    template <bool COUNT, bool LEAF_AFTER_PAIR, class Stack>
     __device__ __forceinline__ bool step(Stack& stack, bool& overflow) {
         if (cur == kNone) {
             // Pop until an entry survives the cull test (aabb.rs:171-177).
@@ -296,6 +299,7 @@ struct RefillRay {
                 if (--sp > 0) top = stack.load(sp - 1);
                 if (!geq(__uint_as_float(e.y), h.t)) {
                     cur = e.x;
+                    cur_t = __uint_as_float(e.y);
                     break;
                 }
             }
@@ -318,14 +322,8 @@ struct RefillRay {
             // the child pair (64 bytes per pair).
             const float4* np = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + cur);
             float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
-            BoxT b0, b1;
-            if constexpr (SELECT) {
-                b0 = box_test_sel(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
-                b1 = box_test_sel(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
-            } else {
-                b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
-                b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
-            }
+            const BoxT b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
+            const BoxT b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
             bool first0 = !sneg(b0.tmin - b1.tmin);
             bool hit0 = b0.mask & !sneg(b0.tmax);
             bool hit1 = b1.mask & !sneg(b1.tmax);
@@ -346,6 +344,7 @@ struct RefillRay {
                 sp++;
             }
             cur = (hit_second && !geq(t_second, h.t)) ? ref_second : kNone;
+            cur_t = t_second;
             if (!LEAF_AFTER_PAIR || cur == kNone) return false;
             len = cur & 31u;
             idx = cur >> 5;
@@ -360,6 +359,98 @@ struct RefillRay {
             cur = kNone;
         }
         return false;
+    }
+
+    // The same traversal with the leaf tests postponed (select form): walk()
+    // goes on from node pair to node pair while at most one leaf waits in
+    // `leaf`, and test_leaf() tests that leaf's triangles. A warp alternates a
+    // few walk() steps with one test_leaf(), so the triangle code runs once per
+    // round for all lanes that reached a leaf in it, not at nearly every step
+    // for one or two lanes.
+    //
+    // The results are those of step(): a node walked on to before the waiting
+    // leaf was tested may be one that step(), knowing the leaf's hit, would have
+    // culled (entry distance t at or beyond the hit). Its children then have
+    // entry distances of at least t: their bounds lie inside the node's
+    // (DeviceScene::nested), and differences, products and the minima and maxima
+    // of the slab test are monotonic in the bounds, for finite values. So they
+    // are culled when they are popped, or by test_leaf() where one is `cur`, and
+    // no triangle is tested that step() does not test, nor in another order. Box
+    // tests do not depend on the hit distance. (With the stack limit lowered, a
+    // push below such a node can overflow.)
+    //
+    // Does nothing when the stack is empty or the next node is a leaf and one
+    // waits already.
+    template <class Stack>
+    __device__ __forceinline__ void walk(Stack& stack, bool& overflow) {
+        while (cur == kNone && sp > 0) {
+            uint2 e = top;
+            if (--sp > 0) top = stack.load(sp - 1);
+            if (!geq(__uint_as_float(e.y), h.t)) {
+                if ((e.x & 31u) != 0u && leaf == 0u) {
+                    leaf = e.x;
+                } else {
+                    cur = e.x;
+                    cur_t = __uint_as_float(e.y);
+                }
+            }
+        }
+        if ((cur & 31u) != 0u) return;  // nothing left, or a second leaf
+        const float4* np = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + cur);
+        float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
+        const BoxT b0 = box_test_sel(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
+        const BoxT b1 = box_test_sel(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
+        const bool first0 = !sneg(b0.tmin - b1.tmin);
+        const bool hit0 = b0.mask & !sneg(b0.tmax);
+        const bool hit1 = b1.mask & !sneg(b1.tmax);
+        const uint32_t r0 = __float_as_uint(q3.x), r1 = __float_as_uint(q3.y);
+        // The reference pushes `first` then `second` and pops `second` first.
+        const bool hit_first = first0 ? hit0 : hit1, hit_second = first0 ? hit1 : hit0;
+        const uint32_t ref_first = first0 ? r0 : r1, ref_second = first0 ? r1 : r0;
+        const float t_first = first0 ? b0.tmin : b1.tmin, t_second = first0 ? b1.tmin : b0.tmin;
+        if (sp + (int)hit_first + (int)hit_second > c_stack_limit) {
+            overflow = true;
+            sp = 0;
+            cur = kNone;
+            leaf = 0u;
+            return;
+        }
+        if (hit_first) {
+            if (sp > 0) stack.store(sp - 1, top);
+            top = make_uint2(ref_first, __float_as_uint(t_first));
+            sp++;
+        }
+        cur = (hit_second && !geq(t_second, h.t)) ? ref_second : kNone;
+        cur_t = t_second;
+        if (cur != kNone && (cur & 31u) != 0u && leaf == 0u) {
+            leaf = cur;
+            cur = kNone;
+        }
+    }
+    // Tests the waiting leaf, if any, and drops `cur` if its hit culls it.
+    // Returns true when the ray is finished.
+    __device__ __forceinline__ bool test_leaf() {
+        if (leaf != 0u) {
+            uint32_t len = leaf & 31u, idx = leaf >> 5;
+            leaf_range(nodes, idx, len);
+#pragma unroll 1
+            for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o, d, true, h);
+            leaf = 0u;
+            if (geq(cur_t, h.t)) cur = kNone;
+            if (cur != kNone && (cur & 31u) != 0u) {  // the second leaf is next
+                leaf = cur;
+                cur = kNone;
+            }
+        }
+        return cur == kNone && sp == 0 && leaf == 0u;
+    }
+    // From postponed leaves back to step(): after test_leaf() a waiting leaf is
+    // the next node.
+    __device__ __forceinline__ void settle() {
+        if (leaf != 0u) {
+            cur = leaf;
+            leaf = 0u;
+        }
     }
 };
 
@@ -383,10 +474,11 @@ __device__ __forceinline__ typename std::conditional<N == 0, LocalStack, SharedL
 // not depend on it (each ray's traversal is independent of when it starts).
 // Returns false if a ray overflowed the stack (its hit is then incomplete).
 // SELECT: every ray whose reciprocals meet select_form_ray is traversed with
-// the select-form slab test; the others are handed to src.defer(r) untraced
-// (the caller traces them afterwards with the x86 form). STEPS: traversal
-// steps per round of the warp's votes (a lane whose ray ends within a round
-// waits for the next round's claim).
+// the select-form slab test and postponed leaves (RefillRay::walk); the others
+// are handed to src.defer(r) untraced (the caller traces them afterwards with
+// the x86 form). STEPS: node pairs (SELECT) or traversal steps per round of the
+// warp's votes (a lane whose ray ends within a round waits for the next
+// round's claim).
 template <bool COUNT, bool LEAF_AFTER_PAIR, int CLAIM_MIN, int SHARED_STACK = 0, bool SELECT = false, int STEPS = 1,
           class Src, class Claim>
 __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, const ApproxTables& tab,
@@ -399,6 +491,8 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
     ray.top = make_uint2(0u, 0u);
     ray.sp = 0;
     ray.cur = 0;
+    ray.leaf = 0u;
+    ray.cur_t = 0.0f;
     ray.na = ray.nt = 0;
     ray.nodes = ray.geom = nullptr;
     ray.o = ray.d = ray.inv = f3(0, 0, 0);
@@ -434,10 +528,21 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
             }
         }
         if (__all_sync(0xffffffffu, done)) break;
-        for (int st = 0; st < STEPS && have; st++) {
-            if (ray.step<COUNT, LEAF_AFTER_PAIR, SELECT>(stack, overflow)) {
-                src.store(r_id, ray.h, ray.na, ray.nt);
-                have = false;
+        if constexpr (SELECT) {
+            if (have) {
+#pragma unroll
+                for (int st = 0; st < STEPS; st++) ray.walk(stack, overflow);
+                if (ray.test_leaf()) {
+                    src.store(r_id, ray.h, 0u, 0u);
+                    have = false;
+                }
+            }
+        } else {
+            for (int st = 0; st < STEPS && have; st++) {
+                if (ray.step<COUNT, LEAF_AFTER_PAIR>(stack, overflow)) {
+                    src.store(r_id, ray.h, ray.na, ray.nt);
+                    have = false;
+                }
             }
         }
     }

@@ -508,11 +508,18 @@ struct WavePaths {
 // loop form as the frame kernel's (k_render_refill).
 // 7 resident blocks per SM (72 registers and a small spill): 6 (80 registers,
 // no spill) served the 415-request mix at 2,014 against 2,083 Mrays/s.
+// With postponed leaves (below) again: 6 blocks 2,744 against 2,869 Mrays/s.
 constexpr int kRefillWaveBlocksPerSm = 7;
+// Node pairs a lane walks per round. With postponed leaves (RefillRay::walk),
+// whose rounds test their leaves once, five; against the x86-form rounds of
+// two steps before, a served 1280x736 request of 16 samples takes: room 11.2 ->
+// 9.5 ms, 82k icosphere 20.7 -> 17.3 ms, 870k tube 38.2 -> 31.4 ms, although
+// the spill grows from 82-94 to 112-120 bytes (three steps: 9.7, 17.8, 31.3).
+constexpr int kRefillWaveSteps = 5;
 // As the frame kernel: waves whose trees are deeper than 40 levels keep the
 // first 16 stack entries of each lane in shared memory and read the tables
 // from global memory (4 tube views of 1280x736, 2 samples: 21.5 -> 20.3 ms;
-// 12 entries 20.5 ms; three or four steps per round 20.3, 22.5 ms).
+// 12 entries 20.5 ms).
 constexpr int kDeepWaveStackShared = 16;
 template <int CLAIM_MIN, bool SLOTS = false>
 __global__ void __launch_bounds__(128, kRefillWaveBlocksPerSm) k_wave_refill(const Job* __restrict__ jobs,
@@ -524,12 +531,12 @@ __global__ void __launch_bounds__(128, kRefillWaveBlocksPerSm) k_wave_refill(con
     bool ok;
     if constexpr (kShared > 0) {
         __shared__ uint2 sstack[4][kShared][32];
-        ok = path_refill<CLAIM_MIN, 2, false, false, kShared>(P, g_tables_wf,
+        ok = path_refill<CLAIM_MIN, kRefillWaveSteps, false, true, kShared>(P, g_tables_wf,
                                                                &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
     } else {
         __shared__ ApproxTables tab;
         load_tables_wf(tab);
-        ok = path_refill<CLAIM_MIN, 2>(P, tab);  // three steps: room waves 5.24 -> 5.34 ms
+        ok = path_refill<CLAIM_MIN, kRefillWaveSteps, false, true>(P, tab);
     }
     if (!ok) atomicOr(out.err, kErrStackOverflow);
 }
