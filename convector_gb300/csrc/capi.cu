@@ -116,7 +116,7 @@ struct cvx_scene {
     // read the caller's ray arrays in place. host_access: CVX_HOST_ACCESS_*.
     bool host_page_tables = false;
     bool slab_sel = false;  // DeviceScene::slab_sel
-    bool nested = false;    // DeviceScene::nested
+    float4* d_wide = nullptr;  // DeviceScene::wide
     uint32_t host_access = CVX_HOST_ACCESS_AUTO;
     bool reads_host_in_place() const { return host_page_tables && host_access == CVX_HOST_ACCESS_AUTO; }
     // scratch for the host-buffer query
@@ -143,11 +143,12 @@ struct cvx_scene {
         s.general_pick = general_pick;
         s.depth = depth;
         s.slab_sel = slab_sel ? 1u : 0u;
-        s.nested = nested ? 1u : 0u;
+        s.wide = d_wide;
         return s;
     }
     ~cvx_scene() {
         cudaFree(d_nodes);
+        cudaFree(d_wide);
         cudaFree(d_geom);
         cudaFree(d_shade);
         cudaFree(d_lights);
@@ -315,24 +316,26 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     if ((st = dalloc(&s->d_shade, n_tris, "shading data"))) return st;
     if ((st = dalloc(&s->d_lights, (size_t)s->n_lights * 5, "lights"))) return st;
     if ((st = dalloc(&s->d_err, 2, "status"))) return st;  // [0] status, [1] ray counter
-    // The select-form slab test (box_test_sel) needs every bound finite and
-    // ordered, and none -0.
+    // The select-form slab test (box_test_sel) needs every bound at most
+    // kSelectMax in magnitude and ordered, and none -0.
     s->slab_sel = true;
     for (uint32_t i = 0; i < n_nodes && s->slab_sel; i++)
         for (int c = 0; c < 3; c++) {
             const float lo = nodes[i].origin[c], hi = nodes[i].far_[c];
-            if (!std::isfinite(lo) || !std::isfinite(hi) || !(lo <= hi) || (lo == 0.0f && std::signbit(lo)) ||
+            if (!(std::fabs(lo) <= 1.0e18f) || !(std::fabs(hi) <= 1.0e18f) || !(lo <= hi) || (lo == 0.0f && std::signbit(lo)) ||
                 (hi == 0.0f && std::signbit(hi)))
                 s->slab_sel = false;
         }
-    s->nested = s->slab_sel;
-    for (uint32_t i = 0; i < n_nodes && s->nested; i++) {
+    // The wide records need every node's bounds to be exactly the enclosure of
+    // its children's, as the build makes them.
+    bool tight = s->slab_sel;
+    for (uint32_t i = 0; i < n_nodes && tight; i++) {
         if (nodes[i].len != 0) continue;
-        for (uint32_t k = 0; k < 2; k++) {
-            const cvx_bvh_node& child = nodes[nodes[i].index + k];
-            for (int c = 0; c < 3; c++)
-                if (child.origin[c] < nodes[i].origin[c] || child.far_[c] > nodes[i].far_[c]) s->nested = false;
-        }
+        const cvx_bvh_node &c0 = nodes[nodes[i].index], &c1 = nodes[nodes[i].index + 1];
+        for (int c = 0; c < 3; c++)
+            if (std::min(c0.origin[c], c1.origin[c]) != nodes[i].origin[c] ||
+                std::max(c0.far_[c], c1.far_[c]) != nodes[i].far_[c])
+                tight = false;
     }
     // Node pairs: q0 = lo0 hi0.x | q1 = hi0.yz lo1.xy | q2 = lo1.z hi1 | q3 = index/len x2
     // q3 holds the two children's stack references, the form the traversal
@@ -369,6 +372,10 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     CK(cudaMemcpyAsync(s->d_nodes, node_buf.data(), node_buf.size() * sizeof(float4), cudaMemcpyHostToDevice,
                        s->stream),
        "upload nodes");
+    if (tight && depth <= kWideMaxDepth) {
+        if ((st = dalloc(&s->d_wide, (size_t)n_nodes / 2 * 8, "wide nodes"))) return st;
+        CK(launch_prep_wide(s->d_nodes + s->node_offset, n_nodes / 2, s->d_wide, s->stream), "wide nodes");
+    }
     cvx_triangle* d_src = nullptr;
     uint32_t* d_ds = nullptr;
     if ((st = dalloc(&d_src, n_tris, "staging"))) return st;

@@ -47,6 +47,44 @@ __global__ void k_prep_geom(const cvx_triangle* __restrict__ tris, uint32_t n, f
     }
 }
 
+// The wide records (traverse.cuh) of a scene's node pairs.
+__global__ void k_prep_wide(const float4* __restrict__ nodes, uint32_t n_pairs, float4* __restrict__ wide) {
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n_pairs; p += gridDim.x * blockDim.x) {
+        const float4* np = nodes + 4 * (size_t)p;
+        const float4 q0 = np[0], q1 = np[1], q2 = np[2], q3 = np[3];
+        const float own[2][6] = {{q0.x, q0.y, q0.z, q0.w, q1.x, q1.y}, {q1.z, q1.w, q2.x, q2.y, q2.z, q2.w}};
+        const uint32_t own_ref[2] = {__float_as_uint(q3.x), __float_as_uint(q3.y)};
+        float b[4][6];
+        uint32_t ref[4];
+        for (int c = 0; c < 2; c++) {
+            if ((own_ref[c] & 31u) == 0u) {  // internal: its children's boxes
+                const float4* cp = nodes + 4 * (size_t)(own_ref[c] >> 6);
+                const float4 c0 = cp[0], c1 = cp[1], c2 = cp[2], c3 = cp[3];
+                const float kids[2][6] = {{c0.x, c0.y, c0.z, c0.w, c1.x, c1.y}, {c1.z, c1.w, c2.x, c2.y, c2.z, c2.w}};
+                for (int k = 0; k < 2; k++)
+                    for (int a = 0; a < 6; a++) b[2 * c + k][a] = kids[k][a];
+                ref[2 * c] = __float_as_uint(c3.x);
+                ref[2 * c + 1] = __float_as_uint(c3.y);
+            } else {
+                for (int a = 0; a < 6; a++) {
+                    b[2 * c][a] = own[c][a];
+                    b[2 * c + 1][a] = a < 3 ? kEmptyLo : -kEmptyLo;
+                }
+                ref[2 * c] = own_ref[c];
+                ref[2 * c + 1] = 0u;
+            }
+        }
+        float4* w = wide + 8 * (size_t)p;
+        for (int a = 0; a < 3; a++) {
+            w[2 * a] = make_float4(b[0][a], b[1][a], b[2][a], b[3][a]);
+            w[2 * a + 1] = make_float4(b[0][a + 3], b[1][a + 3], b[2][a + 3], b[3][a + 3]);
+        }
+        w[6] = make_float4(__uint_as_float(ref[0]), __uint_as_float(ref[1]), __uint_as_float(ref[2]),
+                           __uint_as_float(ref[3]));
+        w[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
+
 // LightRec (5 x float4): v0 area | e1 rnorm | e2 - | n - | normal -
 __global__ void k_prep_lights(const cvx_triangle* __restrict__ tris, const uint32_t* __restrict__ ds, uint32_t n,
                               float4* __restrict__ lights) {
@@ -105,7 +143,7 @@ __global__ void __launch_bounds__(256) k_intersect(DeviceScene s, const RayCols 
         // decided once per packet outside the traversal loop (4M random rays:
         // 3.05 -> 2.92 ms; the same results).
         const bool sel = PACKET && s.slab_sel && !counters &&
-                         oct_all(omask, select_form_ray(f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab))));
+                         oct_all(omask, select_form_ray(o, f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab))));
         if (sel) ok = traverse<true, true>(s, o, d, active, omask, h, tab, nullptr);
         else if (PACKET || active) ok = traverse<PACKET>(s, o, d, active, omask, h, tab, counters ? &c : nullptr);
         if (!ok) atomicOr(err, kErrStackOverflow);
@@ -125,6 +163,7 @@ constexpr int32_t kDeferredRay = -2;  // never a hit index: -1 is the miss
 // Ray source of the isolated nearest-hit query: SoA rays in, (t, index) out.
 struct SoaRays {
     const float4* nodes;
+    const float4* wide;
     const float4* geom;
     RayCols rays;
     uint32_t n;
@@ -140,6 +179,11 @@ struct SoaRays {
         d = f3(__ldg(rays.c[3] + r), __ldg(rays.c[4] + r), __ldg(rays.c[5] + r));
         far = far_dist;
         return true;
+    }
+    __device__ __forceinline__ void first_scene(const float4*& nd, const float4*& wd, const float4*& gm) const {
+        nd = nodes;
+        wd = wide;
+        gm = geom;
     }
     // A ray left to k_intersect_deferred (its index word holds kDeferredRay).
     __device__ __forceinline__ void defer(uint32_t r) const { tri_out[r] = kDeferredRay; }
@@ -202,6 +246,7 @@ struct StagedSoaClaim {
                 in.d = f3(buf[which][3][slot], buf[which][4][slot], buf[which][5][slot]);
                 in.far = src.far_dist;
                 in.nodes = src.nodes;
+                in.wide = src.wide;
                 in.geom = src.geom;
                 res = kClaimRay;
             } else {
@@ -235,20 +280,21 @@ struct StagedSoaClaim {
 // shared, 0.890 with 4, 0.878 with 8, 0.883 with 12. (The wavefront and the
 // path-refill traversals, whose larger working sets need the L1 that the
 // carve-out takes, measured no gain or a loss.)
-// Node pairs a lane walks per round of the warp's claim votes, before the
+// Wide records a lane walks per round of the warp's claim votes, before the
 // round's leaf test (RefillRay::walk; traversal steps, leaves included, in the
-// x86 form). The kernel is bound by instruction issue, and with a leaf tested
-// wherever a lane met one, the triangle code ran at nearly every step for one
-// or two lanes; once per round it runs for about eight. 3, 4, 5, 6, 8 pairs
-// per round: 4M rays of the 28-level icosphere 750, 724, 696, 717, 786 us (806
-// with leaves tested at once, four steps), 1M rays of the 70-level tube 531,
-// 539, 541, 557, 585 us (580), of the 19-level room 183, 175, 180, 182, 189 us
-// (198). The five walks unrolled: 696 -> 684, 543 -> 536, 181 -> 179 us. Ending
-// a round early when fewer than 8 to 20 lanes can walk on costs more in votes
-// than it saves: 748-794 us on the icosphere. The claim thresholds, swept again,
-// stay at 16 (12, 20, 24: 692, 733, 829 us) and 8 for trees deeper than 40
-// levels (6, 12, 16: 543, 542, 547 us).
-constexpr int kQuerySteps = 5;
+// x86 form). The kernel is bound by instruction issue and the ALU pipe: with a
+// leaf tested wherever a lane met one, the triangle code ran at nearly every
+// step for one or two lanes; once per round it runs for about eight. A wide
+// record replaces two to three pair steps (7.0 records against 13.2 pairs per
+// random ray of the icosphere). 4M rays of the 28-level icosphere, 1M of the
+// 70-level tube, 1M of the 19-level room: leaves at once 792, 580, 198 us;
+// postponed, five pairs per round 684, 536, 179; records with the planes
+// selected in registers 718, 522, 160; selected by address 673, 505, 155; and
+// two planes per instruction 643, 490, 149; with the spare stack entry and one
+// limit check per record 608, 468, 146. Two, three, four records per round:
+// 615, 605, 719; 472, 475, 546; 145, 146, 168 us. Ending a round early when few
+// lanes can walk on costs more in votes than it saves (748-794 us with pairs).
+constexpr int kQuerySteps = 2;
 // The default; a scene may choose 0, 4 or 12 instead (cvx_scene_set_query_stack,
 // which the query autotuner sets per scene).
 constexpr int kQueryStackShared = 8;
@@ -296,10 +342,10 @@ __global__ void __launch_bounds__(256) k_intersect_deferred(SoaRays src, uint32_
         const float4 *nodes, *geom;
         src.load(r, o, d, far, nodes, geom);
         RefillRay ray;
-        uint2 local_stack[kStackDepth];
+        uint2 local_stack[kStackSlots];
         LocalStack stack{local_stack};
         ray.top = make_uint2(0u, 0u);
-        ray.start(o, d, far, nodes, geom, g_tables);
+        ray.start(o, d, far, nodes, nullptr, geom, g_tables);
         bool overflow = false;
         while (!ray.step<false, false>(stack, overflow)) {
         }
@@ -472,6 +518,11 @@ struct FramePaths {
         camera_ray(a.cam, x, y, unit_from(rng.next()), tab, o, d);
         return true;
     }
+    __device__ __forceinline__ void first_scene(const float4*& nd, const float4*& wd, const float4*& gm) const {
+        nd = a.s.nodes;
+        wd = a.s.wide;
+        gm = a.s.geom;
+    }
     __device__ __forceinline__ DeviceScene scene(const PathRef&) const { return a.s; }
     __device__ __forceinline__ bool last(const PathRef& r) const { return !MULTI || r.smp + 1u == a.samples; }
     __device__ __forceinline__ void gbuffer(const PathRef& r, uint32_t word) {
@@ -523,15 +574,16 @@ struct FramePaths {
 // room (5k triangles), the 82k-triangle icosphere and the 870k-triangle tube at
 // 1280x736: 7 resident blocks per SM (72 registers, no spill; 8 blocks spill
 // and lose 2-7 %), and a leaf reached from a pair tested in the same step.
-// Trees up to 40 levels: claim threshold 16 and five node pairs per round with
-// the leaves they lead to tested once, at its end (RefillRay::walk). 2, 3, 4,
-// 5, 6 pairs per round: 82k icosphere at 1920x1080 2.53, 2.40, 2.32, 2.31,
-// 2.32 ms (2.79 with leaves tested at once, three steps); room 1280x736 0.61 ms
-// at five (0.70). At five: claim 12, 20, 24 icosphere 2.31, 2.41, 2.58 ms, room
-// 0.63, 0.60, 0.61; 6 and 8 blocks per SM 2.44, 2.36 and 0.61, 0.65; the walks
-// unrolled 2.44 and 0.65 (instruction fetch). Deeper trees: below (kDeepFrame*).
+// Trees up to 40 levels: claim threshold 16 and two wide records per round with
+// the leaves they lead to tested once, at its end (RefillRay::walk): 82k
+// icosphere at 1920x1080 2.02 ms, room 1280x736 0.476 ms (2.79 and 0.70 with
+// pairs and leaves tested at once, 2.31 and 0.61 with five pairs per round and
+// postponed leaves; three and four records per round 1.99, 2.01 and 0.50, 0.48).
+// With pairs: claim 12, 20, 24 icosphere 2.31, 2.41, 2.58 ms, room 0.63, 0.60,
+// 0.61; 6 and 8 blocks per SM 2.44, 2.36 and 0.61, 0.65. Deeper trees: below
+// (kDeepFrame*).
 constexpr int kRefillFrameBlocksPerSm = 7;
-constexpr int kRefillFrameSteps = 5;
+constexpr int kRefillFrameSteps = 2;
 
 // COUNT: the same frame, also counting its work (FrameArgs::work); the
 // counters cost registers, so frames are rendered without them.
@@ -545,13 +597,13 @@ constexpr int kRefillFrameSteps = 5;
 // the same entries cost 3-4 %.
 constexpr int kDeepFrameStackShared = 16;
 
-// Deep trees: claim threshold 8 and four node pairs per round. 870k tube,
-// 1280x736, 16 samples in one launch: 2, 3, 4, 5, 6 pairs per round -> 30.6,
-// 29.4, 28.7, 29.1, 29.9 ms (35.7 with leaves tested at once, three steps);
-// at five, claim 6, 12, 16 -> 29.7, 29.2, 30.5 ms; 6 and 8 resident blocks
-// per SM 30.6 and 30.3 ms.
+// Deep trees: claim threshold 8 and two wide records per round. 870k tube,
+// 1280x736, 16 samples in one launch: 25.7 ms (35.7 with pairs and leaves tested
+// at once, 28.7 with four pairs per round and postponed leaves; three and four
+// records per round 26.1, 27.3). With pairs: claim 6, 12, 16 -> 29.7, 29.2, 30.5
+// ms; 6 and 8 resident blocks per SM 30.6 and 30.3 ms.
 constexpr int kDeepFrameClaim = 8;
-constexpr int kDeepFrameSteps = 4;
+constexpr int kDeepFrameSteps = 2;
 // DEEP: a tree deeper than 40 levels (shared stack entries, the constants above).
 // MULTI: a.samples samples in one launch (FramePaths<true>).
 template <bool DEEP, bool COUNT, bool MULTI = false>
@@ -717,6 +769,14 @@ cudaError_t launch_prep_geom(const cvx_triangle* tris, uint32_t n, float4* geom,
     return cudaGetLastError();
 }
 
+cudaError_t launch_prep_wide(const float4* nodes, uint32_t n_pairs, float4* wide, cudaStream_t st) {
+    uint32_t blocks = (n_pairs + 127) / 128;
+    if (blocks > 4096) blocks = 4096;
+    if (blocks == 0) blocks = 1;
+    k_prep_wide<<<blocks, 128, 0, st>>>(nodes, n_pairs, wide);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_prep_lights(const cvx_triangle* tris, const uint32_t* ds, uint32_t n, float4* lights,
                                cudaStream_t st) {
     uint32_t blocks = (n + 127) / 128;
@@ -750,9 +810,9 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
         uint32_t blocks = (uint32_t)num_sms() * bps;
         uint32_t need = (n + 127u) / 128u;
         if (blocks > need) blocks = need;
-        SoaRays src{s.nodes, s.geom, rays, n, far_dist, t_out, tri_out, counters};
+        SoaRays src{s.nodes, s.wide, s.geom, rays, n, far_dist, t_out, tri_out, counters};
         bool deep = s.depth > 40;
-        const bool sel = s.slab_sel != 0u && s.nested != 0u && !counters;
+        const bool sel = s.wide && !counters;
         if (counters) k_intersect_refill<8, true, 16, false><<<blocks, 128, 0, st>>>(src, err + 1, err);
         else if (!sel) {  // x86-form slab test throughout
             if (deep) k_intersect_refill<8, false, 8, false><<<blocks, 128, 0, st>>>(src, err + 1, err);

@@ -17,6 +17,7 @@ cudaError_t set_stack_limit_wave(int entries);
 cudaError_t upload_tables(const uint16_t* rcp, const uint16_t* rsqrt);
 cudaError_t upload_tables_wave(const uint16_t* rcp, const uint16_t* rsqrt);
 cudaError_t launch_prep_geom(const cvx_triangle* tris, uint32_t n, float4* geom, TriShade* shade, cudaStream_t st);
+cudaError_t launch_prep_wide(const float4* nodes, uint32_t n_pairs, float4* wide, cudaStream_t st);
 cudaError_t launch_prep_lights(const cvx_triangle* tris, const uint32_t* ds, uint32_t n, float4* lights,
                                cudaStream_t st);
 // The six ray components of a nearest-hit query (origin x, y, z, direction

@@ -37,9 +37,10 @@ struct DeviceScene {
     // Every node bound is finite, lo <= hi on each axis and none is -0: the
     // ray-cast kernel may take the select-form slab test (box_test_sel).
     uint32_t slab_sel;
-    // Every node's bounds lie inside its parent's (true of every built tree):
-    // with slab_sel, rays may be traced with postponed leaves (RefillRay::walk).
-    uint32_t nested;
+    // The wide records of the node pairs (traverse.cuh), for the select form;
+    // null unless slab_sel, every node's bounds lie inside its parent's (true of
+    // every built tree) and the tree is at most kWideMaxDepth levels deep.
+    const float4* wide;
 };
 
 struct DeviceCamera {
@@ -48,6 +49,8 @@ struct DeviceCamera {
 
 constexpr uint32_t kSkyMaterial = 0xC0000000u;  // material.rs:85-90
 constexpr int kStackDepth = 128;  // >= BVH depth + 2 (checked at scene creation)
+// Up to three boxes of a wide record wait on the stack: at most 1.5 per level.
+constexpr uint32_t kWideMaxDepth = (kStackDepth - 8) / 3 * 2;
 
 // Error bits a kernel reports through its status word instead of trapping.
 constexpr uint32_t kErrStackOverflow = 1u;

@@ -5,7 +5,7 @@
 //
 // Each lane takes one path at a time from a counter (path p is lane p & 7 of
 // group p >> 3) and carries it through its bounces; every round a lane tracing
-// a ray processes up to STEPS node pairs of it (RefillRay). A lane whose ray is finished waits until CLAIM_MIN lanes of its warp are in that
+// a ray processes up to STEPS records of it (RefillRay). A lane whose ray is finished waits until CLAIM_MIN lanes of its warp are in that
 // state (or none is tracing); those lanes then shade together: the hit record,
 // continue_path, and either the next bounce's ray or the pixel's store and a
 // new path with its camera ray. Warps thus stay busy while paths of 1 to 5
@@ -27,6 +27,8 @@
 //   uint32_t n_paths() const, uint32_t claim(uint32_t n)  (first of n paths)
 //   bool begin(uint32_t p, PathRef&, F3& o, F3& d, LaneRng&, const ApproxTables&)
 //       (false: the path's group lies outside its image; take another)
+//   void first_scene(nodes, wide, geom): the scene pointers before the first
+//       path (the one scene's, where there is one: they need no registers then)
 //   DeviceScene scene(const PathRef&) const  (a copy: its fields stay in
 //       registers through the shading code, which stores to the images)
 //   void gbuffer(const PathRef&, uint32_t word), void mark_emitter(const PathRef&)
@@ -42,7 +44,7 @@
 
 namespace cvx {
 
-// SELECT_ROUNDS: a round walks STEPS node pairs with the select-form slab test
+// SELECT_ROUNDS: a round walks STEPS wide records with the select-form slab test
 // and tests the leaves they led to once, at its end (RefillRay::walk), when
 // every tracing lane's ray allows it (a warp-uniform choice, so neither form's
 // code runs for the other's lanes); otherwise it takes STEPS steps in the x86
@@ -54,7 +56,7 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
     const int lane = threadIdx.x & 31;
     const uint32_t npaths = P.n_paths();
     RefillRay ray;
-    uint2 local_stack[kStackDepth];
+    uint2 local_stack[kStackSlots];
     typename std::conditional<SHARED_STACK == 0, LocalStack, SharedLocalStack<SHARED_STACK>>::type stack =
         make_stack<SHARED_STACK>(shared_stack, local_stack);
     ray.top = make_uint2(0u, 0u);
@@ -63,8 +65,8 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
     ray.leaf = 0u;
     ray.cur_t = 0.0f;
     ray.na = ray.nt = 0;
-    ray.nodes = ray.geom = nullptr;
-    ray.o = ray.d = ray.inv = f3(0, 0, 0);
+    P.first_scene(ray.nodes, ray.wide, ray.geom);
+    ray.no = ray.d = ray.inv = f3(0, 0, 0);
     ray.h = Hit{0.0f, 0.0f, 0.0f, -1};
     LaneRng rng;
     rng.s = rng.f = 0ull;
@@ -87,13 +89,13 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
                 work_tris += ray.nt;
             }
             const DeviceScene s = P.scene(ref);
-            Isect I = make_isect(s, ray.h, ray.o, ray.d, tab);
+            Isect I = make_isect(s, ray.h, ray.o(), ray.d, tab);
             const bool em = (I.mat >> 31) != 0u;
             const bool ends = em || bounce == 4u;
             // continue_path (material.rs:327-411), split so that a lane that
             // ends at an emitter on bounce 0 stops after the Fresnel value of
             // its gbuffer word (its colour modulation is 1).
-            NextRay n{ray.o, ray.d, false};
+            NextRay n{ray.o(), ray.d, false};
             float fr = 0.0f;
             if (bounce == 0u || !ends) n = sample_next(s, I, rng, tab);
             if (em) {
@@ -119,8 +121,8 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
                 has_path = false;
             } else {
                 bounce++;
-                ray.start(n.o, n.d, 1.0e5f, s.nodes, s.geom, tab);
-                ray_sel = SELECT_ROUNDS && s.slab_sel && s.nested && select_form_ray(ray.inv);
+                ray.start(n.o, n.d, 1.0e5f, s.nodes, s.wide, s.geom, tab);
+                ray_sel = SELECT_ROUNDS && s.wide && select_form_ray(ray.no, ray.inv);
                 tracing = true;
                 P.count_ray(ref);
             }
@@ -141,8 +143,8 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
                     F3 o, d;
                     if (P.begin(p, ref, o, d, rng, tab)) {  // else: a group outside its image; take another path
                         const DeviceScene s = P.scene(ref);
-                        ray.start(o, d, 1.0e5f, s.nodes, s.geom, tab);
-                        ray_sel = SELECT_ROUNDS && s.slab_sel && s.nested && select_form_ray(ray.inv);
+                        ray.start(o, d, 1.0e5f, s.nodes, s.wide, s.geom, tab);
+                        ray_sel = SELECT_ROUNDS && s.wide && select_form_ray(ray.no, ray.inv);
                         color = f3(1.0f, 1.0f, 1.0f);
                         bounce = 0u;
                         has_path = true;

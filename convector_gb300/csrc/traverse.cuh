@@ -70,9 +70,136 @@ __device__ __forceinline__ BoxT box_test_sel(float lx, float ly, float lz, float
     float tmax = xmin(fx, xmin(fy, fz));
     return BoxT{tmin, tmax, geq(tmax, tmin)};
 }
-__device__ __forceinline__ bool select_form_ray(F3 inv) {
-    return isfinite(inv.x) && isfinite(inv.y) && isfinite(inv.z) && fabsf(inv.x) >= 0.75f &&
-           fabsf(inv.y) >= 0.75f && fabsf(inv.z) >= 0.75f;
+
+// The wide record of a node pair, 128 B (8 x 16 B): the boxes of the pair's
+// grandchildren, slots 0 and 1 the children of the pair's first node, 2 and 3 of
+// its second. A node that is a leaf takes its first slot itself and leaves the
+// other one empty (lo kEmptyLo, hi -kEmptyLo: never hit). w[2a], w[2a + 1]: lo
+// and hi on axis a of the four slots; w[6]: their references (the same as in the
+// pair records: an internal node is its child pair, whose wide record is at 128
+// bytes times the pair's index).
+constexpr float kEmptyLo = 1.0e30f;
+
+// A difference of two distances that is not negative (no NaN matters here).
+__device__ __forceinline__ bool ge0(float x) { return (int32_t)fb(x) >= 0; }
+
+// sm_100's three-operand minimum and maximum.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// A ray against a wide record in select form: the near and far plane of each
+// axis are picked by the sign of the ray's reciprocal (box_test_sel), by address,
+// so that no select is spent on them, and the four boxes' distances to them take
+// two planes per instruction (packed FP32, sm_100; the negated origin is added,
+// which is the same operation). t: entry distance of each slot's box if it is
+// hit, +inf if not; tc: entry distances of the pair's own two boxes.
+//
+// The axes are joined by max3 and min3. They differ from the x86 min and max
+// only where the result is a zero (of two tied zeros x86 takes the later
+// operand, max3 +0 and min3 -0), and where no exit distance is zero, a ray that
+// hits a grandchild's box hits the child's. Where any of the results is zero (an
+// origin on a bound plane; rare), exact() takes the pair records and the x86
+// form for this step. The products of the results show it (0, or NaN from
+// inf * 0; an underflow only costs time).
+struct WideT {
+    float t[4], tc0, tc1;
+    uint4 r;
+    __device__ __forceinline__ WideT(const float4* __restrict__ nodes, const float4* __restrict__ wide, uint32_t ref,
+                                     F3 no, F3 inv) {
+        const float4* w = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(wide) + (size_t)ref * 2);
+        const char* wb = reinterpret_cast<const char*>(w);
+        auto ld = [](const char* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
+        const int sx = inv.x > 0.0f ? 0 : 16, sy = inv.y > 0.0f ? 0 : 16, sz = inv.z > 0.0f ? 0 : 16;
+        const float4 nx4 = ld(wb + sx), fx4 = ld(wb + 16 - sx), ny4 = ld(wb + 32 + sy), fy4 = ld(wb + 48 - sy),
+                     nz4 = ld(wb + 64 + sz), fz4 = ld(wb + 80 - sz);
+        r = __ldg(reinterpret_cast<const uint4*>(w + 6));
+        auto dist = [](float4 v, float n, float i, float* out) {
+            const float2 n2 = make_float2(n, n), i2 = make_float2(i, i);
+            const float2 a = __fmul2_rn(__fadd2_rn(make_float2(v.x, v.y), n2), i2);
+            const float2 b = __fmul2_rn(__fadd2_rn(make_float2(v.z, v.w), n2), i2);
+            out[0] = a.x; out[1] = a.y; out[2] = b.x; out[3] = b.y;
+        };
+        float nx[4], ny[4], nz[4], fx[4], fy[4], fz[4], e[4];
+        dist(nx4, no.x, inv.x, nx);
+        dist(ny4, no.y, inv.y, ny);
+        dist(nz4, no.z, inv.z, nz);
+        dist(fx4, no.x, inv.x, fx);
+        dist(fy4, no.y, inv.y, fy);
+        dist(fz4, no.z, inv.z, fz);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            t[k] = max3(nx[k], ny[k], nz[k]);
+            e[k] = min3(fx[k], fy[k], fz[k]);
+        }
+        tc0 = max3(fminf(nx[0], nx[1]), fminf(ny[0], ny[1]), fminf(nz[0], nz[1]));
+        tc1 = max3(fminf(nx[2], nx[3]), fminf(ny[2], ny[3]), fminf(nz[2], nz[3]));
+        const float p0 = (t[0] * e[0]) * (t[1] * e[1]) * tc0, p1 = (t[2] * e[2]) * (t[3] * e[3]) * tc1;
+        if (__builtin_expect(!(fabsf(p0) > 0.0f && fabsf(p1) > 0.0f), 0)) {
+            exact(nodes, ref, f3(-no.x, -no.y, -no.z), inv);
+        } else {
+            const float inf = __int_as_float(0x7f800000);
+#pragma unroll
+            for (int k = 0; k < 4; k++) t[k] = (e[k] >= t[k]) & (e[k] > 0.0f) ? t[k] : inf;
+        }
+    }
+    // This step from the pair records: the pair's boxes, then those of its
+    // children that are hit.
+    __device__ __forceinline__ void exact(const float4* __restrict__ nodes, uint32_t ref, F3 o, F3 inv) {
+        const float inf = __int_as_float(0x7f800000);
+#pragma unroll
+        for (int k = 0; k < 4; k++) t[k] = inf;
+        BoxT b[2], c[2];
+        uint32_t br[2], cr[2];
+        pair(nodes, ref, o, inv, b, br);
+        tc0 = b[0].tmin;
+        tc1 = b[1].tmin;
+        if (hit(b[0])) {
+            if ((br[0] & 31u) != 0u) {
+                t[0] = tc0;
+            } else {
+                pair(nodes, br[0], o, inv, c, cr);
+                if (hit(c[0])) t[0] = c[0].tmin;
+                if (hit(c[1])) t[1] = c[1].tmin;
+            }
+        }
+        if (hit(b[1])) {
+            if ((br[1] & 31u) != 0u) {
+                t[2] = tc1;
+            } else {
+                pair(nodes, br[1], o, inv, c, cr);
+                if (hit(c[0])) t[2] = c[0].tmin;
+                if (hit(c[1])) t[3] = c[1].tmin;
+            }
+        }
+    }
+    static __device__ __forceinline__ bool hit(const BoxT& b) { return b.mask & !sneg(b.tmax); }
+    static __device__ __forceinline__ void pair(const float4* __restrict__ nodes, uint32_t ref, F3 o, F3 inv, BoxT* b,
+                                                uint32_t* r) {
+        const float4* np = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + ref);
+        const float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
+        b[0] = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
+        b[1] = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
+        r[0] = __float_as_uint(q3.x);
+        r[1] = __float_as_uint(q3.y);
+    }
+};
+
+// Rays that may take the select form: reciprocals and origin as above, and
+// bounded (with the bounds, DeviceScene::slab_sel), so that no plane distance
+// overflows.
+constexpr float kSelectMax = 1.0e18f;
+__device__ __forceinline__ bool select_form_ray(F3 o, F3 inv) {
+    auto in = [](float x) { return fabsf(x) >= 0.75f && fabsf(x) <= kSelectMax; };
+    return in(inv.x) && in(inv.y) && in(inv.z) && fabsf(o.x) <= kSelectMax && fabsf(o.y) <= kSelectMax &&
+           fabsf(o.z) <= kSelectMax;
 }
 
 // One triangle against one lane; updates the hit when the reference would
@@ -221,22 +348,28 @@ struct RayIn {
     F3 o, d;
     float far;
     const float4* nodes;
+    const float4* wide;  // SELECT only
     const float4* geom;
 };
+
+// A refill traversal's stack: entry 0 is a spare (what `top` holds while the
+// stack is empty is stored there and never used, which saves a test per push
+// and pop), and a wide step may push three entries before it checks the limit.
+constexpr int kStackSlots = kStackDepth + 4;
 
 // Where a refill traversal keeps the stack entries below its top. LocalStack:
 // a local array. SharedLocalStack<N>: the first N entries in shared memory,
 // in this lane's column of a warp's [N][32] block (no bank conflicts, and pops
 // of those never miss the cache), the deeper ones in the local array.
 struct LocalStack {
-    uint2 (&a)[kStackDepth];
+    uint2 (&a)[kStackSlots];
     __device__ __forceinline__ uint2 load(int i) const { return a[i]; }
     __device__ __forceinline__ void store(int i, uint2 v) { a[i] = v; }
 };
 template <int N>
 struct SharedLocalStack {
     uint2* sm;  // entry i at sm[32 * i]
-    uint2 (&a)[kStackDepth];
+    uint2 (&a)[kStackSlots];
     __device__ __forceinline__ uint2 load(int i) const { return i < N ? sm[32 * i] : a[i]; }
     __device__ __forceinline__ void store(int i, uint2 v) {
         if (i < N) sm[32 * i] = v;
@@ -253,8 +386,9 @@ struct SharedLocalStack {
 struct RefillRay {
     static constexpr uint32_t kNone = 0xffffffffu;
     const float4* nodes;
+    const float4* wide;
     const float4* geom;
-    F3 o, d, inv;
+    F3 no, d, inv;  // no: the negated origin
     Hit h;
     // The stack holds (ref, entry distance bits) entries. Its top entry lives
     // in `top`, the entries below it in the caller's local array: a pop takes
@@ -267,11 +401,13 @@ struct RefillRay {
     float cur_t;    // entry distance of cur
     uint32_t na, nt;
 
-    __device__ __forceinline__ void start(F3 o_, F3 d_, float far, const float4* nodes_, const float4* geom_,
-                                          const ApproxTables& tab) {
-        o = o_;
+    __device__ __forceinline__ F3 o() const { return f3(-no.x, -no.y, -no.z); }
+    __device__ __forceinline__ void start(F3 o_, F3 d_, float far, const float4* nodes_, const float4* wide_,
+                                          const float4* geom_, const ApproxTables& tab) {
+        no = f3(-o_.x, -o_.y, -o_.z);
         d = d_;
         nodes = nodes_;
+        wide = wide_;
         geom = geom_;
         inv = f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab));
         h = Hit{far, 0.0f, 0.0f, -1};
@@ -296,7 +432,7 @@ struct RefillRay {
             // Pop until an entry survives the cull test (aabb.rs:171-177).
             while (sp > 0) {
                 uint2 e = top;
-                if (--sp > 0) top = stack.load(sp - 1);
+                top = stack.load(--sp);
                 if (!geq(__uint_as_float(e.y), h.t)) {
                     cur = e.x;
                     cur_t = __uint_as_float(e.y);
@@ -309,7 +445,7 @@ struct RefillRay {
         if (!LEAF_AFTER_PAIR && len != 0u) {  // a popped leaf; the pair loop continues next iteration
             leaf_range(nodes, idx, len);
 #pragma unroll 1
-            for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o, d, true, h);
+            for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o(), d, true, h);
             if (COUNT) nt += len;
             cur = kNone;
             return false;
@@ -322,8 +458,8 @@ struct RefillRay {
             // the child pair (64 bytes per pair).
             const float4* np = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + cur);
             float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
-            const BoxT b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
-            const BoxT b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
+            const BoxT b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o(), inv);
+            const BoxT b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o(), inv);
             bool first0 = !sneg(b0.tmin - b1.tmin);
             bool hit0 = b0.mask & !sneg(b0.tmax);
             bool hit1 = b1.mask & !sneg(b1.tmax);
@@ -339,7 +475,7 @@ struct RefillRay {
                 return false;
             }
             if (hit_first) {
-                if (sp > 0) stack.store(sp - 1, top);
+                stack.store(sp, top);
                 top = make_uint2(ref_first, __float_as_uint(t_first));
                 sp++;
             }
@@ -354,30 +490,40 @@ struct RefillRay {
         if (len != 0u) {
             leaf_range(nodes, idx, len);
 #pragma unroll 1
-            for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o, d, true, h);
+            for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o(), d, true, h);
             if (COUNT) nt += len;
             cur = kNone;
         }
         return false;
     }
 
-    // The same traversal with the leaf tests postponed (select form): walk()
-    // goes on from node pair to node pair while at most one leaf waits in
-    // `leaf`, and test_leaf() tests that leaf's triangles. A warp alternates a
-    // few walk() steps with one test_leaf(), so the triangle code runs once per
-    // round for all lanes that reached a leaf in it, not at nearly every step
-    // for one or two lanes.
+    // The same traversal over the wide records (select form), with the leaf
+    // tests postponed: walk() goes on from record to record while at most one
+    // leaf waits in `leaf`, and test_leaf() tests that leaf's triangles. A warp
+    // alternates a few walk() steps with one test_leaf(), so the triangle code
+    // runs once per round for all lanes that reached a leaf in it, not at nearly
+    // every step for one or two lanes.
     //
-    // The results are those of step(): a node walked on to before the waiting
-    // leaf was tested may be one that step(), knowing the leaf's hit, would have
-    // culled (entry distance t at or beyond the hit). Its children then have
-    // entry distances of at least t: their bounds lie inside the node's
-    // (DeviceScene::nested), and differences, products and the minima and maxima
-    // of the slab test are monotonic in the bounds, for finite values. So they
-    // are culled when they are popped, or by test_leaf() where one is `cur`, and
-    // no triangle is tested that step() does not test, nor in another order. Box
-    // tests do not depend on the hit distance. (With the stack limit lowered, a
-    // push below such a node can overflow.)
+    // A wide record holds the boxes of a pair's four grandchildren (WidePair):
+    // one step does what step() does for the pair and for both its children.
+    // The triangles tested and their order are those of step():
+    //  * Bounds nest (checked at scene creation), and the differences, products,
+    //    minima and maxima of the slab test are monotonic in the bounds, for
+    //    finite values. So a ray that hits a grandchild's box hits the child's,
+    //    with an entry distance not beyond the grandchild's: the child's own
+    //    test and its cull when popped decide nothing that the grandchild's do
+    //    not decide, at the same hit distance.
+    //  * A child's bound on an axis is that of one of its two boxes, so its near
+    //    plane distance is the smaller of theirs and its entry distance, which
+    //    orders the children, the largest over the axes: the same bits, as the
+    //    two boxes' zeros on an axis have one sign.
+    //  * A box entered at or beyond the hit distance would be culled when popped,
+    //    as the hit distance never grows: it is not pushed. One that a waiting
+    //    leaf's hit culls is dropped when popped, or by test_leaf() where it is
+    //    `cur`, and so are the boxes below it, entered no nearer.
+    // (With the stack limit lowered, the overflow status may come at another
+    // node; up to three boxes of a record are pushed, so trees of up to
+    // kWideMaxDepth levels fit the stack.)
     //
     // Does nothing when the stack is empty or the next node is a leaf and one
     // waits already.
@@ -385,7 +531,7 @@ struct RefillRay {
     __device__ __forceinline__ void walk(Stack& stack, bool& overflow) {
         while (cur == kNone && sp > 0) {
             uint2 e = top;
-            if (--sp > 0) top = stack.load(sp - 1);
+            top = stack.load(--sp);
             if (!geq(__uint_as_float(e.y), h.t)) {
                 if ((e.x & 31u) != 0u && leaf == 0u) {
                     leaf = e.x;
@@ -396,32 +542,39 @@ struct RefillRay {
             }
         }
         if ((cur & 31u) != 0u) return;  // nothing left, or a second leaf
-        const float4* np = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + cur);
-        float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
-        const BoxT b0 = box_test_sel(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
-        const BoxT b1 = box_test_sel(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
-        const bool first0 = !sneg(b0.tmin - b1.tmin);
-        const bool hit0 = b0.mask & !sneg(b0.tmax);
-        const bool hit1 = b1.mask & !sneg(b1.tmax);
-        const uint32_t r0 = __float_as_uint(q3.x), r1 = __float_as_uint(q3.y);
-        // The reference pushes `first` then `second` and pops `second` first.
-        const bool hit_first = first0 ? hit0 : hit1, hit_second = first0 ? hit1 : hit0;
-        const uint32_t ref_first = first0 ? r0 : r1, ref_second = first0 ? r1 : r0;
-        const float t_first = first0 ? b0.tmin : b1.tmin, t_second = first0 ? b1.tmin : b0.tmin;
-        if (sp + (int)hit_first + (int)hit_second > c_stack_limit) {
+        const WideT w(nodes, wide, cur, no, inv);
+        cur = kNone;
+        // The order of step(): of two boxes the reference pops first the one it
+        // pushes second (the second, unless the first is entered nearer), and
+        // the boxes of the child it pops first before the other child's.
+        const bool in0 = ge0(w.t[0] - w.t[1]), in1 = ge0(w.t[2] - w.t[3]), ch = ge0(w.tc0 - w.tc1);
+        const float a0 = in0 ? w.t[0] : w.t[1], a1 = in0 ? w.t[1] : w.t[0];  // child 0: last, first
+        const float b0 = in1 ? w.t[2] : w.t[3], b1 = in1 ? w.t[3] : w.t[2];
+        const uint32_t ra0 = in0 ? w.r.x : w.r.y, ra1 = in0 ? w.r.y : w.r.x;
+        const uint32_t rb0 = in1 ? w.r.z : w.r.w, rb1 = in1 ? w.r.w : w.r.z;
+        const float t[4] = {ch ? a0 : b0, ch ? a1 : b1, ch ? b0 : a0, ch ? b1 : a1};
+        const uint32_t r[4] = {ch ? ra0 : rb0, ch ? ra1 : rb1, ch ? rb0 : ra0, ch ? rb1 : ra1};
+        // From the last to the first: each box hit becomes the next node, and
+        // the one before it is pushed.
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (t[k] < h.t) {
+                if (k > 0 && cur != kNone) {
+                    stack.store(sp, top);
+                    top = make_uint2(cur, __float_as_uint(cur_t));
+                    sp++;
+                }
+                cur = r[k];
+                cur_t = t[k];
+            }
+        }
+        if (sp > c_stack_limit) {
             overflow = true;
             sp = 0;
             cur = kNone;
             leaf = 0u;
             return;
         }
-        if (hit_first) {
-            if (sp > 0) stack.store(sp - 1, top);
-            top = make_uint2(ref_first, __float_as_uint(t_first));
-            sp++;
-        }
-        cur = (hit_second && !geq(t_second, h.t)) ? ref_second : kNone;
-        cur_t = t_second;
         if (cur != kNone && (cur & 31u) != 0u && leaf == 0u) {
             leaf = cur;
             cur = kNone;
@@ -434,7 +587,7 @@ struct RefillRay {
             uint32_t len = leaf & 31u, idx = leaf >> 5;
             leaf_range(nodes, idx, len);
 #pragma unroll 1
-            for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o, d, true, h);
+            for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o(), d, true, h);
             leaf = 0u;
             if (geq(cur_t, h.t)) cur = kNone;
             if (cur != kNone && (cur & 31u) != 0u) {  // the second leaf is next
@@ -456,7 +609,7 @@ struct RefillRay {
 
 template <int N>
 __device__ __forceinline__ typename std::conditional<N == 0, LocalStack, SharedLocalStack<N>>::type make_stack(
-    uint2* sm, uint2 (&a)[kStackDepth]) {
+    uint2* sm, uint2 (&a)[kStackSlots]) {
     if constexpr (N == 0) return LocalStack{a};
     else return SharedLocalStack<N>{sm, a};
 }
@@ -466,6 +619,9 @@ __device__ __forceinline__ typename std::conditional<N == 0, LocalStack, SharedL
 // a lane whose ray is finished takes the next unclaimed ray, so warps stay
 // full while rays of different lengths finish.
 // The whole warp must call this. `src` provides
+//   void first_scene(nodes, wide, geom): what the scene pointers hold before
+//   the first ray (a source of one scene gives that scene's, so that the
+//   pointers need no registers)
 //   void store(r, const Hit&, uint32_t boxes, uint32_t triangles)
 // (box and triangle counts when COUNT, else 0). LEAF_AFTER_PAIR: a lane whose
 // pair test leads to a leaf tests that leaf in the same iteration (fewer
@@ -485,7 +641,7 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
                                                 uint2* shared_stack = nullptr) {
     const int lane = threadIdx.x & 31;
     RefillRay ray;
-    uint2 local_stack[kStackDepth];
+    uint2 local_stack[kStackSlots];
     typename std::conditional<SHARED_STACK == 0, LocalStack, SharedLocalStack<SHARED_STACK>>::type stack =
         make_stack<SHARED_STACK>(shared_stack, local_stack);
     ray.top = make_uint2(0u, 0u);
@@ -494,8 +650,8 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
     ray.leaf = 0u;
     ray.cur_t = 0.0f;
     ray.na = ray.nt = 0;
-    ray.nodes = ray.geom = nullptr;
-    ray.o = ray.d = ray.inv = f3(0, 0, 0);
+    src.first_scene(ray.nodes, ray.wide, ray.geom);
+    ray.no = ray.d = ray.inv = f3(0, 0, 0);
     ray.h = Hit{0.0f, 0.0f, 0.0f, -1};
     uint32_t r_id = 0;
     bool have = false, done = false, overflow = false;
@@ -514,10 +670,10 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
             if (want) {
                 if (got == kClaimRay) {
                     r_id = r;
-                    ray.start(in.o, in.d, in.far, in.nodes, in.geom, tab);
+                    ray.start(in.o, in.d, in.far, in.nodes, in.wide, in.geom, tab);
                     have = true;
                     if constexpr (SELECT) {
-                        if (!select_form_ray(ray.inv)) {
+                        if (!select_form_ray(ray.no, ray.inv)) {
                             src.defer(r);
                             have = false;
                         }

@@ -168,6 +168,9 @@ __global__ void __launch_bounds__(128, 8) k_wf_traverse_octet(const Job* __restr
 // its result is stored without reading the queue again.
 struct QueueStore {
     WaveState st;
+    __device__ __forceinline__ void first_scene(const float4*& nd, const float4*& wd, const float4*& gm) const {
+        nd = wd = gm = nullptr;
+    }
     __device__ __forceinline__ void store(uint32_t l, const Hit& h, uint32_t, uint32_t) const {
         st.ht[l] = h.t;
         st.hu[l] = h.u;
@@ -202,6 +205,7 @@ struct QueueClaim {
         }
         const DeviceScene* s = scenes + jobs[st.group_job[gi]].scene;
         in.nodes = s->nodes;
+        in.wide = nullptr;
         in.geom = s->geom;
         in.o = f3(st.ox[l], st.oy[l], st.oz[l]);
         in.d = f3(st.dx[l], st.dy[l], st.dz[l]);
@@ -453,6 +457,9 @@ struct WavePaths {
         camera_ray(j.cam, x, y, unit_from(rng.next()), tab, o, d);
         return true;
     }
+    __device__ __forceinline__ void first_scene(const float4*& nd, const float4*& wd, const float4*& gm) const {
+        nd = wd = gm = nullptr;
+    }
     __device__ __forceinline__ DeviceScene scene(const PathRef& r) const { return scenes[__ldg(&jobs[r.job].scene)]; }
     __device__ __forceinline__ void gbuffer(const PathRef& r, uint32_t word) {
         if (!out.gbuf) return;
@@ -510,12 +517,13 @@ struct WavePaths {
 // no spill) served the 415-request mix at 2,014 against 2,083 Mrays/s.
 // With postponed leaves (below) again: 6 blocks 2,744 against 2,869 Mrays/s.
 constexpr int kRefillWaveBlocksPerSm = 7;
-// Node pairs a lane walks per round. With postponed leaves (RefillRay::walk),
-// whose rounds test their leaves once, five; against the x86-form rounds of
-// two steps before, a served 1280x736 request of 16 samples takes: room 11.2 ->
-// 9.5 ms, 82k icosphere 20.7 -> 17.3 ms, 870k tube 38.2 -> 31.4 ms, although
-// the spill grows from 82-94 to 112-120 bytes (three steps: 9.7, 17.8, 31.3).
-constexpr int kRefillWaveSteps = 5;
+// Wide records a lane walks per round (RefillRay::walk), whose leaves are tested
+// once at its end. Five node pairs per round against x86-form rounds of two
+// steps, a served 1280x736 request of 16 samples: room 11.2 -> 9.5 ms, 82k
+// icosphere 20.7 -> 17.3 ms, 870k tube 38.2 -> 31.4 ms, although the spill grows
+// from 82-94 to 112-120 bytes. Records instead of pairs, 16 mixed requests: 159
+// -> 149 ms (three and four per round 147, 153).
+constexpr int kRefillWaveSteps = 2;
 // As the frame kernel: waves whose trees are deeper than 40 levels keep the
 // first 16 stack entries of each lane in shared memory and read the tables
 // from global memory (4 tube views of 1280x736, 2 samples: 21.5 -> 20.3 ms;

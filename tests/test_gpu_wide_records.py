@@ -1,0 +1,124 @@
+"""Traversal over the wide records with postponed leaves (RefillRay::walk)
+against the oracle's traversals, bit for bit: scenes whose leaves are large,
+whose nodes do not nest or enclose loosely, whose tree is too deep, or whose
+bounds are too large (which keep the x86 form), rays that start on box corners
+(tied zeros in the slab test), directions beyond the select form, and rays with
+a short far distance, at counts around a claim's 32 rays.
+"""
+
+import numpy as np
+import pytest
+
+from convector_gb300 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene_arrays(gpu, kind):
+    tris = scenes.spheres_and_boxes(3000, 5, obj=False)[0]
+    if kind == "large leaves":  # stacks of coincident triangles: leaves of several triangles
+        tris = np.concatenate([np.repeat(tris[:40], 20, axis=0), tris])
+    b = gpu.Bvh.build(tris)
+    nodes = b.nodes.copy()
+    if kind == "not nested":  # every third node reaches out of its parent
+        f = nodes.view(np.float32)
+        f[2::3, 3:6] += np.float32(0.25)
+    if kind == "loose":  # the roots reach further than their children
+        f = nodes.view(np.float32)
+        f[0:2, 0:3] -= np.float32(0.5)
+        f[0:2, 3:6] += np.float32(0.5)
+    return b, nodes
+
+
+def _chain(n):
+    """A chain of n pairs, each node 0 a leaf and node 1 the rest: n + 1 levels deep."""
+    tris = np.zeros((n + 1, 16), np.uint32)
+    f = tris.view(np.float32)
+    x = np.arange(n + 1, dtype=np.float32) * np.float32(0.02) - np.float32(1.0)
+    f[:, 0:9] = np.stack([x, x * 0 + 0.5, x * 0 - 2, x, x * 0 + 1.5, x * 0 - 2.5, x, x * 0 + 1, x * 0 - 1], 1)
+    tris[:, 15] = 0x00FFFFFF
+    tris[::4, 15] |= 0x40000000
+    nodes = np.zeros((2 * n, 8), np.uint32)
+    g = nodes.view(np.float32)
+    lo, hi = np.array([0.5, -2.5], np.float32), np.array([1.5, -1.0], np.float32)
+    for p in range(n):
+        for k, (a, b) in enumerate(((p, p), (p + 1, n))):
+            g[2 * p + k, 0:6] = [x[a], lo[0], lo[1], x[b], hi[0], hi[1]]
+        nodes[2 * p, 6:8] = (p, 1)
+        nodes[2 * p + 1, 6:8] = (2 * p + 2, 0) if p + 1 < n else (n, 1)
+    return tris, nodes
+
+
+def _rays(nodes, n, seed):
+    o, d = scenes.random_rays(n, seed=seed)
+    f = nodes.view(np.float32)
+    corners = np.stack([f[:, [a, b, c]] for a in (0, 3) for b in (1, 4) for c in (2, 5)], 1).reshape(-1, 3)
+    k = n // 2
+    o[:k] = corners[np.random.default_rng(seed).integers(0, corners.shape[0], k)]
+    return o, d
+
+
+@pytest.mark.parametrize("kind", ["plain", "large leaves", "not nested", "loose"])
+@pytest.mark.parametrize("n,far", [(1, 1.0e5), (31, 1.0e5), (33, 1.0e5), (40007, 1.0e5), (40007, 0.5)])
+def test_query_equals_oracle(gpu, orc, kind, n, far):
+    b, nodes = _scene_arrays(gpu, kind)
+    b.nodes = nodes
+    scene, osc = gpu.Scene(b), orc.OracleScene(b.triangles, nodes)
+    o, d = _rays(nodes, n, seed=n)
+    for traversal in (gpu.TRAVERSE_SINGLE, gpu.TRAVERSE_PACKET):
+        t, tri = scene.intersect_nearest(o, d, far=far, traversal=traversal)
+        ot, otri = osc.intersect(o, d, far=far, mode=traversal)
+        assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
+        assert (t.view(np.uint32) == ot.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("kind", ["plain", "large leaves", "not nested"])
+@pytest.mark.parametrize("refill", ["REFILL_ALL", "REFILL_NONE"])
+def test_frame_equals_oracle(gpu, orc, kind, refill):
+    b, nodes = _scene_arrays(gpu, kind)
+    b.nodes = nodes
+    scene, osc = gpu.Scene(b), orc.OracleScene(b.triangles, nodes)
+    # the eye on a box corner of the tree, so that camera rays meet tied zeros
+    f = nodes.view(np.float32)
+    scenes.default_camera(scene.camera, eye=tuple(float(v) for v in f[4, 3:6]), target=(0.0, 1.0, -2.0))
+    r = gpu.Renderer(scene, 83, 45, traversal=gpu.TRAVERSE_SINGLE, refill_mode=getattr(gpu, refill))
+    rgba, gb = r.render_frame_u8(9)
+    orgba, ogb, ocol, orays = osc.render(scene.camera.as_array(), 83, 45, 9, rng_order=orc.RNG_GROUP, traversal=1)
+    assert (rgba == orgba).all() and (gb == ogb).all()
+    assert (r.read_frame_f32().view(np.uint32) == ocol.view(np.uint32)).all()
+    assert r.stats()[0] == orays
+
+
+@pytest.mark.parametrize("pairs", [1, 2, 79, 80, 81, 125])
+def test_chains_equal_oracle(gpu, orc, pairs):
+    """Trees of 2 levels (every child a leaf) up to the deepest accepted, on both
+    sides of the deepest with wide records (80 levels)."""
+    tris, nodes = _chain(pairs)
+    b = type("B", (), {"triangles": tris, "nodes": nodes})()
+    scene, osc = gpu.Scene(b), orc.OracleScene(tris, nodes)
+    o, d = _rays(nodes, 2003, seed=pairs)
+    d[::5] = [1.0, 0.0, 0.0]                 # axis-parallel, through every level
+    d[1::5] *= np.float32(1.0e-30)           # reciprocals beyond the select form
+    d[2::5] *= np.float32(3.0)
+    o[3::5] = o[3::5] * np.float32(1.0e25)   # origins beyond it
+    for traversal in (gpu.TRAVERSE_SINGLE, gpu.TRAVERSE_PACKET):
+        t, tri = scene.intersect_nearest(o, d, traversal=traversal)
+        ot, otri = osc.intersect(o, d, mode=traversal)
+        assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
+        assert (t.view(np.uint32) == ot.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("scale", [1.0e-4, 1.0, 1.0e16, 1.0e18])
+def test_scales_equal_oracle(gpu, orc, scale):
+    """Scenes whose distances underflow the zero check or whose bounds exceed the select form's."""
+    tris = scenes.spheres_and_boxes(600, 5, obj=False)[0].copy()
+    tris.view(np.float32)[:, :9] *= np.float32(scale)
+    b = gpu.Bvh.build(tris)
+    scene, osc = gpu.Scene(b), orc.OracleScene.from_bvh(b)
+    o, d = scenes.random_rays(3001, seed=3)
+    o = (o * np.float32(scale)).astype(np.float32)
+    for traversal in (gpu.TRAVERSE_SINGLE, gpu.TRAVERSE_PACKET):
+        t, tri = scene.intersect_nearest(o, d, far=1.0e30, traversal=traversal)
+        ot, otri = osc.intersect(o, d, far=1.0e30, mode=traversal)
+        assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
+        assert (t.view(np.uint32) == ot.view(np.uint32)).all()
