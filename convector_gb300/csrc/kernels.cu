@@ -6,6 +6,7 @@
 #include <atomic>
 
 #include "kernels.h"
+#include "packet_refill.cuh"
 #include "path_refill.cuh"
 #include "shade.cuh"
 
@@ -317,6 +318,31 @@ __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uin
     if (!ok) atomicOr(err, kErrStackOverflow);
 }
 
+// The packet query: packets of a warp stepped together (packet_refill.cuh). Rays
+// are staged as in k_intersect_refill; an octet takes 8 consecutive ones.
+// Bound by instruction issue and the ALU pipe. One packet per octet, each octet
+// on its own path (the counting form below), against this: 1M rays of the
+// 19-level room 345 -> 311 us, of the 28-level icosphere 817 -> 628 us, of the
+// 70-level tube 1544 -> 1210 us. Stepping pairs instead of wide records 353, 738,
+// 1340 us. 7 blocks per SM (72 registers; 8 blocks spill: 329, 676, 1355 us).
+// STEPS records per round: 1, 2, 3 -> 309, 311, 379 us (room), 650, 628, 716
+// (icosphere), 1210, 1279, 1543 (tube): 1 for trees deeper than 40 levels, else 2.
+// 4, 8 or 12 shared stack entries are alike; waiting for two finished packets
+// before taking new ones 322, 701, 1312 us.
+constexpr int kPacketBlocksPerSm = 7;
+template <int STEPS>
+__global__ void __launch_bounds__(128, kPacketBlocksPerSm) k_intersect_packets(SoaRays src,
+                                                                               uint32_t* __restrict__ next_ray,
+                                                                               uint32_t* __restrict__ err) {
+    __shared__ float stage[4][2][6][32];
+    __shared__ uint2 sstack[4][kQueryStackShared][32];
+    StagedSoaClaim claim{src, next_ray, stage[threadIdx.x >> 5], 0u, 0u, 0u, 0};
+    claim.init(threadIdx.x & 31);
+    bool ok = traverse_packets<STEPS, kQueryStackShared>(src, claim, g_tables,
+                                                         &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
+    if (!ok) atomicOr(err, kErrStackOverflow);
+}
+
 // After k_intersect_refill<SELECT>: the rays it left (index word kDeferredRay:
 // a reciprocal infinite or below 0.75 in magnitude) with the x86-form slab
 // test. Such rays are rare (axis-parallel or very long directions), so the
@@ -622,6 +648,23 @@ __global__ void __launch_bounds__(128, kRefillFrameBlocksPerSm) k_render_refill(
     if (!ok) atomicOr(a.err, kErrStackOverflow);
 }
 
+// Frames in packet traversal, per-group RNG order: an octet holds one 8-pixel
+// group at a time and the packets of a warp step together (packet_refill.cuh).
+// One group per octet traced to its end (k_render_group) against this, 1280x736:
+// room 1.22 -> 1.13 ms, icosphere 3.66 -> 2.75, tube 8.88 -> 6.34; 320x184: room
+// 0.65 -> 0.39, icosphere 1.06 -> 0.57 ms. Two wide records per round and 5 blocks
+// per SM (80 registers and more, no spill; 6 and 7 blocks: room 1.14, 1.21 ms,
+// icosphere 2.77, 2.76 ms, the small one 0.61, 0.64 ms); trees deeper than 40
+// levels one record and 6 blocks (6.34 ms; two records 6.81-6.85).
+template <bool DEEP>
+__global__ void __launch_bounds__(128, DEEP ? 6 : 5) k_render_packets(FrameArgs a) {
+    __shared__ ApproxTables tab;
+    load_tables(tab);
+    FramePaths<false> P{a, (a.w + 15u) / 16u, (a.h + 3u) / 4u, 0u};
+    bool ok = group_refill<DEEP ? 1 : 2>(P, tab);
+    if (!ok) atomicOr(a.err, kErrStackOverflow);
+}
+
 // After k_render_refill: a group whose 8 lanes all hit an emitter at bounce 0
 // leaves the reference's path loop before its gbuffer values are taken
 // (renderer.rs:413-468), so its gbuffer words are 0.
@@ -834,6 +877,14 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
     }
     cudaError_t e = cudaMemsetAsync(err + 1, 0, 4, st);  // packet counter
     if (e != cudaSuccess) return e;
+    if (!counters) {
+        uint32_t blocks = (uint32_t)num_sms() * kPacketBlocksPerSm, need = (n + 127u) / 128u;
+        if (blocks > need) blocks = need;
+        SoaRays src{s.nodes, s.wide, s.geom, rays, n, far_dist, t_out, tri_out, nullptr};
+        if (s.depth > 40) k_intersect_packets<1><<<blocks, 128, 0, st>>>(src, err + 1, err);
+        else k_intersect_packets<2><<<blocks, 128, 0, st>>>(src, err + 1, err);
+        return cudaGetLastError();
+    }
     if (block == 0) block = 128;
     if (blocks_per_sm == 0) blocks_per_sm = 8;
     uint32_t need = ((n + 7u) & ~7u) / block + 1u;
@@ -896,7 +947,12 @@ cudaError_t launch_render(const DeviceScene& s, const DeviceCamera& cam, uint32_
         uint32_t need = (units * 8 + block - 1) / block;
         uint32_t blocks = (uint32_t)num_sms() * 16u;
         if (blocks > need) blocks = need;
-        if (packet) k_render_group<true><<<blocks, block, 0, st>>>(a);
+        if (packet && !debug) {
+            const bool deep = s.depth > 40;
+            blocks = std::min((uint32_t)num_sms() * (deep ? 6u : 5u), (units * 8u + 127u) / 128u);
+            if (deep) k_render_packets<true><<<blocks, 128, 0, st>>>(a);
+            else k_render_packets<false><<<blocks, 128, 0, st>>>(a);
+        } else if (packet) k_render_group<true><<<blocks, block, 0, st>>>(a);
         else k_render_group<false><<<blocks, block, 0, st>>>(a);
     }
     return cudaGetLastError();

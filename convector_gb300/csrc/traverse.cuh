@@ -98,36 +98,38 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // A ray against a wide record in select form: the near and far plane of each
 // axis are picked by the sign of the ray's reciprocal (box_test_sel), by address,
 // so that no select is spent on them, and the four boxes' distances to them take
-// two planes per instruction (packed FP32, sm_100; the negated origin is added,
-// which is the same operation). t: entry distance of each slot's box if it is
-// hit, +inf if not; tc: entry distances of the pair's own two boxes.
+// two planes per instruction (packed FP32, sm_100; the negated origin `no` is
+// added, which is the same operation). t, e: entry and exit distance of each
+// slot's box; tc: entry distances of the pair's own two boxes.
 //
 // The axes are joined by max3 and min3. They differ from the x86 min and max
 // only where the result is a zero (of two tied zeros x86 takes the later
-// operand, max3 +0 and min3 -0), and where no exit distance is zero, a ray that
-// hits a grandchild's box hits the child's. Where any of the results is zero (an
-// origin on a bound plane; rare), exact() takes the pair records and the x86
-// form for this step. The products of the results show it (0, or NaN from
-// inf * 0; an underflow only costs time).
-struct WideT {
-    float t[4], tc0, tc1;
+// operand, max3 +0 and min3 -0); and where no exit distance is zero, a ray that
+// hits a grandchild's box hits the child's. `zero` is set where one of the results
+// is zero (an origin on a bound plane; rare): the step is then to be decided from
+// the pair records in the x86 form. The products of the results show it (0, or
+// NaN from inf * 0; an underflow only costs time).
+struct WidePlanes {
+    float t[4], e[4], tc0, tc1;
     uint4 r;
-    __device__ __forceinline__ WideT(const float4* __restrict__ nodes, const float4* __restrict__ wide, uint32_t ref,
-                                     F3 no, F3 inv) {
-        const float4* w = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(wide) + (size_t)ref * 2);
-        const char* wb = reinterpret_cast<const char*>(w);
+    bool zero;
+    __device__ __forceinline__ WidePlanes(const float4* __restrict__ wide, uint32_t ref, F3 no, F3 inv) {
+        const char* w = reinterpret_cast<const char*>(wide) + (size_t)ref * 2;
         auto ld = [](const char* p) { return __ldg(reinterpret_cast<const float4*>(p)); };
         const int sx = inv.x > 0.0f ? 0 : 16, sy = inv.y > 0.0f ? 0 : 16, sz = inv.z > 0.0f ? 0 : 16;
-        const float4 nx4 = ld(wb + sx), fx4 = ld(wb + 16 - sx), ny4 = ld(wb + 32 + sy), fy4 = ld(wb + 48 - sy),
-                     nz4 = ld(wb + 64 + sz), fz4 = ld(wb + 80 - sz);
-        r = __ldg(reinterpret_cast<const uint4*>(w + 6));
+        const float4 nx4 = ld(w + sx), fx4 = ld(w + 16 - sx), ny4 = ld(w + 32 + sy), fy4 = ld(w + 48 - sy),
+                     nz4 = ld(w + 64 + sz), fz4 = ld(w + 80 - sz);
+        r = __ldg(reinterpret_cast<const uint4*>(w + 96));
         auto dist = [](float4 v, float n, float i, float* out) {
             const float2 n2 = make_float2(n, n), i2 = make_float2(i, i);
             const float2 a = __fmul2_rn(__fadd2_rn(make_float2(v.x, v.y), n2), i2);
             const float2 b = __fmul2_rn(__fadd2_rn(make_float2(v.z, v.w), n2), i2);
-            out[0] = a.x; out[1] = a.y; out[2] = b.x; out[3] = b.y;
+            out[0] = a.x;
+            out[1] = a.y;
+            out[2] = b.x;
+            out[3] = b.y;
         };
-        float nx[4], ny[4], nz[4], fx[4], fy[4], fz[4], e[4];
+        float nx[4], ny[4], nz[4], fx[4], fy[4], fz[4];
         dist(nx4, no.x, inv.x, nx);
         dist(ny4, no.y, inv.y, ny);
         dist(nz4, no.z, inv.z, nz);
@@ -142,12 +144,26 @@ struct WideT {
         tc0 = max3(fminf(nx[0], nx[1]), fminf(ny[0], ny[1]), fminf(nz[0], nz[1]));
         tc1 = max3(fminf(nx[2], nx[3]), fminf(ny[2], ny[3]), fminf(nz[2], nz[3]));
         const float p0 = (t[0] * e[0]) * (t[1] * e[1]) * tc0, p1 = (t[2] * e[2]) * (t[3] * e[3]) * tc1;
-        if (__builtin_expect(!(fabsf(p0) > 0.0f && fabsf(p1) > 0.0f), 0)) {
+        zero = !(fabsf(p0) > 0.0f && fabsf(p1) > 0.0f);
+    }
+};
+// The decisions of one ray on a wide record. t: entry distance of each slot's box
+// if it is hit, +inf if not.
+struct WideT {
+    float t[4], tc0, tc1;
+    uint4 r;
+    __device__ __forceinline__ WideT(const float4* __restrict__ nodes, const float4* __restrict__ wide, uint32_t ref,
+                                     F3 no, F3 inv) {
+        const WidePlanes p(wide, ref, no, inv);
+        r = p.r;
+        if (__builtin_expect(p.zero, 0)) {
             exact(nodes, ref, f3(-no.x, -no.y, -no.z), inv);
         } else {
             const float inf = __int_as_float(0x7f800000);
+            tc0 = p.tc0;
+            tc1 = p.tc1;
 #pragma unroll
-            for (int k = 0; k < 4; k++) t[k] = (e[k] >= t[k]) & (e[k] > 0.0f) ? t[k] : inf;
+            for (int k = 0; k < 4; k++) t[k] = (p.e[k] >= p.t[k]) & (p.e[k] > 0.0f) ? p.t[k] : inf;
         }
     }
     // This step from the pair records: the pair's boxes, then those of its

@@ -72,18 +72,22 @@ def test_query_equals_oracle(gpu, orc, kind, n, far):
         assert (t.view(np.uint32) == ot.view(np.uint32)).all()
 
 
-@pytest.mark.parametrize("kind", ["plain", "large leaves", "not nested"])
-@pytest.mark.parametrize("refill", ["REFILL_ALL", "REFILL_NONE"])
-def test_frame_equals_oracle(gpu, orc, kind, refill):
+@pytest.mark.parametrize("kind", ["plain", "large leaves", "not nested", "loose"])
+@pytest.mark.parametrize("form", ["REFILL_ALL", "REFILL_NONE", "packets"])
+@pytest.mark.parametrize("w,h", [(83, 45), (1, 1), (17, 5)])
+def test_frame_equals_oracle(gpu, orc, kind, form, w, h):
     b, nodes = _scene_arrays(gpu, kind)
     b.nodes = nodes
     scene, osc = gpu.Scene(b), orc.OracleScene(b.triangles, nodes)
     # the eye on a box corner of the tree, so that camera rays meet tied zeros
     f = nodes.view(np.float32)
     scenes.default_camera(scene.camera, eye=tuple(float(v) for v in f[4, 3:6]), target=(0.0, 1.0, -2.0))
-    r = gpu.Renderer(scene, 83, 45, traversal=gpu.TRAVERSE_SINGLE, refill_mode=getattr(gpu, refill))
+    single = form != "packets"
+    r = gpu.Renderer(scene, w, h, traversal=gpu.TRAVERSE_SINGLE if single else gpu.TRAVERSE_PACKET,
+                     refill_mode=getattr(gpu, form) if single else gpu.REFILL_AFTER_CAMERA)
     rgba, gb = r.render_frame_u8(9)
-    orgba, ogb, ocol, orays = osc.render(scene.camera.as_array(), 83, 45, 9, rng_order=orc.RNG_GROUP, traversal=1)
+    orgba, ogb, ocol, orays = osc.render(scene.camera.as_array(), w, h, 9, rng_order=orc.RNG_GROUP,
+                                         traversal=int(single))
     assert (rgba == orgba).all() and (gb == ogb).all()
     assert (r.read_frame_f32().view(np.uint32) == ocol.view(np.uint32)).all()
     assert r.stats()[0] == orays
