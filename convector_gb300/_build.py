@@ -24,7 +24,7 @@ PROBE_LIB = os.path.join(PKG, "lib", "libconvector_l2probe.so")
 
 CU_SOURCES = ["kernels.cu", "wavefront.cu", "engine.cu", "capi.cu", "noalloc.cu", "postprocess.cu", "bvh_build.cu"]
 CPP_SOURCES = ["host_scene.cpp"]
-HEADERS = ["x86sem.cuh", "layout.cuh", "traverse.cuh", "shade.cuh", "path_refill.cuh", "packet_refill.cuh",
+HEADERS = ["x86sem.cuh", "layout.cuh", "traverse.cuh", "shade.cuh", "path_refill.cuh", "packet_refill.cuh", "packet_warp.cuh",
            "kernels.h", "internal.h",
            "x86_approx_tables.h", "wavefront.cuh", "engine.h", "device_guard.cuh"]
 

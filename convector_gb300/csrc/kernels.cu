@@ -7,6 +7,7 @@
 
 #include "kernels.h"
 #include "packet_refill.cuh"
+#include "packet_warp.cuh"
 #include "path_refill.cuh"
 #include "shade.cuh"
 
@@ -755,6 +756,120 @@ __global__ void __launch_bounds__(128, 1) k_render_patch(FrameArgs a) {
     if (k == 0 && v) atomicAdd(a.rays, v);
 }
 
+// Patch order in packet traversal: W warps per patch, one packet per warp
+// (packet_warp.cuh). A patch is one chain: a group's generator state depends on
+// how many bounces every group before it took. But the generator jumps to any
+// state (after n draws it is s * f^n mod 2^64), so the warps of a round render
+// the next groups at once, each from the state it has if the groups before it in
+// the round take the patch's most frequent bounce count. The groups up to the
+// first wrong guess are right and are stored; the others are rendered again.
+// Where guesses miss, a round takes as many groups as the last one confirmed and
+// one more.
+//
+// The frame's time is that of its slowest patches (the room's slowest takes four
+// times the mean): their rays stay inside and nearly every group takes all five
+// bounces (125 of 128), so guesses hold where they matter. Room 1280x736: one
+// octet per patch 16.6 ms, one warp per patch 12.0, two warps with guesses 7.8,
+// four 5.7, eight 6.5 (64 registers, 4 blocks per SM; 7.5 with 3), sixteen 10.5:
+// idle warps keep other patches' blocks off the SM. Icosphere 26.8, 18.2, 12.6,
+// 12.1, 15.8, 23.5 ms. 6 blocks of 4 warps per SM hold the frame's 920 patches
+// at once (4, 5, 7, 8 blocks: 5.7, 5.6, 5.9, 6.4 and 14.2, 13.6, 13.2, 13.7 ms).
+constexpr int kPatchWarps = 4;
+template <int W>
+__global__ void __launch_bounds__(32 * W, 24 / W) k_render_patch_warp(FrameArgs a) {
+    __shared__ ApproxTables tab;
+    __shared__ WarpStack stacks[W];
+    __shared__ int taken[2][W];  // by parity of the round: bounces of each warp's group
+    load_tables(tab);
+    const uint32_t lane = threadIdx.x & 31u, k = lane & 7u;
+    const int wid = (int)(threadIdx.x >> 5);
+    const uint32_t ph = (a.h + a.patch - 1u) / a.patch;
+    const uint32_t hb = a.patch / 4u, total = a.patch / 16u * hb * 8u;  // 16x4 blocks up a patch, groups of a patch
+    const uint32_t pi = blockIdx.x;
+    const uint32_t x0 = a.patches ? a.patches[2 * pi] : (pi / ph) * a.patch;
+    const uint32_t y0 = a.patches ? a.patches[2 * pi + 1] : (pi % ph) * a.patch;
+    LaneRng rng;
+    rng.seed(x0, y0, a.frame, (int)k);
+    const uint64_t f = rng.f, f2 = f * f, f4 = f2 * f2, f6 = f4 * f2, f8 = f4 * f4, f16 = f8 * f8;
+    auto group_factor = [&](int bounces) {
+        uint64_t r = f;
+        for (int i = 0; i < bounces; i++) r *= f6;
+        return r;
+    };
+    // Confirmed: the state before group `done` (before its block's jitter draws
+    // if it is the block's first), and before its block's jitter draws.
+    uint64_t state = rng.s, block = rng.s;
+    uint32_t done = 0, rays = 0;
+    int width = 1, guess = 5, parity = 0;
+    uint64_t seen = 0;  // how often each bounce count was confirmed, 8 bits each
+    bool ok = true;
+    while (done < total) {
+        const int n = (int)min((uint32_t)width, total - done);
+        PixelOut p;
+        uint32_t px = 0, py = 0, r = 0;
+        bool fits = true;
+        if (wid < n) {
+            const uint32_t mine = done + (uint32_t)wid;
+            const uint64_t step = group_factor(guess);
+            uint64_t s = state, b = block;
+            for (uint32_t i = done; i < mine; i++) {
+                if ((i & 7u) == 0u) {
+                    b = s;
+                    s *= f16;
+                }
+                s *= step;
+            }
+            if ((mine & 7u) == 0u) {
+                b = s;
+                s *= f16;
+            }
+            const int g = (int)(mine & 7u);
+            for (int i = 0; i < g; i++) b *= f;
+            auto draw = [&](uint64_t v) { return unit_from(rng.hi ? (uint32_t)(v >> 32) : (uint32_t)v); };
+            const uint32_t xb = x0 + (mine >> 3) / hb * 16u, yb = y0 + (mine >> 3) % hb * 4u;
+            float x, y, scale;
+            block_coord(a.w, a.h, xb, yb, g, (int)k, &x, &y, &scale);
+            x = fmaf(draw(b), scale, x);
+            y = fmaf(draw(b * f8), scale, y);
+            rng.s = s;
+            int bounces;
+            fits = render_pixels_warp(a.s, a.cam, x, y, rng, tab, stacks[wid], p, r, bounces);
+            px = xb + 4u * (uint32_t)(g >> 1) + (k & 3u);
+            py = yb + 2u * (uint32_t)(g & 1) + (k >> 2);
+            if (lane == 0u) taken[parity][wid] = bounces;
+        }
+        __syncthreads();
+        // The groups whose predecessors of this round all took what was guessed.
+        int valid = 1;
+        while (valid < n && taken[parity][valid - 1] == guess) valid++;
+        if (wid < valid) {
+            ok &= fits;
+            if (lane < 8u) {
+                store_pixel(a, px, py, p);
+                rays += r;
+            }
+        }
+        for (int i = 0; i < valid; i++) {
+            if (((done + (uint32_t)i) & 7u) == 0u) {
+                block = state;
+                state *= f16;
+            }
+            const int t = taken[parity][i];
+            state *= group_factor(t);
+            if ((seen >> (8 * t) & 0xffu) >= 64u) seen = (seen >> 1) & 0x7f7f7f7f7f7full;
+            seen += 1ull << (8 * t);
+        }
+        done += (uint32_t)valid;
+        width = valid == n ? min(W, 2 * width) : min(W, valid + 1);
+        guess = 5;
+        for (int t = 4; t >= 0; t--)
+            if ((seen >> (8 * t) & 0xffu) > (seen >> (8 * guess) & 0xffu)) guess = t;
+        parity ^= 1;
+    }
+    if (!ok) atomicOr(a.err, kErrStackOverflow);
+    flush_rays(a, rays);
+}
+
 __global__ void k_resolve(const float* __restrict__ accum, uint32_t npx, float factor, uint32_t* __restrict__ rgba) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += gridDim.x * blockDim.x) {
         F3 c = f3(accum[3 * i] * factor, accum[3 * i + 1] * factor, accum[3 * i + 2] * factor);
@@ -940,7 +1055,8 @@ cudaError_t launch_render(const DeviceScene& s, const DeviceCamera& cam, uint32_
     if (patch_order) {
         uint32_t units = patches ? n_patches : ((w + patch - 1) / patch) * ((h + patch - 1) / patch);
         uint32_t blocks = (units * 32 + block - 1) / block;  // one warp per patch
-        if (packet) k_render_patch<true><<<blocks, block, 0, st>>>(a);
+        if (packet && !debug) k_render_patch_warp<kPatchWarps><<<units, 32 * kPatchWarps, 0, st>>>(a);
+        else if (packet) k_render_patch<true><<<blocks, block, 0, st>>>(a);
         else k_render_patch<false><<<blocks, block, 0, st>>>(a);
     } else {
         uint32_t units = ((w + 15) / 16) * ((h + 3) / 4) * 8;

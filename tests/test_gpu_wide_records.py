@@ -73,7 +73,7 @@ def test_query_equals_oracle(gpu, orc, kind, n, far):
 
 
 @pytest.mark.parametrize("kind", ["plain", "large leaves", "not nested", "loose"])
-@pytest.mark.parametrize("form", ["REFILL_ALL", "REFILL_NONE", "packets"])
+@pytest.mark.parametrize("form", ["REFILL_ALL", "REFILL_NONE", "packets", "patches"])
 @pytest.mark.parametrize("w,h", [(83, 45), (1, 1), (17, 5)])
 def test_frame_equals_oracle(gpu, orc, kind, form, w, h):
     b, nodes = _scene_arrays(gpu, kind)
@@ -82,11 +82,12 @@ def test_frame_equals_oracle(gpu, orc, kind, form, w, h):
     # the eye on a box corner of the tree, so that camera rays meet tied zeros
     f = nodes.view(np.float32)
     scenes.default_camera(scene.camera, eye=tuple(float(v) for v in f[4, 3:6]), target=(0.0, 1.0, -2.0))
-    single = form != "packets"
-    r = gpu.Renderer(scene, w, h, traversal=gpu.TRAVERSE_SINGLE if single else gpu.TRAVERSE_PACKET,
+    single = form.startswith("REFILL")
+    order = "RNG_PATCH" if form == "patches" else "RNG_GROUP"
+    r = gpu.Renderer(scene, w, h, rng_order=getattr(gpu, order), traversal=gpu.TRAVERSE_SINGLE if single else gpu.TRAVERSE_PACKET,
                      refill_mode=getattr(gpu, form) if single else gpu.REFILL_AFTER_CAMERA)
     rgba, gb = r.render_frame_u8(9)
-    orgba, ogb, ocol, orays = osc.render(scene.camera.as_array(), w, h, 9, rng_order=orc.RNG_GROUP,
+    orgba, ogb, ocol, orays = osc.render(scene.camera.as_array(), w, h, 9, rng_order=getattr(orc, order),
                                          traversal=int(single))
     assert (rgba == orgba).all() and (gb == ogb).all()
     assert (r.read_frame_f32().view(np.uint32) == ocol.view(np.uint32)).all()
@@ -126,3 +127,21 @@ def test_scales_equal_oracle(gpu, orc, scale):
         ot, otri = osc.intersect(o, d, far=1.0e30, mode=traversal)
         assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
         assert (t.view(np.uint32) == ot.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("width", [16, 48, 64])
+def test_patch_widths_equal_oracle(gpu, orc, width):
+    """Patches of other widths, on a view whose groups end after any number of
+    bounces (what a round guesses from the groups before is then often wrong)."""
+    b, nodes = _scene_arrays(gpu, "plain")
+    scene, osc = gpu.Scene(b), orc.OracleScene(b.triangles, nodes)
+    scenes.default_camera(scene.camera)
+    w, h = 150, 70
+    origins = [(0, 0), (64, 4), (144, 60), (96, 12)]
+    r = gpu.Renderer(scene, w, h)
+    rgba, gb = np.full((h, w), 7, np.uint32), np.full((h, w), 7, np.uint32)
+    r.render_patches_u8(width, origins, 5, rgba, gb)
+    orgba, ogb = np.full((h, w), 7, np.uint32), np.full((h, w), 7, np.uint32)
+    orays = osc.render_patches(scene.camera.as_array(), w, h, 5, width, origins, traversal=0, rgba=orgba, gbuf=ogb)
+    assert (rgba == orgba).all() and (gb == ogb).all()
+    assert r.stats()[0] == orays
