@@ -656,7 +656,7 @@ static int32_t run_frame(cvx_renderer* r, uint32_t frame, bool accumulate, uint3
                      r->cfg.rng_order == CVX_RNG_PATCH, accumulate ? nullptr : r->d_rgba, r->d_gbuf, r->d_color,
                      accumulate ? r->d_accum : nullptr, r->d_rays, r->d_err, r->cfg.block_size, r->debug,
                      r->stream, 32, nullptr, 0,
-                     path_refill_frames(r->cfg.refill_mode, r->scene->depth) ? r->d_group_em : nullptr),
+                     path_refill_frames(r->cfg.refill_mode, r->scene->depth, npx) ? r->d_group_em : nullptr),
        "render launch");
     CK(cudaEventRecord(r->e1, r->stream), "event");
     if (rgba) CK(cudaMemcpyAsync(rgba, r->d_rgba, npx * 4, cudaMemcpyDeviceToHost, r->stream), "copy colour");

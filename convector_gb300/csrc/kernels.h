@@ -41,17 +41,24 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
 // Single-launch form of single-ray frames and waves in the per-group RNG
 // order: paths per lane with ray refill (k_render_refill, k_wave_refill), or
 // one octet per 8-pixel group (k_render_group, k_wave_fused). CVX_REFILL_ALL
-// and CVX_REFILL_NONE choose; by default the depth of the frame's scene
-// decides, and for a wave whether at least half of its groups belong to scenes
-// that deep. Measured at 1280x736 (octet against refill, ms per frame): the
-// 19-level room 0.82 / 0.73, the 28-level icosphere 1.87 / 1.45, the 70-level
-// tube 5.36 / 3.14; 256 scenes of 11 to 23 levels (median 16), batched: 53 / 66
-// ms, one at a time: 2,808 / 2,546 Mrays/s. Refill wins clearly from the
-// icosphere's depth on; the shallow open scenes, whose paths are mostly one or
-// two rays, keep warps of neighbouring camera rays together.
+// and CVX_REFILL_NONE choose. By default the tree's depth and the frame's size
+// decide: refill keeps lanes busy where paths are long and many, the octets keep
+// warps of neighbouring camera rays together, and start a frame that does not
+// fill the GPU sooner. Measured, octet against refill, us per frame:
+//                            320x184    640x368    900x516     1280x736    1920x1080
+//   tube, 70 levels         1018/964  1446/1255  2099/1508   3506/2216   6909/4062
+//   icosphere, 28 levels     248/280    450/418    747/610   1365/1018   2834/1991
+//   room, 19 levels          152/187    219/242    340/301     623/481    1287/932
+//   open scene, 21 levels    124/152    152/187    198/230     286/312     528/543
+//   open scene, 16 levels      73/91     88/109    102/131     127/153     191/240
+// (480x276: icosphere 331/345.) The open scene of 21 levels loses 3-9 % by the
+// line at 18 levels, a closed room gains 13-40 %; nothing in the tree tells them
+// apart. For a wave, whether at least half of its groups belong to scenes of
+// kRefillMinDepth levels (32 open scenes of 11 to 20 levels, 6.4/7.9 ms).
 constexpr uint32_t kRefillMinDepth = 25;
-inline bool path_refill_frames(uint32_t refill_mode, uint32_t depth) {
-    return refill_mode == CVX_REFILL_ALL || (refill_mode == CVX_REFILL_AFTER_CAMERA && depth >= kRefillMinDepth);
+inline bool path_refill_frames(uint32_t refill_mode, uint32_t depth, uint64_t pixels) {
+    if (refill_mode != CVX_REFILL_AFTER_CAMERA) return refill_mode == CVX_REFILL_ALL;
+    return depth > 40 || (depth >= kRefillMinDepth && pixels >= 160000) || (depth >= 18 && pixels >= 400000);
 }
 // deep_groups of a wave's groups belong to scenes of kRefillMinDepth levels or more.
 inline bool path_refill_wave(uint32_t refill_mode, uint32_t deep_groups, uint32_t groups) {

@@ -241,9 +241,11 @@ enum { CVX_MODE_MEGAKERNEL = 0, CVX_MODE_WAVEFRONT = 1, CVX_MODE_AUTO = 2 };
  * group per octet through all its bounces; CVX_REFILL_ALL gives each lane one
  * path at a time, refilled ray by ray (a lane whose ray is finished shades it
  * together with the others of its warp that are, then traces the next);
- * CVX_REFILL_AFTER_CAMERA (default) takes the second for scenes of 25 levels
- * and more (for a wave of a batch or server: when at least half of its groups
- * belong to such scenes), the first below. The image is the same either way. */
+ * CVX_REFILL_AFTER_CAMERA (default) takes the second for deep scenes and large
+ * frames: above 40 levels, from 25 levels and 160,000 pixels, and from 18 levels
+ * and 400,000 pixels (for a wave of a batch or server: when at least half of its
+ * groups belong to scenes of 25 levels and more), the first below. The image is
+ * the same either way. */
 enum { CVX_REFILL_AFTER_CAMERA = 0, CVX_REFILL_ALL = 1, CVX_REFILL_NONE = 2 };
 
 typedef struct cvx_render_config {
