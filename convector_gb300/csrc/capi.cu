@@ -453,6 +453,39 @@ int32_t cvx_intersect_nearest_device(cvx_scene* s, const float* rays, uint32_t n
     return CVX_OK;
 }
 
+// The whole call of a small host query in one launch: the kernel reads the
+// caller's rays and writes the caller's hits and a page-locked status word over
+// the CPU-GPU link. Two pageable copies, a copied status and the waits for three
+// streams were half of such a call (1 ray: 63 -> 28 us, 1021 rays of the
+// icosphere in packets 131 -> 78 us with the kernel's own gain, 65,536 rays 343 ->
+// 261 us). From about 200,000 rays on the copies win (262,144 rays, single, of the
+// icosphere 887 and 842 us; 524,288: 1721 and 1774).
+constexpr uint32_t kQueryChunks = 4;  // of the pipeline below, each with a status word
+constexpr uint32_t kDirectHostRays = 131072;
+static int32_t intersect_direct(cvx_scene* s, const float* ox, const float* oy, const float* oz, const float* dx,
+                                const float* dy, const float* dz, uint32_t n, float far_dist, uint32_t traversal,
+                                float* t_out, int32_t* tri_out) {
+    if (!s->h_qerr) CK(cudaHostAlloc((void**)&s->h_qerr, 8 * kQueryChunks, cudaHostAllocDefault), "cudaHostAlloc status");
+    cudaStream_t& q = s->qstreams[0];
+    if (!q) CK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate");
+    // First touch on the CPU: the device's own faults on fresh pages are slow.
+    for (size_t i = 0; i < (size_t)n + 1023; i += 1024) {
+        const size_t at = std::min<size_t>(i, n - 1u);
+        reinterpret_cast<volatile float*>(t_out)[at] = 0.0f;
+        reinterpret_cast<volatile int32_t*>(tri_out)[at] = 0;
+    }
+    *reinterpret_cast<volatile uint32_t*>(s->h_qerr) = 0u;
+    const RayCols cols{{ox, oy, oz, dx, dy, dz}};
+    StreamSync sync(q);
+    CK(launch_intersect(s->view(), cols, n, far_dist, traversal == CVX_TRAVERSE_PACKET, t_out, tri_out, nullptr,
+                        s->h_qerr, 0, s->blocks_per_sm, q, s->query_stack),
+       "intersect launch");
+    CK(cudaStreamSynchronize(q), "intersect");
+    if (*reinterpret_cast<volatile uint32_t*>(s->h_qerr))
+        return set_error(CVX_ERR_DEVICE, "traversal stack overflow reported by the kernel");
+    return CVX_OK;
+}
+
 int32_t cvx_intersect_nearest(cvx_scene* s, const float* ox, const float* oy, const float* oz, const float* dx,
                               const float* dy, const float* dz, uint32_t n, float far_dist, uint32_t traversal,
                               float* t_out, int32_t* tri_out) {
@@ -467,6 +500,14 @@ int32_t cvx_intersect_nearest(cvx_scene* s, const float* ox, const float* oy, co
     // link as it consumes them (a warp stages each batch of 32 rays one batch
     // ahead), so the transfer overlaps traversal and no ray copy is made.
     const bool in_place = s->reads_host_in_place();
+    // (A caller may let its hits overwrite its rays: then they are copied out.)
+    auto overlap = [n](const void* a, const void* b) {
+        const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b, len = (uintptr_t)n * 4u;
+        return x < y + len && y < x + len;
+    };
+    bool apart = true;
+    for (const float* c : {ox, oy, oz, dx, dy, dz}) apart = apart && !overlap(c, t_out) && !overlap(c, tri_out);
+    if (in_place && apart && n <= kDirectHostRays) return intersect_direct(s, ox, oy, oz, dx, dy, dz, n, far_dist, traversal, t_out, tri_out);
     if (s->scratch_n < n || (!in_place && !s->d_rays)) {
         cudaFree(s->d_rays);
         cudaFree(s->d_t);
@@ -488,7 +529,7 @@ int32_t cvx_intersect_nearest(cvx_scene* s, const float* ox, const float* oy, co
     // remain to overlap); 1 when any buffer is pageable, as the driver stages
     // each pageable copy through its own buffers and every extra chunk adds
     // one such round trip.
-    constexpr uint32_t kMaxChunks = 4, kMinChunk = 1u << 19;
+    constexpr uint32_t kMaxChunks = kQueryChunks, kMinChunk = 1u << 19;
     if (!s->d_qerr && (st = dalloc(&s->d_qerr, 2 * kMaxChunks, "status"))) return st;
     if (!s->h_qerr) {
         CK(cudaHostAlloc((void**)&s->h_qerr, 8 * kMaxChunks, cudaHostAllocDefault), "cudaHostAlloc status");

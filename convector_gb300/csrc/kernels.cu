@@ -344,6 +344,64 @@ __global__ void __launch_bounds__(128, kPacketBlocksPerSm) k_intersect_packets(S
     if (!ok) atomicOr(err, kErrStackOverflow);
 }
 
+// Queries of up to kDirectRays rays in the default launch shape, whose time is
+// that of their longest rays: no ray supply to set up, no counter to reset, no
+// pass over deferred rays. Device time with the launch, before (k_intersect_
+// packets, k_intersect_refill and its pass) -> one packet per warp / one ray per
+// lane, us at 1021, 65,536, 262,144, 524,288 rays: packets, 28-level icosphere 93
+// -> 68, 189 -> 130, 331 -> 270, 421 -> 449; single rays 69 -> 54, 121 -> 95, 145
+// -> 124, 181 -> 182; packets, 19-level room 59 -> 46, 94 -> 63, 165 -> 123, 212 ->
+// 198; 70-level tube 241 -> 163, 421 -> 255, 640 -> 497, 839 -> 787; single rays,
+// room 52 -> 42, 68 -> 51, 91 -> 70, 112 -> 102, tube 234 -> 186, 218 -> 165, 312
+// -> 287, 419 -> 470. `err` may be page-locked host memory (it is stored to).
+constexpr uint32_t kDirectRays = 262144;
+__global__ void __launch_bounds__(64) k_intersect_warp(DeviceScene s, const RayCols rays, uint32_t n, float far_dist,
+                                                       float* __restrict__ t_out, int32_t* __restrict__ tri_out,
+                                                       uint32_t* err) {
+    __shared__ WarpStack stacks[2];
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const uint32_t i = (blockIdx.x * 2u + wid) * 8u + (lane & 7u);
+    if ((i & ~7u) >= n) return;
+    const bool active = i < n;
+    const uint32_t src = active ? i : (i & ~7u);
+    const F3 o = f3(__ldg(rays.c[0] + src), __ldg(rays.c[1] + src), __ldg(rays.c[2] + src));
+    const F3 d = f3(__ldg(rays.c[3] + src), __ldg(rays.c[4] + src), __ldg(rays.c[5] + src));
+    Hit h{far_dist, 0.0f, 0.0f, -1};
+    const bool ok = traverse_warp(s, o, d, active, h, g_tables, stacks[wid]);
+    if (active && lane < 8u) {
+        t_out[i] = h.t;
+        tri_out[i] = h.tri;
+    }
+    if (!ok) *reinterpret_cast<volatile uint32_t*>(err) = kErrStackOverflow;
+}
+
+__global__ void __launch_bounds__(32) k_intersect_lanes(DeviceScene s, const RayCols rays, uint32_t n, float far_dist,
+                                                        float* __restrict__ t_out, int32_t* __restrict__ tri_out,
+                                                        uint32_t* err) {
+    const uint32_t i = blockIdx.x * 32u + threadIdx.x;
+    if (i >= n) return;
+    const F3 o = f3(__ldg(rays.c[0] + i), __ldg(rays.c[1] + i), __ldg(rays.c[2] + i));
+    const F3 d = f3(__ldg(rays.c[3] + i), __ldg(rays.c[4] + i), __ldg(rays.c[5] + i));
+    RefillRay ray;
+    uint2 local_stack[kStackSlots];
+    LocalStack stack{local_stack};
+    ray.top = make_uint2(0u, 0u);
+    ray.start(o, d, far_dist, s.nodes, s.wide, s.geom, g_tables);
+    bool overflow = false;
+    if (s.wide && select_form_ray(o, ray.inv)) {
+        do {
+            ray.walk(stack, overflow);
+            ray.walk(stack, overflow);
+        } while (!ray.test_leaf());
+    } else {
+        while (!ray.step<false, false>(stack, overflow)) {
+        }
+    }
+    t_out[i] = ray.h.t;
+    tri_out[i] = ray.h.tri;
+    if (overflow) *reinterpret_cast<volatile uint32_t*>(err) = kErrStackOverflow;
+}
+
 // After k_intersect_refill<SELECT>: the rays it left (index word kDeferredRay:
 // a reciprocal infinite or below 0.75 in magnitude) with the x86-form slab
 // test. Such rays are rare (axis-parallel or very long directions), so the
@@ -960,6 +1018,13 @@ static void launch_select_stack(uint32_t shared, uint32_t blocks, const SoaRays&
 cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t n, float far_dist, bool packet,
                              float* t_out, int32_t* tri_out, uint32_t* counters, uint32_t* err, uint32_t block,
                              uint32_t blocks_per_sm, cudaStream_t st, uint32_t shared_stack) {
+    // Calls that do not fill the GPU several times over: one packet per warp, or
+    // one ray per lane, with nothing claimed (kDirectRays).
+    if (!counters && n <= kDirectRays && blocks_per_sm == 0 && shared_stack == kQueryStackShared) {
+        if (packet) k_intersect_warp<<<(n + 15u) / 16u, 64, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
+        else k_intersect_lanes<<<(n + 31u) / 32u, 32, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
+        return cudaGetLastError();
+    }
     if (!packet) {
         // persistent ray-refill kernel; err[1] is its ray counter
         cudaError_t e = cudaMemsetAsync(err + 1, 0, 4, st);

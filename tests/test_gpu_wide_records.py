@@ -66,10 +66,12 @@ def test_query_equals_oracle(gpu, orc, kind, n, far):
     scene, osc = gpu.Scene(b), orc.OracleScene(b.triangles, nodes)
     o, d = _rays(nodes, n, seed=n)
     for traversal in (gpu.TRAVERSE_SINGLE, gpu.TRAVERSE_PACKET):
-        t, tri = scene.intersect_nearest(o, d, far=far, traversal=traversal)
         ot, otri = osc.intersect(o, d, far=far, mode=traversal)
-        assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
-        assert (t.view(np.uint32) == ot.view(np.uint32)).all()
+        for blocks_per_sm in (0, 8):  # the small-query kernels, the persistent ones
+            scene.set_query_launch(blocks_per_sm)
+            t, tri = scene.intersect_nearest(o, d, far=far, traversal=traversal)
+            assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
+            assert (t.view(np.uint32) == ot.view(np.uint32)).all()
 
 
 @pytest.mark.parametrize("kind", ["plain", "large leaves", "not nested", "loose"])
@@ -107,10 +109,12 @@ def test_chains_equal_oracle(gpu, orc, pairs):
     d[2::5] *= np.float32(3.0)
     o[3::5] = o[3::5] * np.float32(1.0e25)   # origins beyond it
     for traversal in (gpu.TRAVERSE_SINGLE, gpu.TRAVERSE_PACKET):
-        t, tri = scene.intersect_nearest(o, d, traversal=traversal)
         ot, otri = osc.intersect(o, d, mode=traversal)
-        assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
-        assert (t.view(np.uint32) == ot.view(np.uint32)).all()
+        for blocks_per_sm in (0, 8):
+            scene.set_query_launch(blocks_per_sm)
+            t, tri = scene.intersect_nearest(o, d, traversal=traversal)
+            assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
+            assert (t.view(np.uint32) == ot.view(np.uint32)).all()
 
 
 @pytest.mark.parametrize("scale", [1.0e-4, 1.0, 1.0e16, 1.0e18])
@@ -145,3 +149,44 @@ def test_patch_widths_equal_oracle(gpu, orc, width):
     orays = osc.render_patches(scene.camera.as_array(), w, h, 5, width, origins, traversal=0, rgba=orgba, gbuf=ogb)
     assert (rgba == orgba).all() and (gb == ogb).all()
     assert r.stats()[0] == orays
+
+
+@pytest.mark.parametrize("n", [131071, 131072, 131073, 262143, 262144, 262145])
+def test_query_forms_agree_at_their_limits(gpu, n):
+    """Host and device queries on both sides of the direct forms' limits equal the copying, persistent one."""
+    import torch
+    b, _ = _scene_arrays(gpu, "plain")
+    scene = gpu.Scene(b)
+    o, d = scenes.random_rays(n, seed=n)
+    rays = torch.from_numpy(np.ascontiguousarray(np.concatenate([o.T, d.T]))).cuda()
+    t = torch.empty(n, dtype=torch.float32, device="cuda")
+    tri = torch.empty(n, dtype=torch.int32, device="cuda")
+    for traversal in (gpu.TRAVERSE_SINGLE, gpu.TRAVERSE_PACKET):
+        scene.set_query_launch(8)
+        scene.set_host_access(gpu.HOST_ACCESS_COPY)
+        ot, otri = scene.intersect_nearest(o, d, traversal=traversal)
+        scene.set_query_launch(0)
+        scene.set_host_access(gpu.HOST_ACCESS_AUTO)
+        ht, htri = scene.intersect_nearest(o, d, traversal=traversal)
+        scene.intersect_nearest_device(rays, t, tri, traversal=traversal)
+        torch.cuda.synchronize()
+        for a, c in ((ht, htri), (t.cpu().numpy(), tri.cpu().numpy())):
+            assert (c == otri).all() and (a.view(np.uint32) == ot.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("shift", [0, 5])
+def test_small_query_may_overwrite_its_rays(gpu, shift):
+    """Hits written over the ray columns, exactly or shifted, as any buffers of the C call may be."""
+    b, _ = _scene_arrays(gpu, "plain")
+    scene = gpu.Scene(b)
+    n = 3001
+    o, d = scenes.random_rays(n, seed=1)
+    t, tri = scene.intersect_nearest(o, d)
+    cols = [np.ascontiguousarray(a[:, k]) for a in (o, d) for k in range(3)]
+    buf = np.zeros(n + shift, np.float32)
+    buf[:n] = cols[0]
+    out_t, out_tri = buf[shift:], cols[4].view(np.int32)
+    ptr = [gpu._ptr(buf[:n])] + [gpu._ptr(c) for c in cols[1:]]
+    gpu._check(gpu.lib().cvx_intersect_nearest(scene._h, *ptr, n, 1.0e5, gpu.TRAVERSE_PACKET, gpu._ptr(out_t),
+                                               gpu._ptr(out_tri)))
+    assert (out_tri == tri).all() and (out_t.view(np.uint32) == t.view(np.uint32)).all()
