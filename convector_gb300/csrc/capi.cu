@@ -1,6 +1,7 @@
 // The device half of the C-ABI (include/convector_gpu.h): scene upload,
 // nearest-hit queries and frame rendering.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -97,6 +98,13 @@ bool cvx::injected_allocation_failure() {
     while (v >= 0)
         if (g_alloc_countdown.compare_exchange_weak(v, v - 1)) return v == 0;
     return false;
+}
+
+void cvx::touch_pages(void* p, size_t bytes) {
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* c = static_cast<char*>(p);
+    for (size_t i = 0; i < bytes; i += page) c[i] = 0;
+    if (bytes) c[bytes - 1] = 0;
 }
 
 struct cvx_scene {
@@ -469,11 +477,8 @@ static int32_t intersect_direct(cvx_scene* s, const float* ox, const float* oy, 
     cudaStream_t& q = s->qstreams[0];
     if (!q) CK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate");
     // First touch on the CPU: the device's own faults on fresh pages are slow.
-    for (size_t i = 0; i < (size_t)n + 1023; i += 1024) {
-        const size_t at = std::min<size_t>(i, n - 1u);
-        reinterpret_cast<volatile float*>(t_out)[at] = 0.0f;
-        reinterpret_cast<volatile int32_t*>(tri_out)[at] = 0;
-    }
+    touch_pages(t_out, (size_t)n * 4);
+    touch_pages(tri_out, (size_t)n * 4);
     *reinterpret_cast<volatile uint32_t*>(s->h_qerr) = 0u;
     const RayCols cols{{ox, oy, oz, dx, dy, dz}};
     StreamSync sync(q);
