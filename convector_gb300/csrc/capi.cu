@@ -705,6 +705,8 @@ static int32_t run_frame(cvx_renderer* r, uint32_t frame, bool accumulate, uint3
                      path_refill_frames(r->cfg.refill_mode, r->scene->depth, npx) ? r->d_group_em : nullptr),
        "render launch");
     CK(cudaEventRecord(r->e1, r->stream), "event");
+    if (rgba) touch_pages(rgba, npx * 4);
+    if (gbuf) touch_pages(gbuf, npx * 4);
     if (rgba) CK(cudaMemcpyAsync(rgba, r->d_rgba, npx * 4, cudaMemcpyDeviceToHost, r->stream), "copy colour");
     if (gbuf) CK(cudaMemcpyAsync(gbuf, r->d_gbuf, npx * 4, cudaMemcpyDeviceToHost, r->stream), "copy gbuffer");
     CK(cudaMemcpyAsync(&rays, r->d_rays, 8, cudaMemcpyDeviceToHost, r->stream), "copy counters");
@@ -900,6 +902,7 @@ int32_t cvx_accumulate_frames_f32(cvx_renderer* r, uint32_t first_frame, uint32_
         done += n;
     }
     CK(cudaEventRecord(r->e1, r->stream), "event");
+    if (gbuffer) touch_pages(gbuffer, npx * 4);
     if (gbuffer) CK(cudaMemcpyAsync(gbuffer, r->d_gbuf, npx * 4, cudaMemcpyDeviceToHost, r->stream), "copy gbuffer");
     CK(cudaMemcpyAsync(&rays, r->d_rays, 8, cudaMemcpyDeviceToHost, r->stream), "copy counters");
     CK(cudaMemcpyAsync(&err, r->d_err, 4, cudaMemcpyDeviceToHost, r->stream), "copy status");
@@ -917,6 +920,7 @@ int32_t cvx_resolve_u8(cvx_renderer* r, uint32_t n, uint32_t* rgba) {
     size_t npx = (size_t)r->w * r->h;
     StreamSync sync(r->stream);
     CK(launch_resolve(r->d_accum, (uint32_t)npx, 1.0f / (float)n, r->d_rgba, r->stream), "resolve launch");
+    touch_pages(rgba, npx * 4);
     CK(cudaMemcpyAsync(rgba, r->d_rgba, npx * 4, cudaMemcpyDeviceToHost, r->stream), "copy colour");
     CK(cudaStreamSynchronize(r->stream), "resolve");
     return CVX_OK;

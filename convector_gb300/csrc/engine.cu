@@ -368,6 +368,7 @@ extern "C" int32_t cvx_batch_render(cvx_batch* b, const cvx_view* views, uint32_
     ECK(cudaMemsetAsync(b->d_accum, 0, total * 12, b->stream), "clear accumulator");
     uint64_t rays = 0;
     float ms = 0.0f;
+    bool touched = rgba == nullptr;  // the images' pages, while the first wave runs
     WaveOutputs out{};
     out.accum = b->d_accum;
     // Sample s of every view goes into wave s; a wave's jobs are split by
@@ -382,6 +383,9 @@ extern "C" int32_t cvx_batch_render(cvx_batch* b, const cvx_view* views, uint32_
             float t[2] = {0.0f, 0.0f};
             int32_t st = b->fused.submit(jobs[0], out, b->stream2, false);
             if (!st) st = b->engine.submit(jobs[1], out, b->stream, false);
+            for (uint32_t i = 0; i < n && !touched; i++)
+                if (rgba[i]) touch_pages(rgba[i], (size_t)views[i].width * views[i].height * 4);
+            touched = true;
             int32_t st0 = b->fused.collect(b->stream2, &r[0], nullptr, &t[0]);
             int32_t st1 = b->engine.collect(b->stream, &r[1], nullptr, &t[1]);
             rays += r[0] + r[1];
@@ -782,6 +786,8 @@ struct cvx_server {
                     continue;
                 }
                 cudaEventRecord(fl[e].done, stream_of(e));
+                for (auto& q : start[e])  // the pages of the images this wave completes, while it runs
+                    if (q->host_rgba && q->next_sample + q->wave_k == q->r.spp) touch_pages(q->host_rgba, q->npx * 4);
                 fl[e].busy = true;
                 fl[e].reqs = std::move(start[e]);
                 if (n_busy++ == 0) busy_from = now();
