@@ -1,7 +1,10 @@
 // Shared host-side helpers of libconvector_gpu (not part of the C-ABI).
 #pragma once
 #include <cstdint>
+#include <memory>
+#include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/convector_gpu.h"
@@ -34,9 +37,26 @@ struct InterimNode {
 // TSAH factors for triangle counts 0..n (index 0 unused) and the constant
 // denominator, as the host build computes them.
 void tsah_tables(uint32_t n, std::vector<float>& x, std::vector<float>& t, float* y);
-// crystallize and statistics over an interim tree (same results as the host build).
-int32_t bvh_from_interim(const std::vector<InterimNode>& t, const std::vector<uint32_t>& order,
-                         const cvx_triangle* src, uint32_t n, cvx_bvh** out);
+// A vector whose resize() leaves plain data uninitialised (it is filled whole
+// right after).
+template <class T>
+struct NoInit : std::allocator<T> {
+    template <class U>
+    struct rebind {
+        using other = NoInit<U>;
+    };
+    NoInit() = default;
+    template <class U>
+    NoInit(const NoInit<U>&) {}
+    template <class U>
+    void construct(U* p) {
+        ::new ((void*)p) U;
+    }
+    template <class U, class... A>
+    void construct(U* p, A&&... a) {
+        ::new ((void*)p) U(std::forward<A>(a)...);
+    }
+};
 
 struct MeshTri {
     uint32_t v[3];
@@ -53,9 +73,9 @@ struct cvx_mesh {
 };
 
 struct cvx_bvh {
-    std::vector<cvx_bvh_node> nodes;
-    std::vector<cvx_triangle> triangles;  // BVH (leaf) order
-    std::vector<uint32_t> source_index;   // input index of each BVH-order triangle
+    std::vector<cvx_bvh_node, cvx::NoInit<cvx_bvh_node>> nodes;
+    std::vector<cvx_triangle, cvx::NoInit<cvx_triangle>> triangles;  // BVH (leaf) order
+    std::vector<uint32_t, cvx::NoInit<uint32_t>> source_index;  // input index of each BVH-order triangle
     float avg_area_ratio = 0.0f;
     float avg_tris_per_leaf = 0.0f;
     uint32_t depth = 0;
