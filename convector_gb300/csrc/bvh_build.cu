@@ -335,16 +335,9 @@ __device__ __forceinline__ unsigned long long ukey(const Refs& r, const uint32_t
 
 // One block sorts the positions of one (slot, axis) of at most kBlockSort
 // triangles; srt[axis][beg + rank] = position.
-__global__ void __launch_bounds__(1024) k_sort_block(const Tile* __restrict__ pairs, uint32_t n_pairs, Refs r,
-                                                     const uint32_t* __restrict__ order, uint32_t n,
-                                                     uint32_t* __restrict__ srt, uint32_t* err) {
-    __shared__ unsigned long long k[kBlockSort];
-    if (blockIdx.x >= n_pairs) return;
-    Tile pr = pairs[blockIdx.x];  // slot, axis, start = beg, len = cnt
-    if (pr.len > kBlockSort || pr.start + pr.len > n || pr.axis > 2) {
-        if (threadIdx.x == 0) atomicOr(err, 2u);
-        return;
-    }
+__device__ __forceinline__ void sort_pair(const Tile& pr, unsigned long long* k, const Refs& r,
+                                          const uint32_t* __restrict__ order, uint32_t n,
+                                          uint32_t* __restrict__ srt) {
     uint32_t m = 1;
     while (m < pr.len) m <<= 1;
     for (uint32_t i = threadIdx.x; i < m; i += blockDim.x)
@@ -369,7 +362,26 @@ __global__ void __launch_bounds__(1024) k_sort_block(const Tile* __restrict__ pa
         srt[(size_t)pr.axis * n + pr.start + i] = (uint32_t)k[i];
 }
 
-// Device-wide bitonic sort of one large (slot, axis) in `buf` (m a power of two).
+// The uniform split of every (slot, axis) that fell back and fits one block:
+// the sort, one block per slot and axis; the others return at once, which
+// costs less than the host's look at the modes and its list (a round trip and
+// three uploads per level).
+__global__ void __launch_bounds__(1024) k_sort_slots(const Slot* __restrict__ slots, uint32_t n_slots,
+                                                     const uint32_t* __restrict__ mode, Refs r,
+                                                     const uint32_t* __restrict__ order, uint32_t n,
+                                                     uint32_t* __restrict__ srt, uint32_t* err) {
+    __shared__ unsigned long long k[kBlockSort];
+    const uint32_t slot = blockIdx.x / 3u, axis = blockIdx.x % 3u;
+    if (slot >= n_slots || !mode[3 * slot + axis]) return;
+    const Slot sl = slots[slot];
+    if (sl.cnt > kBlockSort) return;  // sorted through global memory
+    if (sl.beg + sl.cnt > n) {
+        if (threadIdx.x == 0) atomicOr(err, 2u);
+        return;
+    }
+    sort_pair(Tile{slot, axis, sl.beg, sl.cnt}, k, r, order, n, srt);
+}
+
 __global__ void k_sort_fill(Tile pr, uint32_t m, Refs r, const uint32_t* __restrict__ order,
                             unsigned long long* __restrict__ buf) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -433,7 +445,24 @@ __global__ void k_axis_reset(const Tile* __restrict__ pairs, uint32_t n_pairs, B
         st.key[6 * g + 3 + c] = 0u;
     }
 }
+// k_axis_reset of the (slot, axis) pairs of k_sort_slots.
+__global__ void k_axis_reset_slots(const Slot* __restrict__ slots, uint32_t n_slots,
+                                   const uint32_t* __restrict__ mode, BinStats st) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t pair = i / kBins;
+    if (pair >= 3u * n_slots || !mode[pair] || slots[pair / 3u].cnt > kBlockSort) return;
+    st.count[i] = 0u;
+    for (int c = 0; c < 3; c++) {
+        st.key[6 * (size_t)i + c] = ~0u;
+        st.key[6 * (size_t)i + 3 + c] = 0u;
+    }
+}
+
+// slot_mode: `tiles` are the level's tiles (absolute starts), one axis per
+// blockIdx.y, of which the (slot, axis) pairs of k_sort_slots are taken; null:
+// tiles list (slot, axis, relative start) themselves.
 __global__ void __launch_bounds__(kTile) k_uniform_stats(const Tile* __restrict__ tiles, uint32_t n_tiles,
+                                                         const uint32_t* __restrict__ slot_mode,
                                                          const Slot* __restrict__ slots, uint32_t n_slots, Refs r,
                                                          const uint32_t* __restrict__ order, uint32_t n,
                                                          const uint32_t* __restrict__ srt, BinStats st,
@@ -447,6 +476,11 @@ __global__ void __launch_bounds__(kTile) k_uniform_stats(const Tile* __restrict_
         return;
     }
     Slot s = slots[tl.slot];
+    if (slot_mode) {
+        tl.axis = blockIdx.y;
+        if (!slot_mode[3 * tl.slot + tl.axis] || s.cnt > kBlockSort) return;
+        tl.start -= s.beg;
+    }
     if (tl.start + tl.len > s.cnt || s.beg + s.cnt > n) {
         if (threadIdx.x == 0) atomicOr(err, 2u);
         return;
@@ -1104,10 +1138,23 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     if (n > kMaxTris) return set_error(CVX_ERR_CAPACITY, "device BVH build: more than 2^26 triangles");
     cudaStream_t st = nullptr;
     BK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
+    // Host arrays of uploads in flight, kept until the stream has been waited for
+    // (the guard, which goes first, waits on every way out).
+    std::vector<std::shared_ptr<void>> keep;
     struct StreamGuard {
         cudaStream_t s;
-        ~StreamGuard() { cudaStreamDestroy(s); }
+        ~StreamGuard() {
+            cudaStreamSynchronize(s);
+            cudaStreamDestroy(s);
+        }
     } guard{st};
+    auto upload = [&](void* dst, auto&& host) -> int32_t {
+        using V = std::decay_t<decltype(host)>;
+        auto v = std::make_shared<V>(std::forward<decltype(host)>(host));
+        keep.push_back(v);
+        BK(cudaMemcpyAsync(dst, v->data(), v->size() * sizeof((*v)[0]), cudaMemcpyHostToDevice, st), "upload");
+        return CVX_OK;
+    };
 
     std::vector<float> tx, tt;
     float ty;
@@ -1186,16 +1233,14 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
             (e = ensure(d_ids, cap_ids, ids.size() * 4, "ids")) ||
             (e = ensure(d_acc, cap_acc, ids.size() * sizeof(BoxAcc), "boxes")))
             return e;
-        BK(cudaMemcpyAsync(d_tiles2.p, tl.data(), tl.size() * sizeof(Tile), cudaMemcpyHostToDevice, st), "upload");
-        BK(cudaMemcpyAsync(d_ids.p, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st), "upload");
+        const uint32_t n_tl = (uint32_t)tl.size();
+        if ((e = upload(d_tiles2.p, std::move(tl))) || (e = upload(d_ids.p, ids))) return e;
         k_box_init<<<blocks(ids.size(), 128), 128, 0, st>>>((BoxAcc*)d_acc.p, (uint32_t)ids.size());
-        k_box<<<(unsigned)tl.size(), kTile, 0, st>>>((const Tile*)d_tiles2.p, (uint32_t)tl.size(), R, order, n,
-                                                     (BoxAcc*)d_acc.p, (uint32_t)ids.size(), misc + 1);
+        k_box<<<n_tl, kTile, 0, st>>>((const Tile*)d_tiles2.p, n_tl, R, order, n, (BoxAcc*)d_acc.p,
+                                      (uint32_t)ids.size(), misc + 1);
         k_box_store<<<blocks(ids.size(), 128), 128, 0, st>>>((const uint32_t*)d_ids.p, (uint32_t)ids.size(),
                                                               (const BoxAcc*)d_acc.p, R, order, n, nodes, max_nodes,
                                                               inner, misc + 1);
-        // the tile and id buffers are reused by the next call: finish this one
-        BK(cudaStreamSynchronize(st), "node boxes");
         return CVX_OK;
     };
 
@@ -1209,7 +1254,9 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     }
     if ((s = node_boxes(root_ids))) return s;
     uint32_t bad = 0;
-    BK(cudaMemcpy(&bad, misc, 4, cudaMemcpyDeviceToHost), "flags");
+    BK(cudaMemcpyAsync(&bad, misc, 4, cudaMemcpyDeviceToHost, st), "flags");
+    BK(cudaStreamSynchronize(st), "root");
+    keep.clear();
     if (bad)
         return set_error(CVX_ERR_INVALID,
                          "device BVH build: NaN or infinite vertex coordinates (the host build takes them)");
@@ -1228,43 +1275,50 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
             tiles_of(tl, k, 0, h_beg[id], h_cnt[id]);
         }
         if ((s = ensure(d_tiles, cap_tiles, tl.size() * sizeof(Tile), "tiles"))) return s;
-        BK(cudaMemcpyAsync(d_slots.p, slots.data(), K * sizeof(Slot), cudaMemcpyHostToDevice, st), "upload");
-        BK(cudaMemcpyAsync(d_tiles.p, tl.data(), tl.size() * sizeof(Tile), cudaMemcpyHostToDevice, st), "upload");
+        const uint32_t n_tl = (uint32_t)tl.size();
+        if ((s = upload(d_slots.p, slots)) || (s = upload(d_tiles.p, std::move(tl)))) return s;
         const Slot* ds = (const Slot*)d_slots.p;
+        const Tile* dt = (const Tile*)d_tiles.p;
+        uint32_t* dm = (uint32_t*)d_mode.p;
         k_stats_init<<<blocks((size_t)K * 3 * kBins, 256), 256, 0, st>>>(bs, K * 3 * kBins);
-        k_bin_float<<<(unsigned)tl.size(), kTile, 0, st>>>((const Tile*)d_tiles.p, (uint32_t)tl.size(), ds, K, R,
-                                                          order, n, inner, binf, bs, misc + 1);
-        k_fallback<<<blocks(K, 128), 128, 0, st>>>(ds, K, bs, (uint32_t*)d_mode.p);
-        std::vector<uint32_t> mode((size_t)K * 3);
-        BK(cudaMemcpyAsync(mode.data(), d_mode.p, mode.size() * 4, cudaMemcpyDeviceToHost, st), "download");
-        BK(cudaStreamSynchronize(st), "binning");
-
+        k_bin_float<<<n_tl, kTile, 0, st>>>(dt, n_tl, ds, K, R, order, n, inner, binf, bs, misc + 1);
+        k_fallback<<<blocks(K, 128), 128, 0, st>>>(ds, K, bs, dm);
         // Uniform split (bvh.rs:176-201) where coordinate binning fell back.
-        std::vector<Tile> small_pairs, uni_tiles;
-        std::vector<Tile> big_pairs;
+        k_sort_slots<<<3 * K, 1024, 0, st>>>(ds, K, dm, R, order, n, srt, misc + 1);
+        k_axis_reset_slots<<<blocks((size_t)K * 3 * kBins, 256), 256, 0, st>>>(ds, K, dm, bs);
+        k_uniform_stats<<<dim3(n_tl, 3), kTile, 0, st>>>(dt, n_tl, dm, ds, K, R, order, n, srt, bs, misc + 1);
+        k_choose_warp<<<blocks((size_t)K * 32, 128), 128, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
+        std::vector<uint32_t> mode((size_t)K * 3);
+        std::vector<Decision> dec(K);
+        uint32_t errbits = 0;
+        auto decisions = [&]() -> int32_t {
+            BK(cudaMemcpyAsync(dec.data(), d_dec.p, K * sizeof(Decision), cudaMemcpyDeviceToHost, st), "download");
+            BK(cudaMemcpyAsync(mode.data(), dm, mode.size() * 4, cudaMemcpyDeviceToHost, st), "download");
+            BK(cudaMemcpyAsync(&errbits, misc + 1, 4, cudaMemcpyDeviceToHost, st), "flags");
+            BK(cudaStreamSynchronize(st), "split choice");
+            keep.clear();
+            return CVX_OK;
+        };
+        if ((s = decisions())) return s;
+        if (errbits) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
+
+        // Uniform splits too large for one block: sorted through global memory,
+        // and the level's choice made again.
+        std::vector<Tile> uni_tiles, big_pairs;
         for (uint32_t k = 0; k < K; k++)
             for (uint32_t a = 0; a < 3; a++)
-                if (mode[3 * k + a]) {
-                    Tile pr{k, a, slots[k].beg, slots[k].cnt};
-                    (pr.len <= kBlockSort ? small_pairs : big_pairs).push_back(pr);
+                if (mode[3 * k + a] && slots[k].cnt > kBlockSort) {
+                    const Tile pr{k, a, slots[k].beg, slots[k].cnt};
+                    big_pairs.push_back(pr);
                     for (uint32_t r0 = 0; r0 < pr.len; r0 += kTile)
                         uni_tiles.push_back(Tile{k, a, r0, std::min<uint32_t>(kTile, pr.len - r0)});
                 }
-        if (!uni_tiles.empty()) {
-            std::vector<Tile> pairs = small_pairs;
-            pairs.insert(pairs.end(), big_pairs.begin(), big_pairs.end());
-            if ((s = ensure(d_pairs, cap_pairs, pairs.size() * sizeof(Tile), "pairs")) ||
-                (s = ensure(d_tiles2, cap_tiles2, uni_tiles.size() * sizeof(Tile), "tiles")))
+        if (!big_pairs.empty()) {
+            const uint32_t n_uni = (uint32_t)uni_tiles.size();
+            if ((s = ensure(d_pairs, cap_pairs, big_pairs.size() * sizeof(Tile), "pairs")) ||
+                (s = ensure(d_tiles2, cap_tiles2, n_uni * sizeof(Tile), "tiles")) ||
+                (s = upload(d_pairs.p, big_pairs)) || (s = upload(d_tiles2.p, std::move(uni_tiles))))
                 return s;
-            BK(cudaMemcpyAsync(d_pairs.p, pairs.data(), pairs.size() * sizeof(Tile), cudaMemcpyHostToDevice, st),
-               "upload");
-            BK(cudaMemcpyAsync(d_tiles2.p, uni_tiles.data(), uni_tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice,
-                               st),
-               "upload");
-            if (!small_pairs.empty())
-                k_sort_block<<<(unsigned)small_pairs.size(), 1024, 0, st>>>((const Tile*)d_pairs.p,
-                                                                           (uint32_t)small_pairs.size(), R, order, n,
-                                                                           srt, misc + 1);
             for (const Tile& pr : big_pairs) {
                 uint32_t m2 = 4096;
                 while (m2 < pr.len) m2 <<= 1;
@@ -1280,15 +1334,14 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
                 }
                 k_sort_extract<<<blocks(pr.len, 256), 256, 0, st>>>(pr, buf, n, srt);
             }
-            k_axis_reset<<<blocks(pairs.size() * kBins, 256), 256, 0, st>>>((const Tile*)d_pairs.p,
-                                                                             (uint32_t)pairs.size(), bs);
-            k_uniform_stats<<<(unsigned)uni_tiles.size(), kTile, 0, st>>>(
-                (const Tile*)d_tiles2.p, (uint32_t)uni_tiles.size(), ds, K, R, order, n, srt, bs, misc + 1);
+            k_axis_reset<<<blocks(big_pairs.size() * kBins, 256), 256, 0, st>>>((const Tile*)d_pairs.p,
+                                                                               (uint32_t)big_pairs.size(), bs);
+            k_uniform_stats<<<n_uni, kTile, 0, st>>>((const Tile*)d_tiles2.p, n_uni, nullptr, ds, K, R, order, n, srt,
+                                                     bs, misc + 1);
+            k_choose_warp<<<blocks((size_t)K * 32, 128), 128, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
+            if ((s = decisions())) return s;
+            if (errbits) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
         }
-        k_choose_warp<<<blocks((size_t)K * 32, 128), 128, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
-        std::vector<Decision> dec(K);
-        BK(cudaMemcpyAsync(dec.data(), d_dec.p, K * sizeof(Decision), cudaMemcpyDeviceToHost, st), "download");
-        BK(cudaStreamSynchronize(st), "split choice");
 
         // Partition the split slots.
         std::vector<Tile> part;            // axis: 0..2 coordinate bins, 3..5 uniform
@@ -1329,60 +1382,50 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
                 (s = ensure(d_off, cap_off, std::max<size_t>(n_fl, 1) * kBins * 4, "offsets")) ||
                 (s = ensure(d_ids, cap_ids, std::max(slot_tiles.size(), triples.size()) * 4, "ids")))
                 return s;
-            BK(cudaMemcpyAsync(d_tiles.p, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice, st), "upload");
+            const uint32_t n_all = (uint32_t)all.size(), n_children = (uint32_t)children.size(),
+                           n_links = (uint32_t)(triples.size() / 3);
+            if ((s = upload(d_tiles.p, std::move(all)))) return s;
             if (n_fl) {
-                BK(cudaMemcpyAsync(d_ids.p, slot_tiles.data(), slot_tiles.size() * 4, cudaMemcpyHostToDevice, st),
-                   "upload");
+                if ((s = upload(d_ids.p, slot_tiles))) return s;
                 k_tile_hist<<<(unsigned)n_fl, kTile, 0, st>>>((const Tile*)d_tiles.p, (uint32_t)n_fl, binf, n,
                                                               (uint32_t*)d_hist.p);
                 k_tile_offsets<<<(unsigned)(slot_tiles.size() / 2), 1024, 0, st>>>(
                     (const uint32_t*)d_ids.p, (uint32_t)(slot_tiles.size() / 2), (const uint32_t*)d_hist.p,
                     (uint32_t*)d_off.p);
             }
-            k_scatter<<<(unsigned)all.size(), kTile, 0, st>>>((const Tile*)d_tiles.p, (uint32_t)all.size(), ds, K,
-                                                              binf, srt, (const uint32_t*)d_off.p, order, n, order_tmp,
-                                                              misc + 1);
-            k_copy_back<<<(unsigned)all.size(), kTile, 0, st>>>((const Tile*)d_tiles.p, (uint32_t)all.size(),
-                                                                order_tmp, order, n);
-            BK(cudaStreamSynchronize(st), "partition");
+            k_scatter<<<n_all, kTile, 0, st>>>((const Tile*)d_tiles.p, n_all, ds, K, binf, srt,
+                                               (const uint32_t*)d_off.p, order, n, order_tmp, misc + 1);
+            k_copy_back<<<n_all, kTile, 0, st>>>((const Tile*)d_tiles.p, n_all, order_tmp, order, n);
             // Children: ranges, exact boxes, then the parents' links.
             {
-                std::vector<InterimNode> ch(children.size());
-                for (size_t j = 0; j < children.size(); j++) {
+                std::vector<InterimNode> ch(n_children);
+                for (size_t j = 0; j < ch.size(); j++) {
                     ch[j] = InterimNode{};
                     ch[j].beg = h_beg[children[j]];
                     ch[j].cnt = h_cnt[children[j]];
                 }
                 // children ids are consecutive
-                BK(cudaMemcpyAsync(nodes + children[0], ch.data(), ch.size() * sizeof(InterimNode),
-                                   cudaMemcpyHostToDevice, st),
-                   "upload");
+                if ((s = upload(nodes + children[0], std::move(ch)))) return s;
             }
             if ((s = node_boxes(children))) return s;
             if ((s = ensure(d_ids, cap_ids, triples.size() * 4, "ids"))) return s;
-            BK(cudaMemcpyAsync(d_ids.p, triples.data(), triples.size() * 4, cudaMemcpyHostToDevice, st), "upload");
-            k_link<<<blocks(triples.size() / 3, 128), 128, 0, st>>>((const uint32_t*)d_ids.p,
-                                                                     (uint32_t)(triples.size() / 3), nodes, max_nodes,
-                                                                     misc + 1);
-            BK(cudaStreamSynchronize(st), "children");
+            if ((s = upload(d_ids.p, std::move(triples)))) return s;
+            k_link<<<blocks(n_links, 128), 128, 0, st>>>((const uint32_t*)d_ids.p, n_links, nodes, max_nodes,
+                                                         misc + 1);
             for (uint32_t c : children) {
                 if (h_cnt[c] > kSmall) next_active.push_back(c);
                 else if (h_cnt[c] >= 2) small.push_back(c);
             }
         }
         active.swap(next_active);
-        uint32_t errbits = 0;
-        BK(cudaMemcpy(&errbits, misc + 1, 4, cudaMemcpyDeviceToHost), "flags");
-        if (errbits) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
     }
 
     if (!small.empty()) {
         if ((s = ensure(d_ids, cap_ids, small.size() * 4, "ids"))) return s;
-        BK(cudaMemcpyAsync(d_ids.p, small.data(), small.size() * 4, cudaMemcpyHostToDevice, st), "upload");
+        if ((s = upload(d_ids.p, small))) return s;
         BK(cudaMemcpyAsync(misc + 2, &next_id, 4, cudaMemcpyHostToDevice, st), "upload");
         k_small<<<blocks(small.size(), kSmallWarps), 32 * kSmallWarps, 0, st>>>(
             (const uint32_t*)d_ids.p, (uint32_t)small.size(), nodes, max_nodes, misc + 2, order, n, R, ts, misc + 1);
-        BK(cudaMemcpyAsync(&next_id, misc + 2, 4, cudaMemcpyDeviceToHost, st), "download");
     }
     else BK(cudaMemcpyAsync(misc + 2, &next_id, 4, cudaMemcpyHostToDevice, st), "upload");
 
