@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uin
     __shared__ uint2 sstack[4][SHARED > 0 ? SHARED : 1][32];
     StagedSoaClaim claim{src, next_ray, stage[threadIdx.x >> 5], 0u, 0u, 0u, 0};
     claim.init(threadIdx.x & 31);
-    bool ok = traverse_refill<COUNT, false, CLAIM, SHARED, SELECT, kQuerySteps>(
+    bool ok = traverse_refill<COUNT, false, CLAIM, SHARED, SELECT, kQuerySteps, SELECT && CLAIM == 8>(
         src, claim, g_tables, &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
     if (!ok) atomicOr(err, kErrStackOverflow);
 }
@@ -575,6 +575,7 @@ __device__ __forceinline__ void path_pixel(uint32_t p, uint32_t bw, uint32_t& gx
 // 0.588 ms).
 template <bool MULTI>
 struct FramePaths {
+    static constexpr bool kOneScene = true;
     struct PathRef {
         uint32_t path;  // within its sample
         uint32_t smp;
@@ -672,7 +673,7 @@ constexpr int kRefillFrameSteps = 2;
 
 // COUNT: the same frame, also counting its work (FrameArgs::work); the
 // counters cost registers, so frames are rendered without them.
-// Trees deeper than 40 levels (the CLAIM_MIN 8 instantiation) keep the first
+// Trees deeper than 40 levels (the DEEP instantiation) keep the first
 // 16 stack entries of each lane in shared memory and read the approximation
 // tables from global memory instead (the 16 KB of entries per block take the
 // room the tables would); shallower trees keep the whole stack local. Measured
@@ -682,12 +683,13 @@ constexpr int kRefillFrameSteps = 2;
 // the same entries cost 3-4 %.
 constexpr int kDeepFrameStackShared = 16;
 
-// Deep trees: claim threshold 8 and two wide records per round. 870k tube,
-// 1280x736, 16 samples in one launch: 25.7 ms (35.7 with pairs and leaves tested
-// at once, 28.7 with four pairs per round and postponed leaves; three and four
-// records per round 26.1, 27.3). With pairs: claim 6, 12, 16 -> 29.7, 29.2, 30.5
-// ms; 6 and 8 resident blocks per SM 30.6 and 30.3 ms.
-constexpr int kDeepFrameClaim = 8;
+// Deep trees (the DEEP instantiation): claim threshold 12, two wide records per
+// round, and the warp's leaves tested together. 870k tube, 1280x736, 16 samples in
+// one launch: 23.2 ms (35.7 with pairs and leaves tested at once, 28.7 with four
+// pairs per round and postponed leaves, 25.7 with two wide records per round;
+// one and three records per round 24.1-25.6, 25.9; claim 8, 14: 23.9, 23.2; 6 and
+// 8 resident blocks per SM 24.7 and 23.4).
+constexpr int kDeepFrameClaim = 12;
 constexpr int kDeepFrameSteps = 2;
 // DEEP: a tree deeper than 40 levels (shared stack entries, the constants above).
 // MULTI: a.samples samples in one launch (FramePaths<true>).
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(128, kRefillFrameBlocksPerSm) k_render_refill(
     bool ok;
     if constexpr (DEEP) {
         __shared__ uint2 sstack[4][kDeepFrameStackShared][32];
-        ok = path_refill<kDeepFrameClaim, kDeepFrameSteps, COUNT, true, kDeepFrameStackShared>(
+        ok = path_refill<kDeepFrameClaim, kDeepFrameSteps, COUNT, true, kDeepFrameStackShared, true>(
             P, g_tables, &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
     } else {
         __shared__ ApproxTables tab;

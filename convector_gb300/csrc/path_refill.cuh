@@ -24,6 +24,7 @@
 // gbuffer word (the sampled direction, not the light PDFs or the BRDF).
 //
 // Paths provides, for a path reference `PathRef` it fills in:
+//   static constexpr bool kOneScene: every path's scene is the same
 //   uint32_t n_paths() const, uint32_t claim(uint32_t n)  (first of n paths)
 //   bool begin(uint32_t p, PathRef&, F3& o, F3& d, LaneRng&, const ApproxTables&)
 //       (false: the path's group lies outside its image; take another)
@@ -49,10 +50,14 @@ namespace cvx {
 // every tracing lane's ray allows it (a warp-uniform choice, so neither form's
 // code runs for the other's lanes); otherwise it takes STEPS steps in the x86
 // form. Each lane's results are the same either way.
+// POOL_LEAVES: such a round's leaves are tested by the whole warp (RefillRay::
+// test_leaves).
 template <int CLAIM_MIN, int STEPS, bool COUNT = false, bool SELECT_ROUNDS = false, int SHARED_STACK = 0,
-          class Paths>
+          bool POOL_LEAVES = false, class Paths>
 __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, uint2* shared_stack = nullptr) {
     typedef typename Paths::PathRef PathRef;
+    __shared__ uint8_t owners[4][32];  // RefillRay::test_leaves, blocks of four warps
+    uint8_t* const owner = owners[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const uint32_t npaths = P.n_paths();
     RefillRay ray;
@@ -159,8 +164,11 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
             if (tracing) {
 #pragma unroll 1
                 for (int st = 0; st < STEPS; st++) ray.walk(stack, overflow);
-                if (ray.test_leaf()) tracing = false;
             }
+            bool finished;
+            if constexpr (POOL_LEAVES) finished = ray.test_leaves<Paths::kOneScene>(owner, tracing);
+            else finished = tracing && ray.test_leaf();
+            if (finished) tracing = false;
         } else {
             if (SELECT_ROUNDS && !COUNT) ray.settle();
             for (int st = 0; st < STEPS && tracing; st++)

@@ -218,10 +218,13 @@ __device__ __forceinline__ bool select_form_ray(F3 o, F3 inv) {
            fabsf(o.z) <= kSelectMax;
 }
 
-// One triangle against one lane; updates the hit when the reference would
-// pick the new intersection (triangle.rs:122-147).
-__device__ __forceinline__ void tri_test(const float4* __restrict__ geom, uint32_t i, F3 o, F3 d, bool active,
-                                         Hit& h) {
+// One triangle against one ray: `in` when the reference's tests that do not look
+// at the nearest hit so far pass (triangle.rs:122-147).
+struct TriT {
+    float t, u, v;
+    bool in;
+};
+__device__ __forceinline__ TriT tri_eval(const float4* __restrict__ geom, uint32_t i, F3 o, F3 d) {
     float4 A = __ldg(geom + 3 * i), B = __ldg(geom + 3 * i + 1), C = __ldg(geom + 3 * i + 2);
     F3 v0 = f3(A.x, A.y, A.z), e1 = f3(B.x, B.y, B.z), e2 = f3(C.x, C.y, C.z), n = f3(A.w, B.w, C.w);
     F3 fr = sub(v0, o);
@@ -231,11 +234,19 @@ __device__ __forceinline__ void tri_test(const float4* __restrict__ geom, uint32
     float u = dot(c, e2) * denom;
     float v = dot(c, e1) * denom;
     float w = (1.0f - u) - v;
-    bool reject = sneg(t) | sneg(u) | sneg(v) | sneg(w) | !active | geq(t, h.t);
+    return TriT{t, u, v, !(sneg(t) | sneg(u) | sneg(v) | sneg(w))};
+}
+
+// The same; updates the hit when the reference would pick the new
+// intersection.
+__device__ __forceinline__ void tri_test(const float4* __restrict__ geom, uint32_t i, F3 o, F3 d, bool active,
+                                         Hit& h) {
+    const TriT x = tri_eval(geom, i, o, d);
+    bool reject = !x.in | !active | geq(x.t, h.t);
     if (!reject) {
-        h.t = t;
-        h.u = u;
-        h.v = v;
+        h.t = x.t;
+        h.u = x.u;
+        h.v = x.v;
         h.tri = (int32_t)i;
     }
 }
@@ -613,6 +624,93 @@ struct RefillRay {
         }
         return cur == kNone && sp == 0 && leaf == 0u;
     }
+    // test_leaf() for a whole warp, which must call it converged (`on`: lanes that
+    // trace a ray). Where some leaf has more than two triangles, the waiting
+    // leaves' triangles are laid out one after the other over the warp's lanes,
+    // each lane tests one of them for its ray's lane, and that lane then looks
+    // at its triangles that are hit in their order: the same decisions as
+    // test_leaf()'s, in about a pass per 32 triangles instead of one per triangle of
+    // the longest leaf. Laying out, shuffling the rays and looking at the hits
+    // make such a pass cost a little more than two of the others'.
+    //
+    // For trees deeper than 40 levels. A round of the 870k tube's frame has 15
+    // leaves of 2 triangles on average and the longest 4.6: 4.6 passes of 7 lanes
+    // become 1.4. One triangle at a time -> this, 1M random rays 470 -> 427 us, a
+    // 1280x736 sample of 16 in one launch 25.7 -> 23.2 ms (also when leaves of up to
+    // two or three triangles are laid out 23.9-24.3 at the old claim threshold).
+    // Shallower trees reach 10 triangles a round and lose by the warp's votes: 4M
+    // rays on the 28-level icosphere 614 -> 629 us, the room's samples 6.33 -> 6.20 ms,
+    // the icosphere's frame 2.01 -> 2.06 ms.
+    //
+    // owner: 32 bytes of shared memory of the warp's own. ONE_SCENE: every lane's
+    // `geom` is the same.
+    template <bool ONE_SCENE>
+    __device__ __forceinline__ bool test_leaves(uint8_t* owner, bool on) {
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t len = 0, idx = 0;
+        if (on && leaf != 0u) {
+            len = leaf & 31u;
+            idx = leaf >> 5;
+            leaf_range(nodes, idx, len);
+        }
+        for (;;) {
+            if (!__any_sync(0xffffffffu, len != 0u)) break;
+            if (__ballot_sync(0xffffffffu, len > 2u) == 0u) {
+#pragma unroll 1
+                for (uint32_t i = idx; i < idx + len; i++) tri_test(geom, i, o(), d, true, h);
+                break;
+            }
+            // Slots p .. p + n - 1 are this lane's (at most seven triangles a pass).
+            uint32_t n = min(len, 7u);
+            const unsigned b0 = __ballot_sync(0xffffffffu, n & 1u), b1 = __ballot_sync(0xffffffffu, n & 2u),
+                           b2 = __ballot_sync(0xffffffffu, n & 4u), lt = (1u << lane) - 1u;
+            const uint32_t p = __popc(b0 & lt) + 2u * __popc(b1 & lt) + 4u * __popc(b2 & lt);
+            const uint32_t total = __popc(b0) + 2u * __popc(b1) + 4u * __popc(b2);
+            n = p < 32u ? min(n, 32u - p) : 0u;
+            const unsigned starts = __reduce_or_sync(0xffffffffu, n ? 1u << p : 0u);
+            __syncwarp();
+            if (n) owner[p] = (uint8_t)lane;
+            __syncwarp();
+            const int start = 31 - __clz((int)(starts & (lt | 1u << lane)));  // slot 0 always starts a leaf
+            const int w = owner[start];
+            const uint32_t i = __shfl_sync(0xffffffffu, idx, w) + (lane - (uint32_t)start);
+            const F3 ro = f3(-__shfl_sync(0xffffffffu, no.x, w), -__shfl_sync(0xffffffffu, no.y, w),
+                             -__shfl_sync(0xffffffffu, no.z, w));
+            const F3 rd = f3(__shfl_sync(0xffffffffu, d.x, w), __shfl_sync(0xffffffffu, d.y, w),
+                             __shfl_sync(0xffffffffu, d.z, w));
+            const float4* g = geom;
+            if (!ONE_SCENE)
+                g = reinterpret_cast<const float4*>(
+                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(geom), w));
+            TriT x{0.0f, 0.0f, 0.0f, false};
+            if (lane < total) x = tri_eval(g, i, ro, rd);
+            unsigned mine = __ballot_sync(0xffffffffu, x.in) >> (p & 31u) & ((1u << n) - 1u);
+            while (__any_sync(0xffffffffu, mine != 0u)) {
+                const uint32_t k = (uint32_t)__ffs((int)mine) - 1u;  // of no lane's hits: unused
+                const int j = (int)(p + k);
+                const float t = __shfl_sync(0xffffffffu, x.t, j), u = __shfl_sync(0xffffffffu, x.u, j),
+                            v = __shfl_sync(0xffffffffu, x.v, j);
+                if (mine != 0u && !geq(t, h.t)) {
+                    h.t = t;
+                    h.u = u;
+                    h.v = v;
+                    h.tri = (int32_t)(idx + k);
+                }
+                mine &= mine - 1u;
+            }
+            idx += n;
+            len -= n;
+        }
+        if (on && leaf != 0u) {
+            leaf = 0u;
+            if (geq(cur_t, h.t)) cur = kNone;
+            if (cur != kNone && (cur & 31u) != 0u) {
+                leaf = cur;
+                cur = kNone;
+            }
+        }
+        return on && cur == kNone && sp == 0 && leaf == 0u;
+    }
     // From postponed leaves back to step(): after test_leaf() a waiting leaf is
     // the next node.
     __device__ __forceinline__ void settle() {
@@ -651,10 +749,14 @@ __device__ __forceinline__ typename std::conditional<N == 0, LocalStack, SharedL
 // the x86 form). STEPS: node pairs (SELECT) or traversal steps per round of the
 // warp's votes (a lane whose ray ends within a round waits for the next
 // round's claim).
+// POOL_LEAVES (with SELECT): a round's leaves are tested by the whole warp
+// (RefillRay::test_leaves).
 template <bool COUNT, bool LEAF_AFTER_PAIR, int CLAIM_MIN, int SHARED_STACK = 0, bool SELECT = false, int STEPS = 1,
-          class Src, class Claim>
+          bool POOL_LEAVES = false, class Src, class Claim>
 __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, const ApproxTables& tab,
                                                 uint2* shared_stack = nullptr) {
+    __shared__ uint8_t owners[4][32];  // test_leaves(), blocks of four warps
+    uint8_t* const owner = owners[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     RefillRay ray;
     uint2 local_stack[kStackSlots];
@@ -704,10 +806,13 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
             if (have) {
 #pragma unroll
                 for (int st = 0; st < STEPS; st++) ray.walk(stack, overflow);
-                if (ray.test_leaf()) {
-                    src.store(r_id, ray.h, 0u, 0u);
-                    have = false;
-                }
+            }
+            bool finished;
+            if constexpr (POOL_LEAVES) finished = ray.test_leaves<true>(owner, have);
+            else finished = have && ray.test_leaf();
+            if (finished) {
+                src.store(r_id, ray.h, 0u, 0u);
+                have = false;
             }
         } else {
             for (int st = 0; st < STEPS && have; st++) {

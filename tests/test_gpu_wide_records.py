@@ -190,3 +190,48 @@ def test_small_query_may_overwrite_its_rays(gpu, shift):
     gpu._check(gpu.lib().cvx_intersect_nearest(scene._h, *ptr, n, 1.0e5, gpu.TRAVERSE_PACKET, gpu._ptr(out_t),
                                                gpu._ptr(out_tri)))
     assert (out_tri == tri).all() and (out_t.view(np.uint32) == t.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("most", [2, 3, 7, 8, 31, 70])
+def test_pooled_leaves_equal_oracle(gpu, orc, most):
+    """Trees deeper than 40 levels, whose leaves' triangles are spread over the warp: leaves of 1 to `most`
+    triangles, each one twice (ties), on both sides of a pass's seven per lane and 32 per warp."""
+    pairs = 60
+    rng = np.random.default_rng(most)
+    tris, nodes = _chain(pairs)
+    lens = rng.integers(1, most + 1, pairs + 1)
+    lens[::7] = most
+    first = np.concatenate([[0], np.cumsum(lens)])
+    tris = np.repeat(tris, lens, axis=0)
+    f = tris.view(np.float32)
+    shift = np.repeat(rng.uniform(-0.4, 0.4, (f.shape[0] + 1) // 2).astype(np.float32), 2)[: f.shape[0]]
+    f[:, [1, 4, 7]] += shift[:, None] * np.float32(0.5)
+    for p in range(pairs):
+        nodes[2 * p, 6:8] = (first[p], lens[p])
+    nodes[2 * pairs - 1, 6:8] = (first[pairs], lens[pairs])
+    g = nodes.view(np.float32)
+    g[:, 1], g[:, 4] = 0.25, 1.75
+    b = type("B", (), {"triangles": tris, "nodes": nodes})()
+    scene, osc = gpu.Scene(b), orc.OracleScene(tris, nodes)
+    o, d = _rays(nodes, 5003, seed=most)
+    d[::2] = d[::2] * np.float32([1.0, 0.1, 0.1])  # through many levels
+    t, tri = (scene.set_query_launch(8), scene.intersect_nearest(o, d, traversal=gpu.TRAVERSE_SINGLE))[1]
+    ot, otri = osc.intersect(o, d, mode=gpu.TRAVERSE_SINGLE)
+    assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
+    assert (t.view(np.uint32) == ot.view(np.uint32)).all()
+    # frames, and a wave of two scenes
+    w, h = 83, 45
+    cam = scenes.default_camera(gpu.Camera(), eye=(-0.9, 1.0, 0.2), target=(0.0, 1.0, -2.0))
+    scenes.default_camera(scene.camera, eye=(-0.9, 1.0, 0.2), target=(0.0, 1.0, -2.0))
+    orgba, ogb, ocol, orays = osc.render(cam.as_array(), w, h, 9, rng_order=orc.RNG_GROUP, traversal=1)
+    r = gpu.Renderer(scene, w, h, rng_order=gpu.RNG_GROUP, traversal=gpu.TRAVERSE_SINGLE, refill_mode=gpu.REFILL_ALL)
+    rgba, gb = r.render_frame_u8(9)
+    assert (rgba == orgba).all() and (gb == ogb).all() and r.stats()[0] == orays
+    other = gpu.Scene(gpu.Bvh.build(scenes.spheres_and_boxes(600, 5, obj=False)[0]))
+    batch = gpu.Batch([other, scene], max_groups=1 << 14, max_pixels=3 * w * h, mode=gpu.MODE_MEGAKERNEL,
+                      refill_mode=gpu.REFILL_ALL)
+    images = batch.render([gpu.View(0, w, h, 1, 9, cam), gpu.View(1, w, h, 1, 9, cam), gpu.View(1, w, h, 1, 9, cam)])[0]
+    acc = np.zeros((h, w, 3), np.float32)
+    osc.render(cam.as_array(), w, h, 9, rng_order=orc.RNG_GROUP, traversal=1, accum=acc)
+    for image in images[1:]:
+        assert (np.asarray(image) == orc.resolve(acc, 1)).all()
