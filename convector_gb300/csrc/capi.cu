@@ -380,7 +380,7 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     CK(cudaMemcpyAsync(s->d_nodes, node_buf.data(), node_buf.size() * sizeof(float4), cudaMemcpyHostToDevice,
                        s->stream),
        "upload nodes");
-    if (tight && depth <= kWideMaxDepth) {
+    if (tight && depth <= kWideMaxDepth && n_nodes / 2 <= (1u << 25)) {  // 32-bit offsets into the records
         if ((st = dalloc(&s->d_wide, (size_t)n_nodes / 2 * 8, "wide nodes"))) return st;
         CK(launch_prep_wide(s->d_nodes + s->node_offset, n_nodes / 2, s->d_wide, s->stream), "wide nodes");
     }

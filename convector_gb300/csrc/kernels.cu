@@ -78,12 +78,13 @@ __global__ void k_prep_wide(const float4* __restrict__ nodes, uint32_t n_pairs, 
         }
         float4* w = wide + 8 * (size_t)p;
         for (int a = 0; a < 3; a++) {
-            w[2 * a] = make_float4(b[0][a], b[1][a], b[2][a], b[3][a]);
-            w[2 * a + 1] = make_float4(b[0][a + 3], b[1][a + 3], b[2][a + 3], b[3][a + 3]);
+            const int lo = a == 0 ? 0 : a == 1 ? 4 : 3, hi = lo + (1 << a);
+            w[lo] = make_float4(b[0][a], b[1][a], b[2][a], b[3][a]);
+            w[hi] = make_float4(b[0][a + 3], b[1][a + 3], b[2][a + 3], b[3][a + 3]);
         }
-        w[6] = make_float4(__uint_as_float(ref[0]), __uint_as_float(ref[1]), __uint_as_float(ref[2]),
+        w[2] = make_float4(__uint_as_float(ref[0]), __uint_as_float(ref[1]), __uint_as_float(ref[2]),
                            __uint_as_float(ref[3]));
-        w[7] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        w[5] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
 

@@ -29,8 +29,8 @@ __device__ __forceinline__ bool traverse_warp(const DeviceScene& s, F3 o, F3 d, 
     const bool sel = s.wide && __all_sync(kAll, select_form_ray(o, inv));
     // This slot's planes in the records (WidePlanes): near and far by the signs.
     const uint32_t nx_at = 4u * q + (inv.x > 0.0f ? 0u : 16u), fx_at = 8u * q + 16u - nx_at;
-    const uint32_t ny_at = 4u * q + (inv.y > 0.0f ? 0u : 16u), fy_at = 8u * q + 16u - ny_at;
-    const uint32_t nz_at = 4u * q + (inv.z > 0.0f ? 0u : 16u), fz_at = 8u * q + 16u - nz_at;
+    const uint32_t ny_at = 4u * q + (inv.y > 0.0f ? 64u : 96u), fy_at = 8u * q + 160u - ny_at;
+    const uint32_t nz_at = 4u * q + (inv.z > 0.0f ? 48u : 112u), fz_at = 8u * q + 160u - nz_at;
     int sp = 0;
     uint32_t cur = 0;
     for (;;) {
@@ -40,9 +40,9 @@ __device__ __forceinline__ bool traverse_warp(const DeviceScene& s, F3 o, F3 d, 
             const char* w = reinterpret_cast<const char*>(s.wide) + (size_t)cur * 2;
             auto ld = [](const char* p) { return __ldg(reinterpret_cast<const float*>(p)); };
             const float nx = (ld(w + nx_at) + no.x) * inv.x, fx = (ld(w + fx_at) + no.x) * inv.x;
-            const float ny = (ld(w + 32 + ny_at) + no.y) * inv.y, fy = (ld(w + 32 + fy_at) + no.y) * inv.y;
-            const float nz = (ld(w + 64 + nz_at) + no.z) * inv.z, fz = (ld(w + 64 + fz_at) + no.z) * inv.z;
-            const uint32_t r = __float_as_uint(ld(w + 96 + 4u * q));
+            const float ny = (ld(w + ny_at) + no.y) * inv.y, fy = (ld(w + fy_at) + no.y) * inv.y;
+            const float nz = (ld(w + nz_at) + no.z) * inv.z, fz = (ld(w + fz_at) + no.z) * inv.z;
+            const uint32_t r = __float_as_uint(ld(w + 32 + 4u * q));
             const float t = max3(nx, ny, nz), e = min3(fx, fy, fz);
             // Entry distance of the child this slot belongs to, from both its boxes.
             const float tc = max3(fminf(nx, __shfl_xor_sync(kAll, nx, 8)), fminf(ny, __shfl_xor_sync(kAll, ny, 8)),
