@@ -150,15 +150,26 @@ struct PacketRay {
     }
 
     // The boxes to visit, from the last to the first: each becomes the next
-    // node, and the one before it is pushed. Then a leaf goes to wait, if none
-    // does.
+    // node, and the one before it is pushed: by selects where a push is one
+    // store (frames: room 1.127 -> 1.119 ms, icosphere 2.76 -> 2.72, 320x184 of it
+    // 0.57 -> 0.53), else by branches (queries, whose first entries are in shared
+    // memory: 1M room packets 311, by selects 316 us). Then a leaf goes to wait, if
+    // none does.
     template <int N, class Stack>
     __device__ __forceinline__ void push(const bool (&v)[N], const uint32_t (&r)[N], const float (&t)[N], Stack& stack,
                                          bool& overflow) {
         cur = kNone;
 #pragma unroll
         for (int k = 0; k < N; k++) {
-            if (v[k]) {
+            if constexpr (Stack::kOneStore) {
+                const bool p = k > 0 && v[k] && cur != kNone;
+                if (p) stack.store(sp, top);
+                top.x = p ? cur : top.x;
+                top.y = p ? __float_as_uint(cur_t) : top.y;
+                sp += p;
+                cur = v[k] ? r[k] : cur;
+                cur_t = v[k] ? t[k] : cur_t;
+            } else if (v[k]) {
                 if (k > 0 && cur != kNone) {
                     stack.store(sp, top);
                     top = make_uint2(cur, __float_as_uint(cur_t));
