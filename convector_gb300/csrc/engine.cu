@@ -164,6 +164,17 @@ int32_t WaveEngine::launch(const WaveOutputs& out, bool deep, cudaStream_t strea
     return CVX_OK;
 }
 
+bool WaveEngine::octet_wave(const std::vector<Job>& jobs) const {
+    uint64_t total = 0, deep = 0;
+    for (const Job& j : jobs) {
+        const uint64_t g = groups_of(j.w, j.h);
+        total += g;
+        if (j.scene < n_scenes_ && scene_depth_[j.scene] >= kRefillMinDepth) deep += g;
+    }
+    if (!fused_ || total >= max_groups_) return false;
+    return packet_ || total >= kMaxRefillGroups || !path_refill_wave(refill_mode_, (uint32_t)deep, (uint32_t)total);
+}
+
 int32_t WaveEngine::submit(const std::vector<Job>& jobs_in, WaveOutputs out, cudaStream_t stream,
                            bool want_job_rays) {
     last_jobs_ = 0;
@@ -371,16 +382,27 @@ extern "C" int32_t cvx_batch_render(cvx_batch* b, const cvx_view* views, uint32_
     bool touched = rgba == nullptr;  // the images' pages, while the first wave runs
     WaveOutputs out{};
     out.accum = b->d_accum;
-    // Sample s of every view goes into wave s; a wave's jobs are split by
+    // The next sample of every view goes into a wave; a wave's jobs are split by
     // their scene's kernel organisation, and the two halves run concurrently
     // (disjoint pixels) on two streams. A wave larger than the ray-queue
-    // capacity is split into several.
+    // capacity is split into several. In the octet form up to kWaveSamples samples of a
+    // view share the wave: each wave ends with a drain and a wait of the host (32
+    // open scenes, 13 M pixels, 4 samples: 7.35 -> 6.98 ms).
+    constexpr uint32_t kWaveSamples = 16;
+    std::vector<uint32_t> next(n, 0u);
     for (uint32_t s = 0; s < max_spp; s++) {
         std::vector<Job> jobs[2];
+        std::vector<uint32_t> fused_views;
         uint32_t groups = 0;
         auto flush = [&]() -> int32_t {
             uint64_t r[2] = {0, 0};
             float t[2] = {0.0f, 0.0f};
+            if (b->fused.octet_wave(jobs[0]))
+                for (size_t i = 0; i < jobs[0].size(); i++) {
+                    const uint32_t v = fused_views[i];
+                    jobs[0][i].more = std::min(kWaveSamples - 1u, views[v].spp - next[v]);
+                    next[v] += jobs[0][i].more;
+                }
             int32_t st = b->fused.submit(jobs[0], out, b->stream2, false);
             if (!st) st = b->engine.submit(jobs[1], out, b->stream, false);
             for (uint32_t i = 0; i < n && !touched; i++)
@@ -392,12 +414,13 @@ extern "C" int32_t cvx_batch_render(cvx_batch* b, const cvx_view* views, uint32_
             ms += t[0] > t[1] ? t[0] : t[1];
             jobs[0].clear();
             jobs[1].clear();
+            fused_views.clear();
             groups = 0;
             return st ? st : (st0 ? st0 : st1);
         };
         for (uint32_t i = 0; i < n; i++) {
             const cvx_view& v = views[i];
-            if (v.spp <= s) continue;
+            if (next[i] >= v.spp) continue;
             uint32_t m = b->mode[v.scene];
             uint32_t g = groups_of(v.width, v.height);
             if ((m == 1 && groups + g > b->engine.max_groups()) || jobs[m].size() == b->engine.max_jobs()) {
@@ -409,9 +432,10 @@ extern "C" int32_t cvx_batch_render(cvx_batch* b, const cvx_view* views, uint32_
             j.scene = v.scene;
             j.w = v.width;
             j.h = v.height;
-            j.frame = v.frame_base + s;
+            j.frame = v.frame_base + next[i]++;
             j.out_offset = offset[i];
             jobs[m].push_back(j);
+            if (m == 0) fused_views.push_back(i);
             if (m == 1) groups += g;
         }
         if (!jobs[0].empty() || !jobs[1].empty()) {

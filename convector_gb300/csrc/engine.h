@@ -45,7 +45,7 @@ class WaveEngine {
     // max_groups: ray-queue capacity (8-pixel groups) of one wave. fused: run
     // waves as one persistent fused kernel (no ray queues) instead of the
     // wavefront kernels; refill_mode: CVX_REFILL_* (wavefront: which bounces
-    // refill; fused: path_refill_frames with the wave's deepest scene).
+    // refill; fused: path_refill_wave).
     int32_t init(uint32_t max_groups, uint32_t max_jobs, bool packet, bool use_graph, uint32_t blocks_per_sm,
                  uint32_t refill_mode = CVX_REFILL_AFTER_CAMERA, bool fused = false);
     int32_t set_scenes(cvx_scene* const* scenes, uint32_t n);
@@ -56,6 +56,9 @@ class WaveEngine {
     // submit + collect. rays, job_rays and ms may be null.
     int32_t run(const std::vector<Job>& jobs, WaveOutputs out, cudaStream_t stream, uint64_t* rays,
                 std::vector<uint64_t>* job_rays, float* ms);
+    // Whether a wave of these jobs would take the octet form, whose jobs may hold
+    // several samples (Job::more).
+    bool octet_wave(const std::vector<Job>& jobs) const;
     uint32_t max_groups() const { return max_groups_; }
     uint32_t max_jobs() const { return max_jobs_; }
     bool fused() const { return fused_; }

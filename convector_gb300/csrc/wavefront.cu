@@ -338,7 +338,8 @@ cudaError_t set_stack_limit_wave(int entries) {
 // The fused form over a wave: every octet renders whole groups of any job
 // (camera ray, bounce loop and shading in registers), walking the wave's
 // groups with a grid-stride loop. Same per-group RNG order and outputs as the
-// wavefront kernels.
+// wavefront kernels. A group's samples (Job::more) follow one another on its octet,
+// so each pixel's are added in their order.
 template <bool PACKET>
 // 8 resident blocks per SM (64 registers, small spill): batches of small
 // scenes render 12 % faster than at the compiler's 80 registers (6 blocks).
@@ -363,35 +364,37 @@ __global__ void __launch_bounds__(128, 8) k_wave_fused(const Job* __restrict__ j
         group_origin(j, gi - j.group_base, &xb, &yb, &g, &gx, &gy);
         if (gx >= j.w || gy >= j.h) continue;  // whole group outside the frame (octet-uniform)
         const DeviceScene s = scenes[j.scene];
-        float x, y, scale;
-        block_coord_wf(j.w, j.h, xb, yb, g, k, &x, &y, &scale);
-        LaneRng rng;
-        rng.seed(gx, gy, j.frame, k);
-        x = fmaf(unit_from(rng.next()), scale, x);
-        y = fmaf(unit_from(rng.next()), scale, y);
-        PixelOut p;
-        uint32_t r = 0;
-        ok &= render_pixels<PACKET>(s, j.cam, x, y, rng, omask, tab, p, r);
-        rays += r;
-        if (out.job_rays) {
-            uint32_t tot = r;
-            for (int off = 4; off > 0; off >>= 1) tot += __shfl_down_sync(omask, tot, off, 8);
-            if (k == 0 && tot) atomicAdd(&out.job_rays[ji], (unsigned long long)tot);
-        }
-        uint32_t px = gx + (uint32_t)(k & 3), py = gy + (uint32_t)(k >> 2);
-        if (px < j.w && py < j.h) {
-            size_t idx = (size_t)j.out_offset + (size_t)py * j.w + px;
-            if (out.rgba) out.rgba[idx] = pack_color(p.color);
-            if (out.gbuf) out.gbuf[idx] = pack_gbuffer(p);
-            if (out.color) {
-                out.color[3 * idx] = p.color.x;
-                out.color[3 * idx + 1] = p.color.y;
-                out.color[3 * idx + 2] = p.color.z;
+        for (uint32_t smp = 0; smp <= j.more; smp++) {
+            float x, y, scale;
+            block_coord_wf(j.w, j.h, xb, yb, g, k, &x, &y, &scale);
+            LaneRng rng;
+            rng.seed(gx, gy, j.frame + smp, k);
+            x = fmaf(unit_from(rng.next()), scale, x);
+            y = fmaf(unit_from(rng.next()), scale, y);
+            PixelOut p;
+            uint32_t r = 0;
+            ok &= render_pixels<PACKET>(s, j.cam, x, y, rng, omask, tab, p, r);
+            rays += r;
+            if (out.job_rays) {
+                uint32_t tot = r;
+                for (int off = 4; off > 0; off >>= 1) tot += __shfl_down_sync(omask, tot, off, 8);
+                if (k == 0 && tot) atomicAdd(&out.job_rays[ji], (unsigned long long)tot);
             }
-            if (out.accum) {
-                out.accum[3 * idx] += p.color.x;
-                out.accum[3 * idx + 1] += p.color.y;
-                out.accum[3 * idx + 2] += p.color.z;
+            uint32_t px = gx + (uint32_t)(k & 3), py = gy + (uint32_t)(k >> 2);
+            if (px < j.w && py < j.h) {
+                size_t idx = (size_t)j.out_offset + (size_t)py * j.w + px;
+                if (out.rgba) out.rgba[idx] = pack_color(p.color);
+                if (out.gbuf) out.gbuf[idx] = pack_gbuffer(p);
+                if (out.color) {
+                    out.color[3 * idx] = p.color.x;
+                    out.color[3 * idx + 1] = p.color.y;
+                    out.color[3 * idx + 2] = p.color.z;
+                }
+                if (out.accum) {
+                    out.accum[3 * idx] += p.color.x;
+                    out.accum[3 * idx + 1] += p.color.y;
+                    out.accum[3 * idx + 2] += p.color.z;
+                }
             }
         }
     }

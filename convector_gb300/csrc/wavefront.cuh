@@ -1,8 +1,8 @@
 // Wavefront form of the path loop (renderer.rs:413-468): ray generation,
 // traversal and shading kernels over structure-of-arrays ray queues.
 //
-// A wave is a list of jobs; a job is one sample of one image of one resident
-// scene (its own camera, size, frame number and output slot). All groups of
+// A wave is a list of jobs; a job is one sample (or, Job::more, a few) of one image
+// of one resident scene (its own camera, size, frame number and output slot). All groups of
 // all jobs of a wave share the queues, so images of different scenes and
 // sizes fill the same launches. Every group uses the per-group RNG order, so
 // a job's pixels do not depend on which other jobs share its wave.
@@ -26,6 +26,9 @@ struct Job {
     // adds the slots to the accumulator in sample order (several samples of
     // one image in one wave).
     uint64_t slot;
+    // Waves in the octet form (k_wave_fused) only: the samples of this image
+    // after `frame` that the wave renders too, adding each to the accumulator.
+    uint32_t more;
 };
 constexpr uint64_t kNoSlot = ~0ull;
 
