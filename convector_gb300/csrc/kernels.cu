@@ -822,25 +822,31 @@ __global__ void __launch_bounds__(128, 1) k_render_patch(FrameArgs a) {
 // how many bounces every group before it took. But the generator jumps to any
 // state (after n draws it is s * f^n mod 2^64), so the warps of a round render
 // the next groups at once, each from the state it has if the groups before it in
-// the round take the patch's most frequent bounce count. The groups up to the
-// first wrong guess are right and are stored; the others are rendered again.
-// Where guesses miss, a round takes as many groups as the last one confirmed and
-// one more.
+// the round take certain bounce counts. What counts is by how often each was met
+// so far in the patch (top: the three most frequent): a chain of groups that all take
+// the first; two guesses for the first group and a group beyond; or three guesses
+// for it, whichever is expected to confirm the most groups. The groups whose
+// predecessors took what was guessed are right and are stored; the others are
+// rendered again.
 //
 // The frame's time is that of its slowest patches (the room's slowest takes four
-// times the mean): their rays stay inside and nearly every group takes all five
-// bounces (125 of 128), so guesses hold where they matter. Room 1280x736: one
-// octet per patch 16.6 ms, one warp per patch 12.0, two warps with guesses 7.8,
-// four 5.7, eight 6.5 (64 registers, 4 blocks per SM; 7.5 with 3), sixteen 10.5:
-// idle warps keep other patches' blocks off the SM. Icosphere 26.8, 18.2, 12.6,
-// 12.1, 15.8, 23.5 ms. 6 blocks of 4 warps per SM hold the frame's 920 patches
-// at once (4, 5, 7, 8 blocks: 5.7, 5.6, 5.9, 6.4 and 14.2, 13.6, 13.2, 13.7 ms).
+// times the mean): in some nearly every group takes all five bounces (125 of 128), so
+// chains hold; in others the counts are mixed, and a round confirms two groups of
+// four. Room 1280x736: one octet per patch 16.6 ms, one warp per patch 12.0, a chain
+// of four warps as long as the last round's was right 5.57, this 5.46; icosphere
+// 26.8, 18.2, 11.6, 10.9 ms; the room at 320x184 (60 patches) 4.61, 4.26. (Two warps
+// 7.8 ms, eight 6.5, sixteen 10.5, with chains: idle warps keep other patches' blocks
+// off the SM.) 6 blocks of 4 warps per SM hold the frame's 920 patches at once (4, 5,
+// 7, 8 blocks with chains: 5.7, 5.6, 5.9, 6.4 and 14.2, 13.6, 13.2, 13.7 ms).
+// kPatchChance: 0, 0.18, 0.21 -> 5.58, 5.55, 5.48; 11.08, 10.94, 11.04; 4.31, 4.31,
+// 4.29 ms (0.25, 0.35 and 0.5 3, 7 and 15 % slower).
 constexpr int kPatchWarps = 4;
-template <int W>
-__global__ void __launch_bounds__(32 * W, 24 / W) k_render_patch_warp(FrameArgs a) {
+constexpr float kPatchChance = 0.2f;
+__global__ void __launch_bounds__(32 * kPatchWarps, 24 / kPatchWarps) k_render_patch_warp(FrameArgs a) {
     __shared__ ApproxTables tab;
-    __shared__ WarpStack stacks[W];
-    __shared__ int taken[2][W];  // by parity of the round: bounces of each warp's group
+    __shared__ WarpStack stacks[kPatchWarps];
+    __shared__ uint64_t draws[8][8], group_draws[6][8];
+    __shared__ int taken[2][kPatchWarps];  // by parity of the round: bounces of each warp's group
     load_tables(tab);
     const uint32_t lane = threadIdx.x & 31u, k = lane & 7u;
     const int wid = (int)(threadIdx.x >> 5);
@@ -851,41 +857,63 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_render_patch_warp(FrameArgs 
     const uint32_t y0 = a.patches ? a.patches[2 * pi + 1] : (pi % ph) * a.patch;
     LaneRng rng;
     rng.seed(x0, y0, a.frame, (int)k);
-    const uint64_t f = rng.f, f2 = f * f, f4 = f2 * f2, f6 = f4 * f2, f8 = f4 * f4, f16 = f8 * f8;
-    auto group_factor = [&](int bounces) {
-        uint64_t r = f;
-        for (int i = 0; i < bounces; i++) r *= f6;
-        return r;
-    };
+    // Powers of this lane's generator factor: 1 draw to 7, and those of a group of t
+    // bounces (1 + 6 t draws).
+    const uint64_t f = rng.f, f2 = f * f, f4 = f2 * f2, f8 = f4 * f4, f16 = f8 * f8;
+    if (threadIdx.x < 8u) {
+        uint64_t q = 1;
+        for (int i = 0; i < 8; i++, q *= f) draws[i][k] = q;
+        q = f;
+        for (int t = 0; t < 6; t++, q *= f4 * f2) group_draws[t][k] = q;
+    }
+    __syncthreads();
     // Confirmed: the state before group `done` (before its block's jitter draws
     // if it is the block's first), and before its block's jitter draws.
     uint64_t state = rng.s, block = rng.s;
     uint32_t done = 0, rays = 0;
-    int width = 1, guess = 5, parity = 0;
-    uint64_t seen = 0;  // how often each bounce count was confirmed, 8 bits each
+    int parity = 0;
+    // Lane t < 6: how often t bounces were met (to start with, a guess).
+    uint32_t met = lane >= 1u && lane < 6u ? lane == 5u ? 2u : 1u : 0u;
     bool ok = true;
     while (done < total) {
-        const int n = (int)min((uint32_t)width, total - done);
-        PixelOut p;
+        const float all = (float)__reduce_add_sync(0xffffffffu, met);
+        int top[3];
+        float p[3];
+        uint32_t rest = lane < 6u ? met << 3 | lane : 0u;
+        for (int i = 0; i < 3; i++) {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, rest);
+            top[i] = (int)(m & 7u);
+            p[i] = __fdividef((float)(m >> 3), all);
+            if (rest == m) rest = 0u;
+        }
+        // Groups beyond the first expected to be confirmed: chain, two guesses, three.
+        const float chain = p[0] + p[0] * p[0] * (1.0f + p[0]), two = p[0] + p[1] + p[0] * p[0], three = p[0] + p[1] + p[2];
+        const int guesses = two > chain ? (three > two ? 3 : 2) : (three > chain ? 3 : 1);
+        // Warp w renders group done + ahead(w), if the group before it takes last(w)
+        // and those before that top[0].
+        auto ahead = [&](int w) { return guesses == 1 ? w : guesses == 2 && w == 3 ? 2 : min(w, 1); };
+        auto last = [&](int w) { return w < 2 || guesses == 1 || w > guesses ? top[0] : w == 2 ? top[1] : top[2]; };
+        // The chance that warp w's group is confirmed; a small one is not worth the
+        // issue slots it takes from other patches.
+        const float q = wid == 0 ? 1.0f : wid == 1 ? p[0] : guesses == 1 ? (wid == 2 ? p[0] * p[0] : p[0] * p[0] * p[0])
+                                : wid == 2 ? p[1] : guesses == 2 ? p[0] * p[0] : p[2];
+        const uint32_t mine = done + (uint32_t)ahead(wid);
+        PixelOut out;
         uint32_t px = 0, py = 0, r = 0;
         bool fits = true;
-        if (wid < n) {
-            const uint32_t mine = done + (uint32_t)wid;
-            const uint64_t step = group_factor(guess);
+        if (lane == 0u) taken[parity][wid] = -1;
+        if (mine < total && q >= kPatchChance) {
             uint64_t s = state, b = block;
-            for (uint32_t i = done; i < mine; i++) {
+            for (uint32_t i = done;; i++) {
                 if ((i & 7u) == 0u) {
                     b = s;
                     s *= f16;
                 }
-                s *= step;
-            }
-            if ((mine & 7u) == 0u) {
-                b = s;
-                s *= f16;
+                if (i == mine) break;
+                s *= group_draws[i + 1u == mine ? last(wid) : top[0]][k];
             }
             const int g = (int)(mine & 7u);
-            for (int i = 0; i < g; i++) b *= f;
+            b *= draws[g][k];
             auto draw = [&](uint64_t v) { return unit_from(rng.hi ? (uint32_t)(v >> 32) : (uint32_t)v); };
             const uint32_t xb = x0 + (mine >> 3) / hb * 16u, yb = y0 + (mine >> 3) % hb * 4u;
             float x, y, scale;
@@ -894,37 +922,36 @@ __global__ void __launch_bounds__(32 * W, 24 / W) k_render_patch_warp(FrameArgs 
             y = fmaf(draw(b * f8), scale, y);
             rng.s = s;
             int bounces;
-            fits = render_pixels_warp(a.s, a.cam, x, y, rng, tab, stacks[wid], p, r, bounces);
+            fits = render_pixels_warp(a.s, a.cam, x, y, rng, tab, stacks[wid], out, r, bounces);
             px = xb + 4u * (uint32_t)(g >> 1) + (k & 3u);
             py = yb + 2u * (uint32_t)(g & 1) + (k >> 2);
             if (lane == 0u) taken[parity][wid] = bounces;
         }
         __syncthreads();
-        // The groups whose predecessors of this round all took what was guessed.
-        int valid = 1;
-        while (valid < n && taken[parity][valid - 1] == guess) valid++;
-        if (wid < valid) {
-            ok &= fits;
-            if (lane < 8u) {
-                store_pixel(a, px, py, p);
-                rays += r;
+        // From group to group, by the warp that guessed what the last one took.
+        bool firsts = true;  // the groups before the last one took top[0]
+        for (int w = 0, d = 1; w >= 0; d++) {
+            if (w == wid) {
+                ok &= fits;
+                if (lane < 8u) {
+                    store_pixel(a, px, py, out);
+                    rays += r;
+                }
             }
-        }
-        for (int i = 0; i < valid; i++) {
-            if (((done + (uint32_t)i) & 7u) == 0u) {
+            const int t = taken[parity][w];
+            if ((done & 7u) == 0u) {
                 block = state;
                 state *= f16;
             }
-            const int t = taken[parity][i];
-            state *= group_factor(t);
-            if ((seen >> (8 * t) & 0xffu) >= 64u) seen = (seen >> 1) & 0x7f7f7f7f7f7full;
-            seen += 1ull << (8 * t);
+            state *= group_draws[t][k];
+            if (__any_sync(0xffffffffu, met >= 64u)) met >>= 1;
+            met += (int)lane == t;
+            w = -1;
+            if (++done < total && firsts)
+                for (int v = 1; v < kPatchWarps; v++)
+                    if (ahead(v) == d && last(v) == t && taken[parity][v] >= 0) w = v;
+            firsts &= t == top[0];
         }
-        done += (uint32_t)valid;
-        width = valid == n ? min(W, 2 * width) : min(W, valid + 1);
-        guess = 5;
-        for (int t = 4; t >= 0; t--)
-            if ((seen >> (8 * t) & 0xffu) > (seen >> (8 * guess) & 0xffu)) guess = t;
         parity ^= 1;
     }
     if (!ok) atomicOr(a.err, kErrStackOverflow);
@@ -1123,7 +1150,7 @@ cudaError_t launch_render(const DeviceScene& s, const DeviceCamera& cam, uint32_
     if (patch_order) {
         uint32_t units = patches ? n_patches : ((w + patch - 1) / patch) * ((h + patch - 1) / patch);
         uint32_t blocks = (units * 32 + block - 1) / block;  // one warp per patch
-        if (packet && !debug) k_render_patch_warp<kPatchWarps><<<units, 32 * kPatchWarps, 0, st>>>(a);
+        if (packet && !debug) k_render_patch_warp<<<units, 32 * kPatchWarps, 0, st>>>(a);
         else if (packet) k_render_patch<true><<<blocks, block, 0, st>>>(a);
         else k_render_patch<false><<<blocks, block, 0, st>>>(a);
     } else {
