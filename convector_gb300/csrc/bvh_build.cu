@@ -203,28 +203,25 @@ __global__ void __launch_bounds__(kTile) k_box(const Tile* __restrict__ tiles, u
     }
 }
 
-// Writes the decoded boxes into the interim nodes of list `ids`.
+// Writes the decoded boxes into the interim nodes of list `ids`, a thread per axis:
+// four dependent loads bound it (a thread for all three axes 9 us, this 5).
 __global__ void k_box_store(const uint32_t* __restrict__ ids, uint32_t m, const BoxAcc* __restrict__ acc, Refs r,
                             const uint32_t* __restrict__ order, uint32_t n, InterimNode* nodes, uint32_t n_nodes,
                             float* inner, uint32_t* err) {
-    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, j = i / 3u, c = i % 3u;
     if (j >= m) return;
-    uint32_t id = ids[j];
-    if (id >= n_nodes) {
+    const uint32_t id = ids[j];
+    const uint32_t pmin = (uint32_t)acc[j].omin[c], pmax = 0xffffffffu - (uint32_t)acc[j].omax[c];
+    if (id >= n_nodes || pmin >= n || pmax >= n) {
         atomicOr(err, 2u);
         return;
     }
-    for (int c = 0; c < 3; c++) {
-        uint32_t pmin = (uint32_t)acc[j].omin[c], pmax = 0xffffffffu - (uint32_t)acc[j].omax[c];
-        if (pmin >= n || pmax >= n) {
-            atomicOr(err, 2u);
-            return;
-        }
-        nodes[id].lo[c] = r.lo[c][order[pmin]];
-        nodes[id].hi[c] = r.hi[c][order[pmax]];
-        inner[6 * (size_t)id + c] = from_okey(acc[j].imin[c]);
-        inner[6 * (size_t)id + 3 + c] = from_okey(acc[j].imax[c]);
-    }
+    const float* const lo = c == 0u ? r.lo[0] : c == 1u ? r.lo[1] : r.lo[2];
+    const float* const hi = c == 0u ? r.hi[0] : c == 1u ? r.hi[1] : r.hi[2];
+    nodes[id].lo[c] = lo[order[pmin]];
+    nodes[id].hi[c] = hi[order[pmax]];
+    inner[6 * (size_t)id + c] = from_okey(acc[j].imin[c]);
+    inner[6 * (size_t)id + 3 + c] = from_okey(acc[j].imax[c]);
 }
 
 // ---------------------------------------------------------------------------
@@ -315,15 +312,25 @@ __global__ void __launch_bounds__(kTile) k_bin_float(const Tile* __restrict__ ti
 }
 
 // bvh.rs:160-166: a bin above n/8 triangles (n > 64) sends the axis to the
-// uniform split. mode[slot][axis]: 0 coordinate bins, 1 uniform.
-__global__ void k_fallback(const Slot* __restrict__ slots, uint32_t n_slots, BinStats st, uint32_t* mode) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n_slots) return;
-    uint32_t n = slots[k].cnt;
-    for (int a = 0; a < 3; a++) {
-        uint32_t mx = 0;
-        for (int b = 0; b < kBins; b++) mx = max(mx, st.count[((size_t)k * 3 + a) * kBins + b]);
-        mode[3 * k + a] = (mx > n / 8u && n > (uint32_t)kBins) ? 1u : 0u;
+// uniform split. mode[slot][axis]: 0 coordinate bins, 1 uniform; the statistics of
+// those that k_sort_slots sorts are reset. One warp per (slot, axis): a thread
+// per slot and a pass for the reset took 12 + 3 us a level.
+__global__ void __launch_bounds__(128) k_fallback(const Slot* __restrict__ slots, uint32_t n_slots, BinStats st,
+                                                  uint32_t* __restrict__ mode) {
+    const uint32_t pair = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (pair >= 3u * n_slots) return;  // warp-uniform
+    const uint32_t n = slots[pair / 3u].cnt;
+    uint32_t* const cn = st.count + (size_t)pair * kBins;
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, max(cn[lane], cn[lane + 32u]));
+    const bool uniform = mx > n / 8u && n > (uint32_t)kBins;
+    if (lane == 0u) mode[pair] = uniform ? 1u : 0u;
+    if (!uniform || n > kBlockSort) return;
+    for (uint32_t b = lane; b < (uint32_t)kBins; b += 32u) {
+        cn[b] = 0u;
+        for (int c = 0; c < 3; c++) {
+            st.key[6 * ((size_t)pair * kBins + b) + c] = ~0u;
+            st.key[6 * ((size_t)pair * kBins + b) + 3 + c] = 0u;
+        }
     }
 }
 
@@ -445,19 +452,6 @@ __global__ void k_axis_reset(const Tile* __restrict__ pairs, uint32_t n_pairs, B
         st.key[6 * g + 3 + c] = 0u;
     }
 }
-// k_axis_reset of the (slot, axis) pairs of k_sort_slots.
-__global__ void k_axis_reset_slots(const Slot* __restrict__ slots, uint32_t n_slots,
-                                   const uint32_t* __restrict__ mode, BinStats st) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t pair = i / kBins;
-    if (pair >= 3u * n_slots || !mode[pair] || slots[pair / 3u].cnt > kBlockSort) return;
-    st.count[i] = 0u;
-    for (int c = 0; c < 3; c++) {
-        st.key[6 * (size_t)i + c] = ~0u;
-        st.key[6 * (size_t)i + 3 + c] = 0u;
-    }
-}
-
 // slot_mode: `tiles` are the level's tiles (absolute starts), one axis per
 // blockIdx.y, of which the (slot, axis) pairs of k_sort_slots are taken; null:
 // tiles list (slot, axis, relative start) themselves.
@@ -498,9 +492,10 @@ __global__ void __launch_bounds__(kTile) k_uniform_stats(const Tile* __restrict_
 }
 
 // bvh.rs:218-322: the cheapest split over the three axes, or a leaf. One
-// warp per slot (lane l owns bins l and l + 32):
-// prefix and suffix boxes and counts by warp scans, the candidate costs in
-// parallel, and lane 0 applying the host's first-minimum rule in bin order.
+// warp per slot and axis (lane l owns bins l and l + 32): prefix and suffix boxes
+// and counts by warp scans, the candidate costs in parallel, and their first
+// minimum; then the axes in order. Bound by the chain of shuffles: one warp for
+// the three axes and the candidates one by one took 30 us a level.
 __device__ __forceinline__ void box_scan_empty(Box& b) {
     for (int c = 0; c < 3; c++) {
         b.lo[c] = __int_as_float(0x7f800000);   // +inf
@@ -538,29 +533,31 @@ __device__ __forceinline__ Box box_shfl(const Box& b, int src) {
     return r;
 }
 
-__global__ void __launch_bounds__(128) k_choose_warp(const Slot* __restrict__ slots, uint32_t n_slots,
-                                                     const InterimNode* __restrict__ nodes, BinStats st, Tsah ts,
-                                                     Decision* __restrict__ dec) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (k >= n_slots) return;  // warp-uniform
-    Slot s = slots[k];
+__global__ void __launch_bounds__(96) k_choose(const Slot* __restrict__ slots, uint32_t n_slots,
+                                               const InterimNode* __restrict__ nodes, BinStats st, Tsah ts,
+                                               Decision* __restrict__ dec) {
+    struct Choice {
+        float cost;
+        uint32_t at, nl;  // at 0: the axis has no two bins to split between
+    };
+    __shared__ Choice choice[3];
+    const int lane = threadIdx.x & 31, a = threadIdx.x >> 5;
+    const uint32_t k = blockIdx.x;
+    if (k >= n_slots) return;  // block-uniform
+    const Slot s = slots[k];
     Box outer;
     for (int c = 0; c < 3; c++) {
         outer.lo[c] = nodes[s.id].lo[c];
         outer.hi[c] = nodes[s.id].hi[c];
     }
     const float parent_area = area(outer);
-    float best_cost = 0.0f;
-    bool is_first = true;
-    Decision d{3u, 0u, 0u, 1u};
-    for (int a = 0; a < 3; a++) {
-        const uint32_t* cn = st.count + ((size_t)k * 3 + a) * kBins;
-        const uint32_t* ky = st.key + ((size_t)k * 3 + a) * kBins * 6;
-        uint32_t c0 = cn[lane], c1 = cn[lane + 32];
-        unsigned m0 = __ballot_sync(0xffffffffu, c0 != 0u), m1 = __ballot_sync(0xffffffffu, c1 != 0u);
-        int nonempty = __popc(m0) + __popc(m1);
-        if (nonempty <= 1) continue;  // warp-uniform
+    if (lane == 0) choice[a].at = 0u;
+    const uint32_t* cn = st.count + ((size_t)k * 3 + a) * kBins;
+    const uint32_t* ky = st.key + ((size_t)k * 3 + a) * kBins * 6;
+    uint32_t c0 = cn[lane], c1 = cn[lane + 32];
+    unsigned m0 = __ballot_sync(0xffffffffu, c0 != 0u), m1 = __ballot_sync(0xffffffffu, c1 != 0u);
+    int nonempty = __popc(m0) + __popc(m1);
+    if (nonempty > 1) {  // warp-uniform
         int first = (m0 ? __ffs(m0) - 1 : 32 + __ffs(m1) - 1) + 1;
         int last = (m1 ? 32 + 31 - __clz(m1) : 31 - __clz(m0)) + 1;
         Box b0, b1;
@@ -617,28 +614,35 @@ __global__ void __launch_bounds__(128) k_choose_warp(const Slot* __restrict__ sl
         float cost0 = 0.0f, cost1 = 0.0f;
         if (i0 >= first && i0 < last) cost0 = tsah_cost(ts, parent_area, p0, pc0) + tsah_cost(ts, parent_area, r0, rc0);
         if (i1 >= first && i1 < last) cost1 = tsah_cost(ts, parent_area, p1, pc1) + tsah_cost(ts, parent_area, r1, rc1);
-        // bvh.rs:241-258: the first candidate, then strictly cheaper ones, in bin order.
-        float best = 0.0f;
-        int at = 0;
-        bool first_i = true;
-        for (int i = first; i < last; i++) {
-            float c = i <= 32 ? __shfl_sync(0xffffffffu, cost0, i - 1) : __shfl_sync(0xffffffffu, cost1, i - 33);
-            if (c < best || first_i) {
-                best = c;
-                at = i;
-                first_i = false;
-            }
-        }
-        if (best < best_cost || is_first) {
-            best_cost = best;
+        // bvh.rs:241-258: the first candidate, then strictly cheaper ones, in bin
+        // order: the first of the cheapest, unless the first is not a number.
+        const bool v0 = i0 >= first && i0 < last && cost0 == cost0, v1 = i1 >= first && i1 < last && cost1 == cost1;
+        const uint32_t k0 = v0 ? okey(cost0) : ~0u, k1 = v1 ? okey(cost1) : ~0u;
+        const uint32_t kmin = __reduce_min_sync(0xffffffffu, min(k0, k1));
+        const unsigned e0 = __ballot_sync(0xffffffffu, v0 && k0 == kmin), e1 = __ballot_sync(0xffffffffu, v1 && k1 == kmin);
+        const float c_first = first <= 32 ? __shfl_sync(0xffffffffu, cost0, first - 1)
+                                          : __shfl_sync(0xffffffffu, cost1, first - 33);
+        const int at = c_first != c_first ? first : e0 ? __ffs((int)e0) : 32 + __ffs((int)e1);
+        const float best = at <= 32 ? __shfl_sync(0xffffffffu, cost0, at - 1) : __shfl_sync(0xffffffffu, cost1, at - 33);
+        // left count: prefix count of bin at - 1
+        const uint32_t nl = at <= 32 ? __shfl_sync(0xffffffffu, pc0, at - 1) : __shfl_sync(0xffffffffu, pc1, at - 33);
+        if (lane == 0) choice[a] = Choice{best, (uint32_t)at, nl};
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    float best_cost = 0.0f;
+    bool is_first = true;
+    Decision d{3u, 0u, 0u, 1u};
+    for (int x = 0; x < 3; x++) {
+        const Choice c = choice[x];
+        if (c.at != 0u && (c.cost < best_cost || is_first)) {
+            best_cost = c.cost;
             is_first = false;
-            // left count: prefix count of bin at - 1
-            uint32_t nl = at <= 32 ? __shfl_sync(0xffffffffu, pc0, at - 1) : __shfl_sync(0xffffffffu, pc1, at - 33);
-            d = Decision{(uint32_t)a, (uint32_t)at, nl, 0u};
+            d = Decision{(uint32_t)x, c.at, c.nl, 0u};
         }
     }
     if (is_first || (float)s.cnt * 120.0f < best_cost) d.leaf = 1u;
-    if (lane == 0) dec[k] = d;
+    dec[k] = d;
 }
 
 // Partition of the split slots. Coordinate-binned axis: a stable counting
@@ -1238,7 +1242,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         k_box_init<<<blocks(ids.size(), 128), 128, 0, st>>>((BoxAcc*)d_acc.p, (uint32_t)ids.size());
         k_box<<<n_tl, kTile, 0, st>>>((const Tile*)d_tiles2.p, n_tl, R, order, n, (BoxAcc*)d_acc.p,
                                       (uint32_t)ids.size(), misc + 1);
-        k_box_store<<<blocks(ids.size(), 128), 128, 0, st>>>((const uint32_t*)d_ids.p, (uint32_t)ids.size(),
+        k_box_store<<<blocks(3 * ids.size(), 128), 128, 0, st>>>((const uint32_t*)d_ids.p, (uint32_t)ids.size(),
                                                               (const BoxAcc*)d_acc.p, R, order, n, nodes, max_nodes,
                                                               inner, misc + 1);
         return CVX_OK;
@@ -1282,12 +1286,11 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         uint32_t* dm = (uint32_t*)d_mode.p;
         k_stats_init<<<blocks((size_t)K * 3 * kBins, 256), 256, 0, st>>>(bs, K * 3 * kBins);
         k_bin_float<<<n_tl, kTile, 0, st>>>(dt, n_tl, ds, K, R, order, n, inner, binf, bs, misc + 1);
-        k_fallback<<<blocks(K, 128), 128, 0, st>>>(ds, K, bs, dm);
+        k_fallback<<<blocks((size_t)K * 3 * 32, 128), 128, 0, st>>>(ds, K, bs, dm);
         // Uniform split (bvh.rs:176-201) where coordinate binning fell back.
         k_sort_slots<<<3 * K, 1024, 0, st>>>(ds, K, dm, R, order, n, srt, misc + 1);
-        k_axis_reset_slots<<<blocks((size_t)K * 3 * kBins, 256), 256, 0, st>>>(ds, K, dm, bs);
         k_uniform_stats<<<dim3(n_tl, 3), kTile, 0, st>>>(dt, n_tl, dm, ds, K, R, order, n, srt, bs, misc + 1);
-        k_choose_warp<<<blocks((size_t)K * 32, 128), 128, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
+        k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
         std::vector<uint32_t> mode((size_t)K * 3);
         std::vector<Decision> dec(K);
         uint32_t errbits = 0;
@@ -1338,7 +1341,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
                                                                                (uint32_t)big_pairs.size(), bs);
             k_uniform_stats<<<n_uni, kTile, 0, st>>>((const Tile*)d_tiles2.p, n_uni, nullptr, ds, K, R, order, n, srt,
                                                      bs, misc + 1);
-            k_choose_warp<<<blocks((size_t)K * 32, 128), 128, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
+            k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
             if ((s = decisions())) return s;
             if (errbits) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
         }
