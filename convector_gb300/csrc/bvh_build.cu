@@ -58,8 +58,16 @@ struct Slot {
     uint32_t id, beg, cnt;
 };
 
+// A slot's split, and what else the host reads of a level. axis 3: no axis had two
+// non-empty bins. flags: bit 0 a leaf, bit 1 + a the mode of axis a (k_fallback).
+// The entry after the last slot's holds the error bits in `flags`.
 struct Decision {
-    uint32_t axis, at, nl, leaf;  // axis 3: no axis had two non-empty bins
+    uint32_t axis, at, nl, flags;
+};
+// A split node and its children, l and l + 1: the first nl of its cnt triangles
+// from beg, and the others.
+struct Link {
+    uint32_t id, l, beg, nl, cnt;
 };
 
 // Orderable key of a float with -0 and +0 equal (no NaN reaches here).
@@ -203,14 +211,14 @@ __global__ void __launch_bounds__(kTile) k_box(const Tile* __restrict__ tiles, u
     }
 }
 
-// Writes the decoded boxes into the interim nodes of list `ids`, a thread per axis:
+// Writes the decoded boxes into the interim nodes from `first` on, a thread per axis:
 // four dependent loads bound it (a thread for all three axes 9 us, this 5).
-__global__ void k_box_store(const uint32_t* __restrict__ ids, uint32_t m, const BoxAcc* __restrict__ acc, Refs r,
+__global__ void k_box_store(uint32_t first, uint32_t m, const BoxAcc* __restrict__ acc, Refs r,
                             const uint32_t* __restrict__ order, uint32_t n, InterimNode* nodes, uint32_t n_nodes,
                             float* inner, uint32_t* err) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, j = i / 3u, c = i % 3u;
     if (j >= m) return;
-    const uint32_t id = ids[j];
+    const uint32_t id = first + j;
     const uint32_t pmin = (uint32_t)acc[j].omin[c], pmax = 0xffffffffu - (uint32_t)acc[j].omax[c];
     if (id >= n_nodes || pmin >= n || pmax >= n) {
         atomicOr(err, 2u);
@@ -535,6 +543,7 @@ __device__ __forceinline__ Box box_shfl(const Box& b, int src) {
 
 __global__ void __launch_bounds__(96) k_choose(const Slot* __restrict__ slots, uint32_t n_slots,
                                                const InterimNode* __restrict__ nodes, BinStats st, Tsah ts,
+                                               const uint32_t* __restrict__ mode, const uint32_t* __restrict__ err,
                                                Decision* __restrict__ dec) {
     struct Choice {
         float cost;
@@ -641,8 +650,10 @@ __global__ void __launch_bounds__(96) k_choose(const Slot* __restrict__ slots, u
             d = Decision{(uint32_t)x, c.at, c.nl, 0u};
         }
     }
-    if (is_first || (float)s.cnt * 120.0f < best_cost) d.leaf = 1u;
+    if (is_first || (float)s.cnt * 120.0f < best_cost) d.flags = 1u;
+    for (int x = 0; x < 3; x++) d.flags |= mode[3 * k + x] << (1 + x);
     dec[k] = d;
+    if (k == 0) dec[n_slots] = Decision{0u, 0u, 0u, *err};
 }
 
 // Partition of the split slots. Coordinate-binned axis: a stable counting
@@ -753,13 +764,15 @@ __global__ void k_copy_back(const Tile* __restrict__ tiles, uint32_t n_tiles, co
     if (threadIdx.x < tl.len && p < n) dst[p] = src[p];
 }
 
-// Links split parents to their children, smaller box first (bvh.rs:333-335).
-__global__ void k_link(const uint32_t* __restrict__ triples, uint32_t m, InterimNode* nodes, uint32_t n_nodes,
+// Links split parents to their children, smaller box first (bvh.rs:333-335), and
+// sets the children's ranges.
+__global__ void k_link(const Link* __restrict__ links, uint32_t m, InterimNode* nodes, uint32_t n_nodes,
                        uint32_t* err) {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= m) return;
-    uint32_t parent = triples[3 * j], l = triples[3 * j + 1], r = triples[3 * j + 2];
-    if (parent >= n_nodes || l >= n_nodes || r >= n_nodes) {
+    const Link k = links[j];
+    const uint32_t l = k.l, r = k.l + 1u;
+    if (k.id >= n_nodes || r >= n_nodes) {
         atomicOr(err, 2u);
         return;
     }
@@ -770,9 +783,13 @@ __global__ void k_link(const uint32_t* __restrict__ triples, uint32_t m, Interim
         br.lo[c] = nodes[r].lo[c];
         br.hi[c] = nodes[r].hi[c];
     }
+    nodes[l].beg = k.beg;
+    nodes[l].cnt = k.nl;
+    nodes[r].beg = k.beg + k.nl;
+    nodes[r].cnt = k.cnt - k.nl;
     bool swap = area(bl) > area(br);
-    nodes[parent].c0 = swap ? r : l;
-    nodes[parent].c1 = swap ? l : r;
+    nodes[k.id].c0 = swap ? r : l;
+    nodes[k.id].c1 = swap ? l : r;
 }
 
 // ---------------------------------------------------------------------------
@@ -1137,6 +1154,19 @@ static unsigned blocks(size_t n, unsigned b) { return (unsigned)((n + b - 1) / b
 
 }  // namespace
 
+// The lists of a phase, which go up in one copy (a level made eight, and three
+// down, and lists that grew by the level: 81,920 triangles 5.77 -> 5.11 ms).
+struct Lists {
+    std::vector<unsigned char> bytes;
+    template <class T>
+    size_t add(const std::vector<T>& v) {
+        const size_t at = (bytes.size() + 15) / 16 * 16, size = v.size() * sizeof(T);
+        bytes.resize(at + size);
+        if (size) std::memcpy(bytes.data() + at, v.data(), size);
+        return at;
+    }
+};
+
 int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     if (n == 0) return set_error(CVX_ERR_INVALID, "cannot build a BVH of zero triangles");
     if (n > kMaxTris) return set_error(CVX_ERR_CAPACITY, "device BVH build: more than 2^26 triangles");
@@ -1167,7 +1197,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     const uint32_t max_slots = n / (kSmall + 1) + 1;
 
     DevBuf d_tris, d_refs, d_order, d_tmp, d_srt, d_binf, d_nodes, d_inner, d_tx, d_tt, d_misc, d_cnt, d_key,
-        d_mode, d_dec, d_slots, d_tiles, d_tiles2, d_hist, d_off, d_ids, d_acc, d_sortbuf, d_pairs;
+        d_mode, d_dec, d_level, d_split, d_tiles2, d_hist, d_off, d_ids, d_acc, d_sortbuf, d_pairs;
     int32_t s = 0;
     if ((s = dalloc<cvx_triangle>(d_tris, n, "triangles")) || (s = dalloc<float>(d_refs, (size_t)9 * n, "refs")) ||
         (s = dalloc<uint32_t>(d_order, n, "order")) || (s = dalloc<uint32_t>(d_tmp, n, "order")) ||
@@ -1179,7 +1209,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         (s = dalloc<uint32_t>(d_cnt, (size_t)max_slots * 3 * kBins, "bin counts")) ||
         (s = dalloc<uint32_t>(d_key, (size_t)max_slots * 3 * kBins * 6, "bin boxes")) ||
         (s = dalloc<uint32_t>(d_mode, (size_t)max_slots * 3, "modes")) ||
-        (s = dalloc<Decision>(d_dec, max_slots, "decisions")) || (s = dalloc<Slot>(d_slots, max_slots, "slots")))
+        (s = dalloc<Decision>(d_dec, (size_t)max_slots + 1, "decisions")))
         return s;
     cvx_triangle* tri_d = (cvx_triangle*)d_tris.p;
     float* refs = (float*)d_refs.p;
@@ -1213,50 +1243,50 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     h_beg[0] = 0;
     h_cnt[0] = n;
 
-    // Scratch that grows with the largest list of a level.
-    size_t cap_tiles = 0, cap_tiles2 = 0, cap_ids = 0, cap_pairs = 0, cap_sort = 0;
+    // Scratch that grows with the largest list of a level (to twice what is asked for:
+    // an allocation waits for the device).
+    size_t cap_level = 0, cap_split = 0, cap_tiles2 = 0, cap_ids = 0, cap_pairs = 0, cap_sort = 0;
     auto ensure = [&](DevBuf& b, size_t& cap, size_t bytes, const char* what) -> int32_t {
         if (bytes <= cap) return CVX_OK;
         if (b.p) cudaFree(b.p);
         b.p = nullptr;
-        cap = std::max(bytes, (size_t)4096);
-        cudaError_t e = cudaMalloc(&b.p, cap);
+        cap = 0;
+        const size_t want = std::max(2 * bytes, (size_t)1 << 16);
+        cudaError_t e = cudaMalloc(&b.p, want);
         if (e != cudaSuccess)
             return set_error(CVX_ERR_DEVICE, std::string("device BVH build: ") + what + ": " + cudaGetErrorString(e));
+        cap = want;
         return CVX_OK;
     };
     size_t cap_hist = 0, cap_off = 0, cap_acc = 0;
+    auto upload_lists = [&](DevBuf& b, size_t& cap, Lists& l) -> int32_t {
+        int32_t e = ensure(b, cap, l.bytes.size(), "lists");
+        return e ? e : upload(b.p, std::move(l.bytes));
+    };
 
-    // Exact boxes of a list of interim nodes (their ranges are current).
-    auto node_boxes = [&](const std::vector<uint32_t>& ids) -> int32_t {
-        if (ids.empty()) return CVX_OK;
-        std::vector<Tile> tl;
-        for (size_t j = 0; j < ids.size(); j++) tiles_of(tl, (uint32_t)j, 0, h_beg[ids[j]], h_cnt[ids[j]]);
-        int32_t e;
-        if ((e = ensure(d_tiles2, cap_tiles2, tl.size() * sizeof(Tile), "tiles")) ||
-            (e = ensure(d_ids, cap_ids, ids.size() * 4, "ids")) ||
-            (e = ensure(d_acc, cap_acc, ids.size() * sizeof(BoxAcc), "boxes")))
-            return e;
-        const uint32_t n_tl = (uint32_t)tl.size();
-        if ((e = upload(d_tiles2.p, std::move(tl))) || (e = upload(d_ids.p, ids))) return e;
-        k_box_init<<<blocks(ids.size(), 128), 128, 0, st>>>((BoxAcc*)d_acc.p, (uint32_t)ids.size());
-        k_box<<<n_tl, kTile, 0, st>>>((const Tile*)d_tiles2.p, n_tl, R, order, n, (BoxAcc*)d_acc.p,
-                                      (uint32_t)ids.size(), misc + 1);
-        k_box_store<<<blocks(3 * ids.size(), 128), 128, 0, st>>>((const uint32_t*)d_ids.p, (uint32_t)ids.size(),
-                                                              (const BoxAcc*)d_acc.p, R, order, n, nodes, max_nodes,
-                                                              inner, misc + 1);
+    // Exact boxes of the `count` interim nodes from `first` on, whose tiles are `tl`
+    // (slot: index from `first`).
+    auto node_boxes = [&](uint32_t first, uint32_t count, const Tile* tl, uint32_t n_tl) -> int32_t {
+        int32_t e = ensure(d_acc, cap_acc, count * sizeof(BoxAcc), "boxes");
+        if (e) return e;
+        k_box_init<<<blocks(count, 128), 128, 0, st>>>((BoxAcc*)d_acc.p, count);
+        k_box<<<n_tl, kTile, 0, st>>>(tl, n_tl, R, order, n, (BoxAcc*)d_acc.p, count, misc + 1);
+        k_box_store<<<blocks(3 * (size_t)count, 128), 128, 0, st>>>(first, count, (const BoxAcc*)d_acc.p, R, order, n,
+                                                                    nodes, max_nodes, inner, misc + 1);
         return CVX_OK;
     };
 
     // Root: range [0, n) in input order.
-    std::vector<uint32_t> root_ids{0};
+    const InterimNode r0{{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, 0u, n, 0u, 0u};
     {
-        InterimNode r0{};
-        r0.beg = 0;
-        r0.cnt = n;
         BK(cudaMemcpyAsync(nodes, &r0, sizeof r0, cudaMemcpyHostToDevice, st), "upload");
+        std::vector<Tile> tl;
+        tiles_of(tl, 0, 0, 0, n);
+        const uint32_t n_tl = (uint32_t)tl.size();
+        Lists l;
+        l.add(tl);
+        if ((s = upload_lists(d_split, cap_split, l)) || (s = node_boxes(0, 1, (const Tile*)d_split.p, n_tl))) return s;
     }
-    if ((s = node_boxes(root_ids))) return s;
     uint32_t bad = 0;
     BK(cudaMemcpyAsync(&bad, misc, 4, cudaMemcpyDeviceToHost, st), "flags");
     BK(cudaStreamSynchronize(st), "root");
@@ -1278,11 +1308,12 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
             slots[k] = Slot{id, h_beg[id], h_cnt[id]};
             tiles_of(tl, k, 0, h_beg[id], h_cnt[id]);
         }
-        if ((s = ensure(d_tiles, cap_tiles, tl.size() * sizeof(Tile), "tiles"))) return s;
         const uint32_t n_tl = (uint32_t)tl.size();
-        if ((s = upload(d_slots.p, slots)) || (s = upload(d_tiles.p, std::move(tl)))) return s;
-        const Slot* ds = (const Slot*)d_slots.p;
-        const Tile* dt = (const Tile*)d_tiles.p;
+        Lists lists;
+        const size_t at_slots = lists.add(slots), at_tiles = lists.add(tl);
+        if ((s = upload_lists(d_level, cap_level, lists))) return s;
+        const Slot* ds = (const Slot*)((const char*)d_level.p + at_slots);
+        const Tile* dt = (const Tile*)((const char*)d_level.p + at_tiles);
         uint32_t* dm = (uint32_t*)d_mode.p;
         k_stats_init<<<blocks((size_t)K * 3 * kBins, 256), 256, 0, st>>>(bs, K * 3 * kBins);
         k_bin_float<<<n_tl, kTile, 0, st>>>(dt, n_tl, ds, K, R, order, n, inner, binf, bs, misc + 1);
@@ -1290,27 +1321,25 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         // Uniform split (bvh.rs:176-201) where coordinate binning fell back.
         k_sort_slots<<<3 * K, 1024, 0, st>>>(ds, K, dm, R, order, n, srt, misc + 1);
         k_uniform_stats<<<dim3(n_tl, 3), kTile, 0, st>>>(dt, n_tl, dm, ds, K, R, order, n, srt, bs, misc + 1);
-        k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
-        std::vector<uint32_t> mode((size_t)K * 3);
-        std::vector<Decision> dec(K);
-        uint32_t errbits = 0;
+        k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, dm, misc + 1, (Decision*)d_dec.p);
+        std::vector<Decision> dec((size_t)K + 1);
         auto decisions = [&]() -> int32_t {
-            BK(cudaMemcpyAsync(dec.data(), d_dec.p, K * sizeof(Decision), cudaMemcpyDeviceToHost, st), "download");
-            BK(cudaMemcpyAsync(mode.data(), dm, mode.size() * 4, cudaMemcpyDeviceToHost, st), "download");
-            BK(cudaMemcpyAsync(&errbits, misc + 1, 4, cudaMemcpyDeviceToHost, st), "flags");
+            BK(cudaMemcpyAsync(dec.data(), d_dec.p, dec.size() * sizeof(Decision), cudaMemcpyDeviceToHost, st),
+               "download");
             BK(cudaStreamSynchronize(st), "split choice");
             keep.clear();
+            if (dec[K].flags) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
             return CVX_OK;
         };
         if ((s = decisions())) return s;
-        if (errbits) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
+        auto uniform = [&](uint32_t k, uint32_t a) { return (dec[k].flags >> (1 + a) & 1u) != 0u; };
 
         // Uniform splits too large for one block: sorted through global memory,
         // and the level's choice made again.
         std::vector<Tile> uni_tiles, big_pairs;
         for (uint32_t k = 0; k < K; k++)
             for (uint32_t a = 0; a < 3; a++)
-                if (mode[3 * k + a] && slots[k].cnt > kBlockSort) {
+                if (uniform(k, a) && slots[k].cnt > kBlockSort) {
                     const Tile pr{k, a, slots[k].beg, slots[k].cnt};
                     big_pairs.push_back(pr);
                     for (uint32_t r0 = 0; r0 < pr.len; r0 += kTile)
@@ -1341,22 +1370,24 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
                                                                                (uint32_t)big_pairs.size(), bs);
             k_uniform_stats<<<n_uni, kTile, 0, st>>>((const Tile*)d_tiles2.p, n_uni, nullptr, ds, K, R, order, n, srt,
                                                      bs, misc + 1);
-            k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, (Decision*)d_dec.p);
+            k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, dm, misc + 1, (Decision*)d_dec.p);
             if ((s = decisions())) return s;
-            if (errbits) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
         }
 
         // Partition the split slots.
         std::vector<Tile> part;            // axis: 0..2 coordinate bins, 3..5 uniform
         std::vector<uint32_t> slot_tiles;  // per coordinate-binned split slot: [t0, t1) in `fl`
         std::vector<Tile> fl;              // coordinate-binned tiles (for the histograms)
-        std::vector<uint32_t> triples, children, next_active;
+        std::vector<Tile> boxes;           // of the children
+        std::vector<Link> links;
+        std::vector<uint32_t> next_active;
+        const uint32_t first_child = next_id;
         for (uint32_t k = 0; k < K; k++) {
             const Decision& d = dec[k];
-            if (d.leaf) continue;
-            if (d.axis > 2 || d.nl == 0 || d.nl >= slots[k].cnt) return set_error(CVX_ERR_DEVICE, "device BVH build: bad split");
-            bool uni = mode[3 * k + d.axis] != 0;
-            if (uni) {
+            if (d.flags & 1u) continue;
+            if (d.axis > 2 || d.nl == 0 || d.nl >= slots[k].cnt)
+                return set_error(CVX_ERR_DEVICE, "device BVH build: bad split");
+            if (uniform(k, d.axis)) {
                 tiles_of(part, k, 3 + d.axis, slots[k].beg, slots[k].cnt);
             } else {
                 uint32_t t0 = (uint32_t)fl.size();
@@ -1364,61 +1395,48 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
                 slot_tiles.push_back(t0);
                 slot_tiles.push_back((uint32_t)fl.size());
             }
-            uint32_t l = next_id, r = next_id + 1;
+            const uint32_t l = next_id, r = next_id + 1;
             next_id += 2;
             if (next_id > max_nodes) return set_error(CVX_ERR_DEVICE, "device BVH build: node overflow");
             h_beg[l] = slots[k].beg;
             h_cnt[l] = d.nl;
             h_beg[r] = slots[k].beg + d.nl;
             h_cnt[r] = slots[k].cnt - d.nl;
-            triples.insert(triples.end(), {slots[k].id, l, r});
-            children.push_back(l);
-            children.push_back(r);
-        }
-        if (!children.empty()) {
-            // coordinate-binned tiles first (their block index is the tile_off row), then uniform
-            size_t n_fl = fl.size();
-            std::vector<Tile> all = fl;
-            all.insert(all.end(), part.begin(), part.end());
-            if ((s = ensure(d_tiles, cap_tiles, all.size() * sizeof(Tile), "tiles")) ||
-                (s = ensure(d_hist, cap_hist, std::max<size_t>(n_fl, 1) * kBins * 4, "histograms")) ||
-                (s = ensure(d_off, cap_off, std::max<size_t>(n_fl, 1) * kBins * 4, "offsets")) ||
-                (s = ensure(d_ids, cap_ids, std::max(slot_tiles.size(), triples.size()) * 4, "ids")))
-                return s;
-            const uint32_t n_all = (uint32_t)all.size(), n_children = (uint32_t)children.size(),
-                           n_links = (uint32_t)(triples.size() / 3);
-            if ((s = upload(d_tiles.p, std::move(all)))) return s;
-            if (n_fl) {
-                if ((s = upload(d_ids.p, slot_tiles))) return s;
-                k_tile_hist<<<(unsigned)n_fl, kTile, 0, st>>>((const Tile*)d_tiles.p, (uint32_t)n_fl, binf, n,
-                                                              (uint32_t*)d_hist.p);
-                k_tile_offsets<<<(unsigned)(slot_tiles.size() / 2), 1024, 0, st>>>(
-                    (const uint32_t*)d_ids.p, (uint32_t)(slot_tiles.size() / 2), (const uint32_t*)d_hist.p,
-                    (uint32_t*)d_off.p);
-            }
-            k_scatter<<<n_all, kTile, 0, st>>>((const Tile*)d_tiles.p, n_all, ds, K, binf, srt,
-                                               (const uint32_t*)d_off.p, order, n, order_tmp, misc + 1);
-            k_copy_back<<<n_all, kTile, 0, st>>>((const Tile*)d_tiles.p, n_all, order_tmp, order, n);
-            // Children: ranges, exact boxes, then the parents' links.
-            {
-                std::vector<InterimNode> ch(n_children);
-                for (size_t j = 0; j < ch.size(); j++) {
-                    ch[j] = InterimNode{};
-                    ch[j].beg = h_beg[children[j]];
-                    ch[j].cnt = h_cnt[children[j]];
-                }
-                // children ids are consecutive
-                if ((s = upload(nodes + children[0], std::move(ch)))) return s;
-            }
-            if ((s = node_boxes(children))) return s;
-            if ((s = ensure(d_ids, cap_ids, triples.size() * 4, "ids"))) return s;
-            if ((s = upload(d_ids.p, std::move(triples)))) return s;
-            k_link<<<blocks(n_links, 128), 128, 0, st>>>((const uint32_t*)d_ids.p, n_links, nodes, max_nodes,
-                                                         misc + 1);
-            for (uint32_t c : children) {
+            links.push_back(Link{slots[k].id, l, slots[k].beg, d.nl, slots[k].cnt});
+            for (uint32_t c : {l, r}) {
+                tiles_of(boxes, c - first_child, 0, h_beg[c], h_cnt[c]);
                 if (h_cnt[c] > kSmall) next_active.push_back(c);
                 else if (h_cnt[c] >= 2) small.push_back(c);
             }
+        }
+        if (!links.empty()) {
+            // coordinate-binned tiles first (their block index is the tile_off row), then uniform
+            const size_t n_fl = fl.size();
+            fl.insert(fl.end(), part.begin(), part.end());
+            const uint32_t n_all = (uint32_t)fl.size(), n_links = (uint32_t)links.size(),
+                           n_boxes = (uint32_t)boxes.size();
+            Lists sl;
+            const size_t at_all = sl.add(fl), at_st = sl.add(slot_tiles), at_boxes = sl.add(boxes),
+                         at_links = sl.add(links);
+            if ((s = upload_lists(d_split, cap_split, sl)) ||
+                (s = ensure(d_hist, cap_hist, std::max<size_t>(n_fl, 1) * kBins * 4, "histograms")) ||
+                (s = ensure(d_off, cap_off, std::max<size_t>(n_fl, 1) * kBins * 4, "offsets")))
+                return s;
+            const char* lb = (const char*)d_split.p;
+            const Tile* d_all = (const Tile*)(lb + at_all);
+            if (n_fl) {
+                k_tile_hist<<<(unsigned)n_fl, kTile, 0, st>>>(d_all, (uint32_t)n_fl, binf, n, (uint32_t*)d_hist.p);
+                k_tile_offsets<<<(unsigned)(slot_tiles.size() / 2), 1024, 0, st>>>(
+                    (const uint32_t*)(lb + at_st), (uint32_t)(slot_tiles.size() / 2), (const uint32_t*)d_hist.p,
+                    (uint32_t*)d_off.p);
+            }
+            k_scatter<<<n_all, kTile, 0, st>>>(d_all, n_all, ds, K, binf, srt, (const uint32_t*)d_off.p, order, n,
+                                               order_tmp, misc + 1);
+            k_copy_back<<<n_all, kTile, 0, st>>>(d_all, n_all, order_tmp, order, n);
+            // Children: exact boxes, then the parents' links and the ranges.
+            if ((s = node_boxes(first_child, 2 * n_links, (const Tile*)(lb + at_boxes), n_boxes))) return s;
+            k_link<<<blocks(n_links, 128), 128, 0, st>>>((const Link*)(lb + at_links), n_links, nodes, max_nodes,
+                                                         misc + 1);
         }
         active.swap(next_active);
     }
