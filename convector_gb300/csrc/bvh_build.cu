@@ -1196,42 +1196,53 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     const uint32_t max_nodes = 2 * n;
     const uint32_t max_slots = n / (kSmall + 1) + 1;
 
-    DevBuf d_tris, d_refs, d_order, d_tmp, d_srt, d_binf, d_nodes, d_inner, d_tx, d_tt, d_misc, d_cnt, d_key,
-        d_mode, d_dec, d_level, d_split, d_tiles2, d_hist, d_off, d_ids, d_acc, d_sortbuf, d_pairs;
+    // The arrays whose sizes are known lie in one allocation: each one of its own
+    // takes 20 us to make and 20 to release (81,920 triangles 5.10 -> 4.69 ms).
+    size_t total = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = total;
+        total += (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+        return at;
+    };
+    const size_t at_tris = place((size_t)n * sizeof(cvx_triangle)), at_refs = place((size_t)9 * n * 4),
+                 at_order = place((size_t)n * 4), at_tmp = place((size_t)n * 4), at_srt = place((size_t)3 * n * 4),
+                 at_binf = place((size_t)3 * n), at_nodes = place((size_t)max_nodes * sizeof(InterimNode)),
+                 at_inner = place((size_t)6 * max_nodes * 4), at_tx = place(((size_t)n + 1) * 4),
+                 at_tt = place(((size_t)n + 1) * 4), at_misc = place(4 * 4),
+                 at_cnt = place((size_t)max_slots * 3 * kBins * 4), at_key = place((size_t)max_slots * 3 * kBins * 6 * 4),
+                 at_mode = place((size_t)max_slots * 3 * 4), at_dec = place(((size_t)max_slots + 1) * sizeof(Decision)),
+                 at_out_nodes = place((size_t)max_nodes * sizeof(cvx_bvh_node)),
+                 at_out_tris = place((size_t)n * sizeof(cvx_triangle));
+    DevBuf d_arrays, d_level, d_split, d_tiles2, d_hist, d_off, d_ids, d_acc, d_sortbuf, d_pairs;
     int32_t s = 0;
-    if ((s = dalloc<cvx_triangle>(d_tris, n, "triangles")) || (s = dalloc<float>(d_refs, (size_t)9 * n, "refs")) ||
-        (s = dalloc<uint32_t>(d_order, n, "order")) || (s = dalloc<uint32_t>(d_tmp, n, "order")) ||
-        (s = dalloc<uint32_t>(d_srt, (size_t)3 * n, "sort")) || (s = dalloc<uint8_t>(d_binf, (size_t)3 * n, "bins")) ||
-        (s = dalloc<InterimNode>(d_nodes, max_nodes, "nodes")) ||
-        (s = dalloc<float>(d_inner, (size_t)6 * max_nodes, "inner boxes")) ||
-        (s = dalloc<float>(d_tx, (size_t)n + 1, "tsah")) || (s = dalloc<float>(d_tt, (size_t)n + 1, "tsah")) ||
-        (s = dalloc<uint32_t>(d_misc, 4, "flags")) ||
-        (s = dalloc<uint32_t>(d_cnt, (size_t)max_slots * 3 * kBins, "bin counts")) ||
-        (s = dalloc<uint32_t>(d_key, (size_t)max_slots * 3 * kBins * 6, "bin boxes")) ||
-        (s = dalloc<uint32_t>(d_mode, (size_t)max_slots * 3, "modes")) ||
-        (s = dalloc<Decision>(d_dec, (size_t)max_slots + 1, "decisions")))
-        return s;
-    cvx_triangle* tri_d = (cvx_triangle*)d_tris.p;
-    float* refs = (float*)d_refs.p;
+    if ((s = dalloc<char>(d_arrays, total, "arrays"))) return s;
+    char* const base = (char*)d_arrays.p;
+    cvx_triangle* tri_d = (cvx_triangle*)(base + at_tris);
+    float* refs = (float*)(base + at_refs);
     Refs R;
     for (int c = 0; c < 3; c++) {
         R.lo[c] = refs + (size_t)c * n;
         R.hi[c] = refs + (size_t)(3 + c) * n;
         R.bc[c] = refs + (size_t)(6 + c) * n;
     }
-    uint32_t* order = (uint32_t*)d_order.p;
-    uint32_t* order_tmp = (uint32_t*)d_tmp.p;
-    uint32_t* srt = (uint32_t*)d_srt.p;
-    uint8_t* binf = (uint8_t*)d_binf.p;
-    InterimNode* nodes = (InterimNode*)d_nodes.p;
-    float* inner = (float*)d_inner.p;
-    uint32_t* misc = (uint32_t*)d_misc.p;  // [0] bad input, [1] error bits, [2] next node id, [3] depth
-    BinStats bs{(uint32_t*)d_cnt.p, (uint32_t*)d_key.p};
-    Tsah ts{(const float*)d_tx.p, (const float*)d_tt.p, ty};
+    uint32_t* order = (uint32_t*)(base + at_order);
+    uint32_t* order_tmp = (uint32_t*)(base + at_tmp);
+    uint32_t* srt = (uint32_t*)(base + at_srt);
+    uint8_t* binf = (uint8_t*)(base + at_binf);
+    InterimNode* nodes = (InterimNode*)(base + at_nodes);
+    float* inner = (float*)(base + at_inner);
+    uint32_t* misc = (uint32_t*)(base + at_misc);  // [0] bad input, [1] error bits, [2] next node id, [3] depth
+    BinStats bs{(uint32_t*)(base + at_cnt), (uint32_t*)(base + at_key)};
+    float *d_tx = (float*)(base + at_tx), *d_tt = (float*)(base + at_tt);
+    Tsah ts{d_tx, d_tt, ty};
+    uint32_t* const dm = (uint32_t*)(base + at_mode);
+    Decision* const d_dec = (Decision*)(base + at_dec);
+    cvx_bvh_node* const out_nodes = (cvx_bvh_node*)(base + at_out_nodes);
+    cvx_triangle* const out_tris = (cvx_triangle*)(base + at_out_tris);
 
     BK(cudaMemcpyAsync(tri_d, tris, (size_t)n * sizeof(cvx_triangle), cudaMemcpyHostToDevice, st), "upload");
-    BK(cudaMemcpyAsync(d_tx.p, tx.data(), tx.size() * 4, cudaMemcpyHostToDevice, st), "upload");
-    BK(cudaMemcpyAsync(d_tt.p, tt.data(), tt.size() * 4, cudaMemcpyHostToDevice, st), "upload");
+    BK(cudaMemcpyAsync(d_tx, tx.data(), tx.size() * 4, cudaMemcpyHostToDevice, st), "upload");
+    BK(cudaMemcpyAsync(d_tt, tt.data(), tt.size() * 4, cudaMemcpyHostToDevice, st), "upload");
     BK(cudaMemsetAsync(misc, 0, 16, st), "memset");
     BK(cudaMemsetAsync(nodes, 0, (size_t)max_nodes * sizeof(InterimNode), st), "memset");
     const float third = 1.0f / 3.0f;
@@ -1251,7 +1262,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         if (b.p) cudaFree(b.p);
         b.p = nullptr;
         cap = 0;
-        const size_t want = std::max(2 * bytes, (size_t)1 << 16);
+        const size_t want = std::max(2 * bytes, (size_t)1 << 20);
         cudaError_t e = cudaMalloc(&b.p, want);
         if (e != cudaSuccess)
             return set_error(CVX_ERR_DEVICE, std::string("device BVH build: ") + what + ": " + cudaGetErrorString(e));
@@ -1314,17 +1325,16 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         if ((s = upload_lists(d_level, cap_level, lists))) return s;
         const Slot* ds = (const Slot*)((const char*)d_level.p + at_slots);
         const Tile* dt = (const Tile*)((const char*)d_level.p + at_tiles);
-        uint32_t* dm = (uint32_t*)d_mode.p;
         k_stats_init<<<blocks((size_t)K * 3 * kBins, 256), 256, 0, st>>>(bs, K * 3 * kBins);
         k_bin_float<<<n_tl, kTile, 0, st>>>(dt, n_tl, ds, K, R, order, n, inner, binf, bs, misc + 1);
         k_fallback<<<blocks((size_t)K * 3 * 32, 128), 128, 0, st>>>(ds, K, bs, dm);
         // Uniform split (bvh.rs:176-201) where coordinate binning fell back.
         k_sort_slots<<<3 * K, 1024, 0, st>>>(ds, K, dm, R, order, n, srt, misc + 1);
         k_uniform_stats<<<dim3(n_tl, 3), kTile, 0, st>>>(dt, n_tl, dm, ds, K, R, order, n, srt, bs, misc + 1);
-        k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, dm, misc + 1, (Decision*)d_dec.p);
+        k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, dm, misc + 1, d_dec);
         std::vector<Decision> dec((size_t)K + 1);
         auto decisions = [&]() -> int32_t {
-            BK(cudaMemcpyAsync(dec.data(), d_dec.p, dec.size() * sizeof(Decision), cudaMemcpyDeviceToHost, st),
+            BK(cudaMemcpyAsync(dec.data(), d_dec, dec.size() * sizeof(Decision), cudaMemcpyDeviceToHost, st),
                "download");
             BK(cudaStreamSynchronize(st), "split choice");
             keep.clear();
@@ -1370,7 +1380,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
                                                                                (uint32_t)big_pairs.size(), bs);
             k_uniform_stats<<<n_uni, kTile, 0, st>>>((const Tile*)d_tiles2.p, n_uni, nullptr, ds, K, R, order, n, srt,
                                                      bs, misc + 1);
-            k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, dm, misc + 1, (Decision*)d_dec.p);
+            k_choose<<<K, 96, 0, st>>>(ds, K, nodes, bs, ts, dm, misc + 1, d_dec);
             if ((s = decisions())) return s;
         }
 
@@ -1452,11 +1462,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
 
     // The reference's node array and triangle order. The boxes of the levels
     // are no longer needed: their memory holds the crystallization's state.
-    DevBuf d_out_nodes, d_out_tris;
-    if ((s = dalloc<cvx_bvh_node>(d_out_nodes, max_nodes, "nodes")) ||
-        (s = dalloc<cvx_triangle>(d_out_tris, n, "triangles")))
-        return s;
-    uint32_t* state = (uint32_t*)d_inner.p;  // 6 * max_nodes words
+    uint32_t* state = (uint32_t*)inner;  // 6 * max_nodes words
     const Crystal cr{state, state + max_nodes, state + 2 * (size_t)max_nodes, state + 3 * (size_t)max_nodes,
                      (float*)(state + 4 * (size_t)max_nodes)};
     BK(cudaMemsetAsync(cr.parent, 0xff, (size_t)max_nodes * 4, st), "memset");
@@ -1465,7 +1471,7 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     k_crystal_parents<<<cb, 256, 0, st>>>(nodes, misc + 2, cr, misc + 1);
     k_crystal_up<<<cb, 256, 0, st>>>(nodes, misc + 2, cr, misc + 1);
     k_crystal_emit<<<cb, 256, 0, st>>>(nodes, misc + 2, cr, order, n, (const float4*)tri_d,
-                                       (cvx_bvh_node*)d_out_nodes.p, (float4*)d_out_tris.p, order_tmp, misc + 3,
+                                       out_nodes, (float4*)out_tris, order_tmp, misc + 3,
                                        misc + 1);
     BK(cudaGetLastError(), "crystallize");
     // The result's memory, while the kernels run.
@@ -1496,9 +1502,9 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         return set_error(CVX_ERR_DEVICE, "device BVH build: unreachable interim nodes");
     const size_t m = 2 * (size_t)root_inner;
     bvh->nodes.resize(m);
-    BK(cudaMemcpyAsync(bvh->nodes.data(), d_out_nodes.p, m * sizeof(cvx_bvh_node), cudaMemcpyDeviceToHost, st),
+    BK(cudaMemcpyAsync(bvh->nodes.data(), out_nodes, m * sizeof(cvx_bvh_node), cudaMemcpyDeviceToHost, st),
        "download");
-    BK(cudaMemcpyAsync(bvh->triangles.data(), d_out_tris.p, (size_t)n * sizeof(cvx_triangle), cudaMemcpyDeviceToHost,
+    BK(cudaMemcpyAsync(bvh->triangles.data(), out_tris, (size_t)n * sizeof(cvx_triangle), cudaMemcpyDeviceToHost,
                        st),
        "download");
     BK(cudaMemcpyAsync(bvh->source_index.data(), order_tmp, (size_t)n * 4, cudaMemcpyDeviceToHost, st), "download");
