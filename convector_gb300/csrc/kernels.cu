@@ -110,10 +110,10 @@ __global__ void k_prep_lights(const cvx_triangle* __restrict__ tris, const uint3
 }
 
 // ---------------------------------------------------------------------------
-// Nearest hit over SoA rays (Bvh::intersect_nearest, bvh.rs:659). The packet
-// form (k_intersect<true>: eight consecutive rays are one reference packet)
-// is the reference's traversal exactly; the single-ray form is
-// k_intersect_refill below.
+// Nearest hit over SoA rays (Bvh::intersect_nearest, bvh.rs:659): eight
+// consecutive rays are one reference packet, or each is traced by itself
+// (k_intersect_packets, k_intersect_warp; k_intersect_refill, k_intersect_lanes
+// below). k_intersect_counts also counts the boxes and triangles of packets.
 
 // Next unit (group or packet) index for the calling octet (one atomic by its lane 0).
 __device__ __forceinline__ uint32_t octet_claim(uint32_t* counter, unsigned omask, int k) {
@@ -122,11 +122,10 @@ __device__ __forceinline__ uint32_t octet_claim(uint32_t* counter, unsigned omas
     return __shfl_sync(omask, g, (int)(threadIdx.x & 24u));
 }
 
-template <bool PACKET>
-__global__ void __launch_bounds__(256) k_intersect(DeviceScene s, const RayCols rays, uint32_t n,
-                                                   float far_dist, float* __restrict__ t_out,
-                                                   int32_t* __restrict__ tri_out, uint32_t* __restrict__ counters,
-                                                   uint32_t* __restrict__ err) {
+__global__ void __launch_bounds__(256) k_intersect_counts(DeviceScene s, const RayCols rays, uint32_t n,
+                                                          float far_dist, float* __restrict__ t_out,
+                                                          int32_t* __restrict__ tri_out,
+                                                          uint32_t* __restrict__ counters, uint32_t* __restrict__ err) {
     __shared__ ApproxTables tab;
     load_tables(tab);
     const unsigned omask = 0xffu << (threadIdx.x & 24u);
@@ -141,22 +140,12 @@ __global__ void __launch_bounds__(256) k_intersect(DeviceScene s, const RayCols 
         F3 d = f3(__ldg(rays.c[3] + src), __ldg(rays.c[4] + src), __ldg(rays.c[5] + src));
         Hit h{far_dist, 0.0f, 0.0f, -1};
         Counters c{0u, 0u};
-        bool ok = true;
-        // The select-form slab test for a packet whose 8 rays all allow it,
-        // decided once per packet outside the traversal loop (4M random rays:
-        // 3.05 -> 2.92 ms; the same results).
-        const bool sel = PACKET && s.slab_sel && !counters &&
-                         oct_all(omask, select_form_ray(o, f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab))));
-        if (sel) ok = traverse<true, true>(s, o, d, active, omask, h, tab, nullptr);
-        else if (PACKET || active) ok = traverse<PACKET>(s, o, d, active, omask, h, tab, counters ? &c : nullptr);
-        if (!ok) atomicOr(err, kErrStackOverflow);
+        if (!traverse<true>(s, o, d, active, omask, h, tab, &c)) atomicOr(err, kErrStackOverflow);
         if (active) {
             t_out[i] = h.t;
             tri_out[i] = h.tri;
-            if (counters) {
-                counters[i] = c.aabb;
-                counters[n + i] = c.tri;
-            }
+            counters[i] = c.aabb;
+            counters[n + i] = c.tri;
         }
     }
 }
@@ -515,6 +504,8 @@ __device__ __forceinline__ void flush_rays(const FrameArgs& a, uint32_t rays) {
     if ((threadIdx.x & 31u) == 0u && v) atomicAdd(a.rays, v);
 }
 
+// An octet renders whole groups: single rays, and the debug view (PACKET: of
+// packets; their frames take k_render_packets).
 template <bool PACKET>
 __global__ void __launch_bounds__(128, 8) k_render_group(FrameArgs a) {
     __shared__ ApproxTables tab;
@@ -544,8 +535,8 @@ __global__ void __launch_bounds__(128, 8) k_render_group(FrameArgs a) {
         x = fmaf(unit_from(rng.next()), scale, x);
         y = fmaf(unit_from(rng.next()), scale, y);
         PixelOut p;
-        if (a.debug) ok &= render_pixels_debug<PACKET>(a.s, a.cam, x, y, omask, tab, p, rays);
-        else ok &= render_pixels<PACKET>(a.s, a.cam, x, y, rng, omask, tab, p, rays);
+        if (PACKET || a.debug) ok &= render_pixels_debug<PACKET>(a.s, a.cam, x, y, omask, tab, p, rays);
+        else ok &= render_pixels<false>(a.s, a.cam, x, y, rng, omask, tab, p, rays);
         store_pixel(a, gx + (uint32_t)(k & 3), gy + (uint32_t)(k >> 2), p);
     }
     if (!ok) atomicOr(a.err, kErrStackOverflow);
@@ -759,14 +750,12 @@ __global__ void __launch_bounds__(256) k_accumulate_samples(float* __restrict__ 
     }
 }
 
-// One resident block per SM is all the launch bound asks: the frame's few
-// hundred chains leave most warp slots empty, so registers are free, and with
-// the bound of 128 threads alone the compiler capped the kernel at 64
-// registers and spilled 48 bytes (packet 32) on the chains' critical path.
-// Without the cap (118 and 100 registers, no spill): room frame 17.49 ->
-// 17.01 ms, icosphere 26.52 -> 26.00 ms. (The packet traversal's stack top
-// held in registers, as in the refill step, measured slower: packet query
-// 2.92 -> 3.03 ms, packet frame 1.21 -> 1.32 ms.)
+// Patch order for single rays, and the debug view (PACKET: of packets; their
+// frames take k_render_patch_warp): an octet per patch. One resident block per SM
+// is all the launch bound asks: the frame's few hundred chains leave most warp
+// slots empty, so registers are free, and with the bound of 128 threads alone the
+// compiler capped the kernel at 64 registers and spilled on the chains' critical
+// path.
 template <bool PACKET>
 __global__ void __launch_bounds__(128, 1) k_render_patch(FrameArgs a) {
     __shared__ ApproxTables tab;
@@ -802,8 +791,8 @@ __global__ void __launch_bounds__(128, 1) k_render_patch(FrameArgs a) {
                     x = fmaf(jx[g], scale, x);
                     y = fmaf(jy[g], scale, y);
                     PixelOut p;
-                    if (a.debug) ok &= render_pixels_debug<PACKET>(a.s, a.cam, x, y, omask, tab, p, rays);
-                    else ok &= render_pixels<PACKET>(a.s, a.cam, x, y, rng, omask, tab, p, rays);
+                    if (PACKET || a.debug) ok &= render_pixels_debug<PACKET>(a.s, a.cam, x, y, omask, tab, p, rays);
+                    else ok &= render_pixels<false>(a.s, a.cam, x, y, rng, omask, tab, p, rays);
                     store_pixel(a, xb + 4u * (uint32_t)(g >> 1) + (uint32_t)(k & 3),
                                 yb + 2u * (uint32_t)(g & 1) + (uint32_t)(k >> 2), p);
                 }
@@ -1100,7 +1089,7 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
     uint32_t need = ((n + 7u) & ~7u) / block + 1u;
     uint32_t blocks = (uint32_t)num_sms() * blocks_per_sm;
     if (blocks > need) blocks = need;
-    k_intersect<true><<<blocks, block, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, counters, err);
+    k_intersect_counts<<<blocks, block, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, counters, err);
     return cudaGetLastError();
 }
 

@@ -224,8 +224,8 @@ int32_t cvx_intersect_nearest_noalloc(cvx_scene* scene, const float* ox, const f
 /* ---- device: renderer ---------------------------------------------------- */
 
 /* RNG order: CVX_RNG_PATCH reproduces the reference's stream exactly (one
- * generator per 32x32 patch, renderer.rs:306-327; one octet per patch on the
- * GPU); CVX_RNG_GROUP seeds each 8-pixel group from its own pixel
+ * generator per 32x32 patch, renderer.rs:306-327; on the GPU each patch is a
+ * chain); CVX_RNG_GROUP seeds each 8-pixel group from its own pixel
  * coordinates so that every group renders in parallel. */
 enum { CVX_RNG_PATCH = 0, CVX_RNG_GROUP = 1 };
 /* Kernel organisation: one fused kernel per frame, or the wavefront form
