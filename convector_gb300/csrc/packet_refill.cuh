@@ -225,6 +225,11 @@ struct PacketRay {
 #pragma unroll 1
             for (int st = 0; st < STEPS; st++) walk<true>(on, stack, overflow);
             fin = test_leaf(on);
+            // Two records may lead to two leaves, of which the second stopped its packet:
+            // tested now instead of after the next round (1M packets: room 311 -> 299
+            // us, icosphere 632 -> 620; frames -0.6 and -1 %). With one record per round a
+            // second test costs 1.5 %.
+            if (STEPS > 1 && __any_sync(kFullWarp, on && leaf != 0u)) fin = test_leaf(on);
         } else {
 #pragma unroll 1
             for (int st = 0; st < STEPS; st++) {
