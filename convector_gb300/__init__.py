@@ -419,7 +419,7 @@ class Scene:
 
     def set_query_stack(self, shared_entries):
         """Stack entries per lane the single-ray query keeps in shared memory
-        (0, 4, 8 or 12; default 8)."""
+        (0, 4, 8 or 12; 0 if never set)."""
         _check(lib().cvx_scene_set_query_stack(self._h, shared_entries))
 
     def set_host_access(self, mode):

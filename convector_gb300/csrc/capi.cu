@@ -118,7 +118,7 @@ struct cvx_scene {
     uint32_t n_nodes = 0, n_tris = 0, n_lights = 0, depth = 0;
     uint32_t general_pick = 1;
     uint32_t blocks_per_sm = 0;  // launch shape of the nearest-hit query (0: default)
-    uint32_t query_stack = 8;    // stack entries per lane in shared memory (cvx_scene_set_query_stack)
+    uint32_t query_stack = kQueryStackDefault;  // entries per lane in shared memory (cvx_scene_set_query_stack)
     // The device reads host memory through the host's page tables (address
     // translation over a coherent CPU-GPU link): the host-buffer query may
     // read the caller's ray arrays in place. host_access: CVX_HOST_ACCESS_*.

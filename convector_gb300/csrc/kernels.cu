@@ -266,12 +266,6 @@ struct StagedSoaClaim {
 // (shallow trees) gain from large batches of claims, long ones lose more to
 // the waiting: 16 for trees up to 40 levels, 8 beyond (measured on the
 // 82k-triangle icosphere and on the 70-level tube).
-// The first entries of each lane's traversal stack live in shared memory,
-// the deeper ones in local memory. Pops of local entries missed L1 about a
-// third of the time (68.7 % hit rate); measured on 4M rays: 0.905 ms with none
-// shared, 0.890 with 4, 0.878 with 8, 0.883 with 12. (The wavefront and the
-// path-refill traversals, whose larger working sets need the L1 that the
-// carve-out takes, measured no gain or a loss.)
 // Wide records a lane walks per round of the warp's claim votes, before the
 // round's leaf test (RefillRay::walk; traversal steps, leaves included, in the
 // x86 form). The kernel is bound by instruction issue and the ALU pipe: with a
@@ -287,8 +281,13 @@ struct StagedSoaClaim {
 // 615, 605, 719; 472, 475, 546; 145, 146, 168 us. Ending a round early when few
 // lanes can walk on costs more in votes than it saves (748-794 us with pairs).
 constexpr int kQuerySteps = 2;
-// The default; a scene may choose 0, 4 or 12 instead (cvx_scene_set_query_stack,
-// which the query autotuner sets per scene).
+// Each lane's traversal stack lies in local memory. A scene may keep the first 4, 8
+// or 12 entries in shared memory instead (cvx_scene_set_query_stack, which the query
+// autotuner sets per scene). Eight shared entries were the better default while
+// pops of local entries waited for L1 (0.905 -> 0.878 ms per 4M rays); with pushes by
+// selects one store to one memory is: 0 and 8 shared, us: 4M icosphere rays 564,
+// 592, 1M tube rays 387, 408, room 136, 143; packets 598, 618, 1165, 1210, 290, 297.
+// The other launch shapes keep 8.
 constexpr int kQueryStackShared = 8;
 
 // SELECT: the select-form slab test and postponed leaves for the rays that
@@ -318,7 +317,7 @@ __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uin
 // 1340 us. 7 blocks per SM (72 registers; 8 blocks spill: 329, 676, 1355 us).
 // STEPS records per round: 1, 2, 3 -> 309, 311, 379 us (room), 650, 628, 716
 // (icosphere), 1210, 1279, 1543 (tube): 1 for trees deeper than 40 levels, else 2.
-// 4, 8 or 12 shared stack entries are alike; waiting for two finished packets
+// Waiting for two finished packets
 // before taking new ones 322, 701, 1312 us.
 constexpr int kPacketBlocksPerSm = 7;
 template <int STEPS>
@@ -326,11 +325,9 @@ __global__ void __launch_bounds__(128, kPacketBlocksPerSm) k_intersect_packets(S
                                                                                uint32_t* __restrict__ next_ray,
                                                                                uint32_t* __restrict__ err) {
     __shared__ float stage[4][2][6][32];
-    __shared__ uint2 sstack[4][kQueryStackShared][32];
     StagedSoaClaim claim{src, next_ray, stage[threadIdx.x >> 5], 0u, 0u, 0u, 0};
     claim.init(threadIdx.x & 31);
-    bool ok = traverse_packets<STEPS, kQueryStackShared>(src, claim, g_tables,
-                                                         &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
+    bool ok = traverse_packets<STEPS>(src, claim, g_tables);
     if (!ok) atomicOr(err, kErrStackOverflow);
 }
 
@@ -665,39 +662,27 @@ constexpr int kRefillFrameSteps = 2;
 
 // COUNT: the same frame, also counting its work (FrameArgs::work); the
 // counters cost registers, so frames are rendered without them.
-// Trees deeper than 40 levels (the DEEP instantiation) keep the first
-// 16 stack entries of each lane in shared memory and read the approximation
-// tables from global memory instead (the 16 KB of entries per block take the
-// room the tables would); shallower trees keep the whole stack local. Measured
-// on the 870k-triangle tube (70 levels), ms per 1280x736 sample: local stack
-// 3.07-3.11; 4, 8 entries 3.11, 3.03; 8, 12, 16 with the tables in global
-// memory 3.10, 3.04, 2.99 (20, 24, 32: 2.96, 3.00, 3.19). On the 19-level room
-// the same entries cost 3-4 %.
-constexpr int kDeepFrameStackShared = 16;
-
 // Deep trees (the DEEP instantiation): claim threshold 12, two wide records per
 // round, and the warp's leaves tested together. 870k tube, 1280x736, 16 samples in
 // one launch: 23.2 ms (35.7 with pairs and leaves tested at once, 28.7 with four
 // pairs per round and postponed leaves, 25.7 with two wide records per round;
 // one and three records per round 24.1-25.6, 25.9; claim 8, 14: 23.9, 23.2; 6 and
-// 8 resident blocks per SM 24.7 and 23.4).
+// 8 resident blocks per SM 24.7 and 23.4); 21.9 with one pop per step, and 21.7
+// with the whole stack in local memory as in shallow trees: 16 shared entries per
+// lane helped while each push and pop was a branch of its own (4 entries 22.3 ms;
+// one sample per launch 1.93 against 1.99 ms).
 constexpr int kDeepFrameClaim = 12;
 constexpr int kDeepFrameSteps = 2;
-// DEEP: a tree deeper than 40 levels (shared stack entries, the constants above).
+// DEEP: a tree deeper than 40 levels (the constants above).
 // MULTI: a.samples samples in one launch (FramePaths<true>).
 template <bool DEEP, bool COUNT, bool MULTI = false>
 __global__ void __launch_bounds__(128, kRefillFrameBlocksPerSm) k_render_refill(FrameArgs a) {
     FramePaths<MULTI> P{a, (a.w + 15u) / 16u, (a.h + 3u) / 4u, 0u};
+    __shared__ ApproxTables tab;
+    load_tables(tab);
     bool ok;
-    if constexpr (DEEP) {
-        __shared__ uint2 sstack[4][kDeepFrameStackShared][32];
-        ok = path_refill<kDeepFrameClaim, kDeepFrameSteps, COUNT, true, kDeepFrameStackShared, true>(
-            P, g_tables, &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
-    } else {
-        __shared__ ApproxTables tab;
-        load_tables(tab);
-        ok = path_refill<16, kRefillFrameSteps, COUNT, true>(P, tab);
-    }
+    if constexpr (DEEP) ok = path_refill<kDeepFrameClaim, kDeepFrameSteps, COUNT, true, true>(P, tab);
+    else ok = path_refill<16, kRefillFrameSteps, COUNT, true>(P, tab);
     if (!ok) atomicOr(a.err, kErrStackOverflow);
 }
 
@@ -1027,10 +1012,10 @@ template <int CLAIM>
 static void launch_select_stack(uint32_t shared, uint32_t blocks, const SoaRays& src, uint32_t* err,
                                 cudaStream_t st) {
     switch (shared) {
-        case 0: k_intersect_refill<8, false, CLAIM, true, 0><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
         case 4: k_intersect_refill<8, false, CLAIM, true, 4><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
         case 12: k_intersect_refill<8, false, CLAIM, true, 12><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
-        default: k_intersect_refill<8, false, CLAIM, true, 8><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
+        case 8: k_intersect_refill<8, false, CLAIM, true, 8><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
+        default: k_intersect_refill<8, false, CLAIM, true, 0><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
     }
 }
 
@@ -1039,7 +1024,8 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
                              uint32_t blocks_per_sm, cudaStream_t st, uint32_t shared_stack) {
     // Calls that do not fill the GPU several times over: one packet per warp, or
     // one ray per lane, with nothing claimed (kDirectRays).
-    if (!counters && n <= kDirectRays && blocks_per_sm == 0 && shared_stack == kQueryStackShared) {
+    if (!counters && n <= kDirectRays && blocks_per_sm == 0 &&
+        (shared_stack == kQueryStackDefault || shared_stack == kQueryStackShared)) {
         if (packet) k_intersect_warp<<<(n + 15u) / 16u, 64, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
         else k_intersect_lanes<<<(n + 31u) / 32u, 32, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
         return cudaGetLastError();

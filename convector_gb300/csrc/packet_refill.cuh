@@ -150,10 +150,9 @@ struct PacketRay {
     }
 
     // The boxes to visit, from the last to the first: each becomes the next
-    // node, and the one before it is pushed: by selects where a push is one
-    // store (frames: room 1.127 -> 1.119 ms, icosphere 2.76 -> 2.72, 320x184 of it
-    // 0.57 -> 0.53), else by branches (queries, whose first entries are in shared
-    // memory: 1M room packets 311, by selects 316 us). Then a leaf goes to wait, if
+    // node, and the one before it is pushed, by selects (as branches, frames: room
+    // 1.127 -> 1.119 ms, icosphere 2.76 -> 2.72, 320x184 of it 0.57 -> 0.53; a push that
+    // may go to shared memory is better as a branch). Then a leaf goes to wait, if
     // none does.
     template <int N, class Stack>
     __device__ __forceinline__ void push(const bool (&v)[N], const uint32_t (&r)[N], const float (&t)[N], Stack& stack,
@@ -161,23 +160,13 @@ struct PacketRay {
         cur = kNone;
 #pragma unroll
         for (int k = 0; k < N; k++) {
-            if constexpr (Stack::kOneStore) {
-                const bool p = k > 0 && v[k] && cur != kNone;
-                if (p) stack.store(sp, top);
-                top.x = p ? cur : top.x;
-                top.y = p ? __float_as_uint(cur_t) : top.y;
-                sp += p;
-                cur = v[k] ? r[k] : cur;
-                cur_t = v[k] ? t[k] : cur_t;
-            } else if (v[k]) {
-                if (k > 0 && cur != kNone) {
-                    stack.store(sp, top);
-                    top = make_uint2(cur, __float_as_uint(cur_t));
-                    sp++;
-                }
-                cur = r[k];
-                cur_t = t[k];
-            }
+            const bool p = k > 0 && v[k] && cur != kNone;
+            if (p) stack.store(sp, top);
+            top.x = p ? cur : top.x;
+            top.y = p ? __float_as_uint(cur_t) : top.y;
+            sp += p;
+            cur = v[k] ? r[k] : cur;
+            cur_t = v[k] ? t[k] : cur_t;
         }
         if (sp > c_stack_limit) {
             overflow = true;
@@ -245,16 +234,14 @@ struct PacketRay {
 // consecutive rays; src as in traverse_refill, with one scene). A finished packet
 // is replaced at once. The lanes of a last, partial packet beyond its rays are
 // inactive copies of its first lane's ray.
-template <int STEPS, int SHARED_STACK, class Src, class Claim>
-__device__ __forceinline__ bool traverse_packets(const Src& src, Claim& claim, const ApproxTables& tab,
-                                                 uint2* shared_stack) {
+template <int STEPS, class Src, class Claim>
+__device__ __forceinline__ bool traverse_packets(const Src& src, Claim& claim, const ApproxTables& tab) {
     const int lane = threadIdx.x & 31;
     PacketRay ray;
     ray.clear();
     src.first_scene(ray.nodes, ray.wide, ray.geom);
     uint2 local_stack[kStackSlots];
-    typename std::conditional<SHARED_STACK == 0, LocalStack, SharedLocalStack<SHARED_STACK>>::type stack =
-        make_stack<SHARED_STACK>(shared_stack, local_stack);
+    LocalStack stack{local_stack};
     uint32_t r_id = 0;
     bool have = false, done = false, sel = false, overflow = false;
     for (;;) {

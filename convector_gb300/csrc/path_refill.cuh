@@ -52,9 +52,9 @@ namespace cvx {
 // form. Each lane's results are the same either way.
 // POOL_LEAVES: such a round's leaves are tested by the whole warp (RefillRay::
 // test_leaves).
-template <int CLAIM_MIN, int STEPS, bool COUNT = false, bool SELECT_ROUNDS = false, int SHARED_STACK = 0,
-          bool POOL_LEAVES = false, class Paths>
-__device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, uint2* shared_stack = nullptr) {
+template <int CLAIM_MIN, int STEPS, bool COUNT = false, bool SELECT_ROUNDS = false, bool POOL_LEAVES = false,
+          class Paths>
+__device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab) {
     typedef typename Paths::PathRef PathRef;
     __shared__ uint8_t owners[4][32];  // RefillRay::test_leaves, blocks of four warps
     uint8_t* const owner = owners[threadIdx.x >> 5];
@@ -62,8 +62,7 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, u
     const uint32_t npaths = P.n_paths();
     RefillRay ray;
     uint2 local_stack[kStackSlots];
-    typename std::conditional<SHARED_STACK == 0, LocalStack, SharedLocalStack<SHARED_STACK>>::type stack =
-        make_stack<SHARED_STACK>(shared_stack, local_stack);
+    LocalStack stack{local_stack};
     ray.top = make_uint2(0u, 0u);
     ray.sp = 0;
     ray.cur = RefillRay::kNone;

@@ -394,14 +394,12 @@ constexpr int kStackSlots = kStackDepth + 4;
 // in this lane's column of a warp's [N][32] block (no bank conflicts, and pops
 // of those never miss the cache), the deeper ones in the local array.
 struct LocalStack {
-    static constexpr bool kOneStore = true;
     uint2 (&a)[kStackSlots];
     __device__ __forceinline__ uint2 load(int i) const { return a[i]; }
     __device__ __forceinline__ void store(int i, uint2 v) { a[i] = v; }
 };
 template <int N>
 struct SharedLocalStack {
-    static constexpr bool kOneStore = false;
     uint2* sm;  // entry i at sm[32 * i]
     uint2 (&a)[kStackSlots];
     __device__ __forceinline__ uint2 load(int i) const { return i < N ? sm[32 * i] : a[i]; }

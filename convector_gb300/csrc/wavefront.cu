@@ -528,12 +528,8 @@ constexpr int kRefillWaveBlocksPerSm = 7;
 // from 82-94 to 112-120 bytes. Records instead of pairs, 16 mixed requests: 159
 // -> 149 ms (three and four per round 147, 153).
 constexpr int kRefillWaveSteps = 2;
-// As the frame kernel: waves whose trees are deeper than 40 levels keep the
-// first 16 stack entries of each lane in shared memory and read the tables
-// from global memory (4 tube views of 1280x736, 2 samples: 21.5 -> 20.3 ms;
-// 12 entries 20.5 ms).
-constexpr int kDeepWaveStackShared = 16;
-// And their lanes wait for 12 to shade, and a warp's leaves are tested together
+// DEEP: a wave with a tree deeper than 40 levels: lanes wait for 12 to shade, and a
+// warp's leaves are tested together
 // (16 mixed requests 148.8 -> 139.8 ms; 144.1 with 8 lanes).
 template <bool DEEP, bool SLOTS = false>
 __global__ void __launch_bounds__(128, kRefillWaveBlocksPerSm) k_wave_refill(const Job* __restrict__ jobs,
@@ -541,16 +537,11 @@ __global__ void __launch_bounds__(128, kRefillWaveBlocksPerSm) k_wave_refill(con
                                                                           const DeviceScene* __restrict__ scenes,
                                                                           WaveOutputs out) {
     WavePaths<SLOTS> P{jobs, scenes, out, hdr->n_jobs, hdr->n_groups, 0u, 0u};
+    __shared__ ApproxTables tab;
+    load_tables_wf(tab);
     bool ok;
-    if constexpr (DEEP) {
-        __shared__ uint2 sstack[4][kDeepWaveStackShared][32];
-        ok = path_refill<12, kRefillWaveSteps, false, true, kDeepWaveStackShared, true>(
-            P, g_tables_wf, &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
-    } else {
-        __shared__ ApproxTables tab;
-        load_tables_wf(tab);
-        ok = path_refill<16, kRefillWaveSteps, false, true>(P, tab);
-    }
+    if constexpr (DEEP) ok = path_refill<12, kRefillWaveSteps, false, true, true>(P, tab);
+    else ok = path_refill<16, kRefillWaveSteps, false, true>(P, tab);
     if (!ok) atomicOr(out.err, kErrStackOverflow);
 }
 

@@ -163,7 +163,7 @@ int32_t cvx_scene_set_light_pick(cvx_scene* scene, uint32_t light_pick);
 int32_t cvx_scene_set_query_launch(cvx_scene* scene, uint32_t blocks_per_sm);
 /* Stack depth of this scene's single-ray nearest-hit queries at the default
  * launch shape: how many of each lane's traversal stack entries are kept in
- * shared memory (0, 4, 8 or 12; default 8), the deeper ones in local memory.
+ * shared memory (0, 4, 8 or 12; 0 if never set), the deeper ones in local memory.
  * Shared entries never miss a cache, but take shared memory from L1; the
  * best depth depends on the tree (convector_gb300.autotune.tune_query times
  * them). Results do not depend on it. No counterpart in the reference, whose
