@@ -47,15 +47,15 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
 // warps of neighbouring camera rays together, and start a frame that does not
 // fill the GPU sooner. Measured, octet against refill, us per frame:
 //                            320x184    640x368    900x516     1280x736    1920x1080
-//   tube, 70 levels         1018/964  1446/1255  2099/1508   3506/2216   6909/4062
-//   icosphere, 28 levels     248/280    450/418    747/610   1365/1018   2834/1991
-//   room, 19 levels          152/187    219/242    340/301     623/481    1287/932
-//   open scene, 21 levels    124/152    152/187    198/230     286/312     528/543
-//   open scene, 16 levels      73/91     88/109    102/131     127/153     191/240
-// (480x276: icosphere 331/345.) The open scene of 21 levels loses 3-9 % by the
-// line at 18 levels, a closed room gains 13-40 %; nothing in the tree tells them
+//   tube, 70 levels         1002/790  1409/1056  2065/1286   3492/1921   6866/3446
+//   icosphere, 28 levels     243/259    448/398    748/590   1372/991    2869/1920
+//   room, 19 levels          144/174    217/239    360/302    659/485    1335/937
+//   open scene, 21 levels    117/137    144/179    192/219    280/306     528/535
+//   open scene, 16 levels     68/85      87/105     97/122    124/150     185/228
+// (480x276: icosphere 324/335.) The open scene of 21 levels loses 1-14 % by the
+// line at 18 levels, a closed room gains 16-30 %; nothing in the tree tells them
 // apart. For a wave, whether at least half of its groups belong to scenes of
-// kRefillMinDepth levels (32 open scenes of 11 to 20 levels, 6.4/7.9 ms).
+// kRefillMinDepth levels (32 open scenes of 11 to 20 levels, 6.1/7.7 ms).
 constexpr uint32_t kRefillMinDepth = 25;
 inline bool path_refill_frames(uint32_t refill_mode, uint32_t depth, uint64_t pixels) {
     if (refill_mode != CVX_REFILL_AFTER_CAMERA) return refill_mode == CVX_REFILL_ALL;
