@@ -317,8 +317,9 @@ __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uin
 // 1340 us. 7 blocks per SM (72 registers; 8 blocks spill: 329, 676, 1355 us).
 // STEPS records per round: 1, 2, 3 -> 309, 311, 379 us (room), 650, 628, 716
 // (icosphere), 1210, 1279, 1543 (tube): 1 for trees deeper than 40 levels, else 2.
-// Waiting for two finished packets
-// before taking new ones 322, 701, 1312 us.
+// Waiting for two finished packets before taking new ones 322, 701, 1312 us. With a
+// round's second leaf tested at once and the stack in local memory: 290, 598, 1164
+// us; 5, 6, 8 blocks 288, 287, 307 us (room), 601, 594, 642 (icosphere).
 constexpr int kPacketBlocksPerSm = 7;
 template <int STEPS>
 __global__ void __launch_bounds__(128, kPacketBlocksPerSm) k_intersect_packets(SoaRays src,
