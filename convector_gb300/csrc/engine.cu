@@ -307,12 +307,14 @@ struct cvx_batch {
     ResolveItem* d_items = nullptr;
     uint32_t max_items = 0;
     cudaStream_t stream = nullptr;
+    cudaEvent_t cleared = nullptr;  // on `stream`, after the accumulator's clear
     ~cvx_batch() {
         cudaFree(d_accum);
         cudaFree(d_rgba);
         cudaFree(d_items);
         if (stream) cudaStreamDestroy(stream);
         if (stream2) cudaStreamDestroy(stream2);
+        if (cleared) cudaEventDestroy(cleared);
     }
 };
 
@@ -335,6 +337,7 @@ extern "C" int32_t cvx_batch_create(cvx_scene* const* scenes, uint32_t n_scenes,
     b->max_pixels = max_pixels;
     ECK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     ECK(cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking), "cudaStreamCreate");
+    ECK(cudaEventCreateWithFlags(&b->cleared, cudaEventDisableTiming), "cudaEventCreate");
     st = b->engine.init(max_groups, 4096, c.traversal == CVX_TRAVERSE_PACKET, c.use_graph != 0,
                                 c.blocks_per_sm, c.refill_mode);
     if (st) return st;
@@ -376,7 +379,10 @@ extern "C" int32_t cvx_batch_render(cvx_batch* b, const cvx_view* views, uint32_
     }
     if (total > b->max_pixels) return set_error(CVX_ERR_CAPACITY, "views exceed the batch framebuffer");
     StreamSync sync(b->stream, b->stream2);
+    // The fused waves, on the other stream, add to the accumulator: they wait for its clear.
     ECK(cudaMemsetAsync(b->d_accum, 0, total * 12, b->stream), "clear accumulator");
+    ECK(cudaEventRecord(b->cleared, b->stream), "event");
+    ECK(cudaStreamWaitEvent(b->stream2, b->cleared, 0), "wait for the clear");
     uint64_t rays = 0;
     float ms = 0.0f;
     bool touched = rgba == nullptr;  // the images' pages, while the first wave runs

@@ -34,3 +34,20 @@ def test_batch_samples_equal_alone(gpu, traversal, refill, mixed, graph):
                 total += r.stats()[0]
             assert (img == r.resolve_u8(v.spp)).all()
         assert rays == total
+
+
+def test_fused_views_behind_a_large_clear(gpu):
+    """Fused views whose pixels lie behind many of wavefront views (cleared last), rendered twice into one
+    batch's accumulator: each image equals the view's alone."""
+    scs = [gpu.Scene(gpu.Bvh.build(scenes.spheres_and_boxes(n, 7, obj=False)[0])) for n in (500, 1500)]
+    cam = scenes.default_camera(gpu.Camera(), eye=(0.1, 1.2, 1.6))
+    views = [gpu.View(0, 4096, 4096, 1, 3, cam)] + [gpu.View(1, 64, 48, 2, 5 + i, cam) for i in range(3)]
+    batch = gpu.Batch(scs, max_groups=1 << 22, max_pixels=(1 << 24) + 3 * 64 * 48, mode=gpu.MODE_MEGAKERNEL)
+    gpu.lib().cvx_batch_set_scene_mode(batch._h, 0, 1)
+    for _ in range(2):
+        imgs = batch.render(views)[0]
+        for v, img in zip(views[1:], imgs[1:]):
+            r = gpu.Renderer(scs[1], v.width, v.height, rng_order=gpu.RNG_GROUP, traversal=gpu.TRAVERSE_SINGLE)
+            r.set_camera(v.camera)
+            r.accumulate_frames_f32(v.frame_base, v.spp)
+            assert (img == r.resolve_u8(v.spp)).all()
