@@ -25,6 +25,10 @@ bool injected_allocation_failure();
 // 1 us where they are in use), and the CPU can do it while the kernels run.
 void touch_pages(void* p, size_t bytes);
 
+// Whether a kernel may access a caller's array of 32-bit values in place: copies
+// take any address, a device's loads and stores only multiples of the size.
+inline bool word_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0u; }
+
 // A node of the interim tree of the device BVH build (bvh.rs:52-62): its
 // exact bounding box, its triangles order[beg .. beg + cnt) and its children
 // (c0 == 0: a leaf; node 0 is the root and never a child).

@@ -280,8 +280,8 @@ int32_t cvx_display_frame(cvx_display* d, const uint32_t* rgba, const uint32_t* 
     CVX_ON_DEVICE(d->device);
     cvx::StreamSync sync(d->stream);
     uint32_t npx = d->w * d->h;
-    // In place where the device shares the host's page tables (and the output
-    // does not lie over the inputs): the first kernel reads the frame and the
+    // In place where the device shares the host's page tables (and the arrays are
+    // aligned, and the output does not lie over the inputs): the first kernel reads the frame and the
     // gbuffer, the second writes the output over the CPU-GPU link, and the output's
     // pages are touched meanwhile. 1280x736: 160 us with copies and separate blend
     // and median passes, 101 us so (reading the inputs takes 38, writing the output
@@ -290,7 +290,8 @@ int32_t cvx_display_frame(cvx_display* d, const uint32_t* rgba, const uint32_t* 
         const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b, len = (uintptr_t)npx * 4u;
         return x < y + len && y < x + len;
     };
-    const bool in_place = d->host_page_tables && !overlap(out_srgb, rgba) && !overlap(out_srgb, gbuffer);
+    const bool in_place = d->host_page_tables && cvx::word_aligned(rgba) && cvx::word_aligned(gbuffer) &&
+                          cvx::word_aligned(out_srgb) && !overlap(out_srgb, rgba) && !overlap(out_srgb, gbuffer);
     const uint32_t *frame = rgba, *gbuf = gbuffer;
     if (!in_place) {
         PCK(cudaMemcpyAsync(d->d_frame, rgba, (size_t)npx * 4, cudaMemcpyHostToDevice, d->stream), "upload frame");
