@@ -506,12 +506,13 @@ int32_t cvx_intersect_nearest(cvx_scene* s, const float* ox, const float* oy, co
     // ahead), so the transfer overlaps traversal and no ray copy is made.
     bool in_place = s->reads_host_in_place();
     for (const float* c : {ox, oy, oz, dx, dy, dz}) in_place = in_place && word_aligned(c);
-    // (A caller may let its hits overwrite its rays: then they are copied out.)
+    // (A caller may let its hits overwrite its rays, or pass one array for both and
+    // get the indices: then they are copied out, in that order.)
     auto overlap = [n](const void* a, const void* b) {
         const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b, len = (uintptr_t)n * 4u;
         return x < y + len && y < x + len;
     };
-    bool apart = word_aligned(t_out) && word_aligned(tri_out);
+    bool apart = word_aligned(t_out) && word_aligned(tri_out) && !overlap(t_out, tri_out);
     for (const float* c : {ox, oy, oz, dx, dy, dz}) apart = apart && !overlap(c, t_out) && !overlap(c, tri_out);
     if (in_place && apart && n <= kDirectHostRays) return intersect_direct(s, ox, oy, oz, dx, dy, dz, n, far_dist, traversal, t_out, tri_out);
     if (s->scratch_n < n || (!in_place && !s->d_rays)) {

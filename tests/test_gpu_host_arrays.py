@@ -48,6 +48,24 @@ def test_unaligned_query_arrays(gpu, scene, n, traversal, which):
     assert (np.array(out_tri) == tri).all() and _same(np.array(out_t), t)
 
 
+@pytest.mark.parametrize("traversal", [0, 1])
+@pytest.mark.parametrize("shift", [0, 1, -7])
+def test_query_outputs_over_one_another(gpu, scene, traversal, shift):
+    """One buffer for distances and indices, exactly or shifted: the indices are written last."""
+    n = 3001
+    o, d = scenes.random_rays(n, seed=4)
+    t, tri = scene.intersect_nearest(o, d, traversal=traversal)
+    cols = [np.ascontiguousarray(a[:, k]) for a in (o, d) for k in range(3)]
+    buf = np.zeros(n + 7, np.uint32)
+    at = max(-shift, 0)
+    want = buf.copy()
+    want[at:at + n] = t.view(np.uint32)
+    want[at + shift:at + shift + n] = tri.view(np.uint32)
+    gpu._check(gpu.lib().cvx_intersect_nearest(scene._h, *[gpu._ptr(c) for c in cols], n, 1.0e5, traversal,
+                                               gpu._ptr(buf[at:]), gpu._ptr(buf[at + shift:])))
+    assert (buf == want).all()
+
+
 @pytest.mark.parametrize("w,h", [(1, 1), (33, 9), (31, 7), (64, 16), (65, 17)])
 @pytest.mark.parametrize("form", ["aligned", "inputs unaligned", "output unaligned", "output over the frame",
                                   "output over the gbuffer"])
