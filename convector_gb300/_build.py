@@ -26,7 +26,8 @@ CU_SOURCES = ["kernels.cu", "wavefront.cu", "engine.cu", "capi.cu", "noalloc.cu"
 CPP_SOURCES = ["host_scene.cpp"]
 HEADERS = ["x86sem.cuh", "layout.cuh", "traverse.cuh", "shade.cuh", "path_refill.cuh", "packet_refill.cuh", "packet_warp.cuh",
            "kernels.h", "internal.h",
-           "x86_approx_tables.h", "wavefront.cuh", "engine.h", "device_guard.cuh"]
+           "x86_approx_tables.h", "wavefront.cuh", "engine.h", "device_guard.cuh",
+           "limits.h", "scene_tree.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_103a,code=sm_103a",

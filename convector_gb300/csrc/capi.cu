@@ -16,6 +16,7 @@
 #include "engine.h"
 #include "internal.h"
 #include "kernels.h"
+#include "scene_tree.h"
 #include "x86_approx_tables.h"
 
 using namespace cvx;
@@ -222,31 +223,6 @@ struct cvx_renderer {
     }
 };
 
-// Checks the tree and returns its depth (roots at depth 1).
-static int32_t validate_tree(const cvx_bvh_node* nodes, uint32_t n_nodes, uint32_t n_tris, uint32_t* depth_out) {
-    if (n_nodes < 2 || (n_nodes & 1u)) return set_error(CVX_ERR_INVALID, "node count must be even and at least 2");
-    std::vector<std::pair<uint32_t, uint32_t>> stack{{0u, 1u}, {1u, 1u}};
-    uint32_t depth = 0;
-    size_t visited = 0;
-    while (!stack.empty()) {
-        auto [i, dep] = stack.back();
-        stack.pop_back();
-        if (++visited > n_nodes) return set_error(CVX_ERR_INVALID, "BVH nodes form a cycle");
-        depth = dep > depth ? dep : depth;
-        const cvx_bvh_node& nd = nodes[i];
-        if (nd.len == 0) {
-            if ((nd.index & 1u) || nd.index + 1 >= n_nodes || nd.index < 2)
-                return set_error(CVX_ERR_INVALID, "internal node child index out of range");
-            stack.push_back({nd.index, dep + 1});
-            stack.push_back({nd.index + 1, dep + 1});
-        } else if ((uint64_t)nd.index + nd.len > n_tris) {
-            return set_error(CVX_ERR_INVALID, "leaf triangle range out of range");
-        }
-    }
-    *depth_out = depth;
-    return CVX_OK;
-}
-
 extern "C" {
 
 int32_t cvx_device_info(int32_t* ordinal, char* name, size_t name_len) {
@@ -289,9 +265,9 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     if (!tris || !nodes || !out || n_tris == 0) return set_error(CVX_ERR_INVALID, "null argument or empty scene");
     if (n_tris >= (1u << 27) || n_nodes >= (1u << 27))
         return set_error(CVX_ERR_INVALID, "scenes are limited to 2^27 triangles and 2^27 nodes");
-    uint32_t depth = 0;
-    int32_t st = validate_tree(nodes, n_nodes, n_tris, &depth);
-    if (st) return st;
+    TreeFacts tree;
+    if (const char* wrong = check_tree(nodes, n_nodes, n_tris, &tree)) return set_error(CVX_ERR_INVALID, wrong);
+    const uint32_t depth = tree.depth;
     if (depth + 2 > (uint32_t)kStackDepth)
         return set_error(CVX_ERR_INVALID, "BVH deeper than the device traversal stack (" +
                                               std::to_string(depth) + " levels)");
@@ -302,7 +278,7 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
         if ((tris[i].material >> 30) & 1u) ds.push_back(i);  // scene.rs:117-122
     }
     int dev = 0;
-    st = ensure_device(&dev);
+    int32_t st = ensure_device(&dev);
     if (st) return st;
     std::unique_ptr<cvx_scene> s(new cvx_scene());
     s->device = dev;
@@ -324,34 +300,14 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     if ((st = dalloc(&s->d_shade, n_tris, "shading data"))) return st;
     if ((st = dalloc(&s->d_lights, (size_t)s->n_lights * 5, "lights"))) return st;
     if ((st = dalloc(&s->d_err, 2, "status"))) return st;  // [0] status, [1] ray counter
-    // The select-form slab test (box_test_sel) needs every bound at most
-    // kSelectMax in magnitude and ordered, and none -0.
-    s->slab_sel = true;
-    for (uint32_t i = 0; i < n_nodes && s->slab_sel; i++)
-        for (int c = 0; c < 3; c++) {
-            const float lo = nodes[i].origin[c], hi = nodes[i].far_[c];
-            if (!(std::fabs(lo) <= 1.0e18f) || !(std::fabs(hi) <= 1.0e18f) || !(lo <= hi) || (lo == 0.0f && std::signbit(lo)) ||
-                (hi == 0.0f && std::signbit(hi)))
-                s->slab_sel = false;
-        }
-    // The wide records need every node's bounds to be exactly the enclosure of
-    // its children's, as the build makes them.
-    bool tight = s->slab_sel;
-    for (uint32_t i = 0; i < n_nodes && tight; i++) {
-        if (nodes[i].len != 0) continue;
-        const cvx_bvh_node &c0 = nodes[nodes[i].index], &c1 = nodes[nodes[i].index + 1];
-        for (int c = 0; c < 3; c++)
-            if (std::min(c0.origin[c], c1.origin[c]) != nodes[i].origin[c] ||
-                std::max(c0.far_[c], c1.far_[c]) != nodes[i].far_[c])
-                tight = false;
-    }
+    s->slab_sel = tree.select;
     // Node pairs: q0 = lo0 hi0.x | q1 = hi0.yz lo1.xy | q2 = lo1.z hi1 | q3 = index/len x2
     // q3 holds the two children's stack references, the form the traversal
     // pushes (traverse.cuh): (index << 5) | len for internal nodes (len 0, index =
     // first child) and leaves of up to 30 triangles; (slot << 5) | 31 for larger
     // leaves, whose (index, len) is escape slot `slot`, the float4 at
     // nodes[-1 - slot] below the pairs (the region is padded to 8 float4, so the
-    // pairs keep their 128-byte alignment).
+    // pairs keep their 128-byte alignment). Pairs that are not reached stay zero.
     std::vector<uint2> esc;
     auto child_ref = [&esc](const cvx_bvh_node& nd) -> uint32_t {
         if (nd.len < 31u) return (nd.index << 5) | nd.len;
@@ -360,6 +316,7 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     };
     std::vector<float4> pairs((size_t)n_nodes / 2 * 4);
     for (uint32_t p = 0; p < n_nodes / 2; p++) {
+        if (!tree.reached(p)) continue;
         const cvx_bvh_node& a = nodes[2 * p];
         const cvx_bvh_node& b = nodes[2 * p + 1];
         float4* q = &pairs[4 * (size_t)p];
@@ -380,7 +337,7 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     CK(cudaMemcpyAsync(s->d_nodes, node_buf.data(), node_buf.size() * sizeof(float4), cudaMemcpyHostToDevice,
                        s->stream),
        "upload nodes");
-    if (tight && depth <= kWideMaxDepth && n_nodes / 2 <= (1u << 25)) {  // 32-bit offsets into the records
+    if (tree.wide) {
         if ((st = dalloc(&s->d_wide, (size_t)n_nodes / 2 * 8, "wide nodes"))) return st;
         CK(launch_prep_wide(s->d_nodes + s->node_offset, n_nodes / 2, s->d_wide, s->stream), "wide nodes");
     }

@@ -18,6 +18,8 @@
 #pragma once
 #include <cstdint>
 
+#include "limits.h"
+
 namespace cvx {
 
 struct TriShade {
@@ -34,12 +36,9 @@ struct DeviceScene {
     uint32_t n_nodes, n_tris, n_lights;
     uint32_t general_pick;  // 1: (bits * n) >> 32; 0: bits >> 29 (needs n == 8)
     uint32_t depth;         // BVH depth (launch choices only)
-    // Every node bound is finite, lo <= hi on each axis and none is -0: the
-    // ray-cast kernel may take the select-form slab test (box_test_sel).
-    uint32_t slab_sel;
-    // The wide records of the node pairs (traverse.cuh), for the select form;
-    // null unless slab_sel, every node's bounds lie inside its parent's (true of
-    // every built tree) and the tree is at most kWideMaxDepth levels deep.
+    uint32_t slab_sel;  // TreeFacts::select
+    // The wide records of the node pairs (traverse.cuh), for the select form; null
+    // where the tree does not allow them (TreeFacts::wide).
     const float4* wide;
 };
 
@@ -48,9 +47,6 @@ struct DeviceCamera {
 };
 
 constexpr uint32_t kSkyMaterial = 0xC0000000u;  // material.rs:85-90
-constexpr int kStackDepth = 128;  // >= BVH depth + 2 (checked at scene creation)
-// Up to three boxes of a wide record wait on the stack: at most 1.5 per level.
-constexpr uint32_t kWideMaxDepth = (kStackDepth - 8) / 3 * 2;
 
 // Error bits a kernel reports through its status word instead of trapping.
 constexpr uint32_t kErrStackOverflow = 1u;

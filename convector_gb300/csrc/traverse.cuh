@@ -216,7 +216,6 @@ struct WideT {
 // Rays that may take the select form: reciprocals and origin as above, and
 // bounded (with the bounds, DeviceScene::slab_sel), so that no plane distance
 // overflows.
-constexpr float kSelectMax = 1.0e18f;
 __device__ __forceinline__ bool select_form_ray(F3 o, F3 inv) {
     auto in = [](float x) { return fabsf(x) >= 0.75f && fabsf(x) <= kSelectMax; };
     return in(inv.x) && in(inv.y) && in(inv.z) && fabsf(o.x) <= kSelectMax && fabsf(o.y) <= kSelectMax &&
