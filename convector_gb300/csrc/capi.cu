@@ -337,10 +337,6 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     CK(cudaMemcpyAsync(s->d_nodes, node_buf.data(), node_buf.size() * sizeof(float4), cudaMemcpyHostToDevice,
                        s->stream),
        "upload nodes");
-    if (tree.wide) {
-        if ((st = dalloc(&s->d_wide, (size_t)n_nodes / 2 * 8, "wide nodes"))) return st;
-        CK(launch_prep_wide(s->d_nodes + s->node_offset, n_nodes / 2, s->d_wide, s->stream), "wide nodes");
-    }
     cvx_triangle* d_src = nullptr;
     uint32_t* d_ds = nullptr;
     if ((st = dalloc(&d_src, n_tris, "staging"))) return st;
@@ -358,6 +354,12 @@ int32_t cvx_scene_create(const cvx_triangle* tris, uint32_t n_tris, const cvx_bv
     cudaFree(d_src);
     cudaFree(d_ds);
     if (e != cudaSuccess) return cuda_fail(e, "scene upload");
+    // The wide records, if the device has room for them: without them every
+    // kernel walks the pairs.
+    if (tree.wide && !dalloc(&s->d_wide, (size_t)n_nodes / 2 * 8, "wide nodes")) {
+        CK(launch_prep_wide(s->d_nodes + s->node_offset, n_nodes / 2, s->d_wide, s->stream), "wide nodes");
+        CK(cudaStreamSynchronize(s->stream), "wide nodes");
+    }
     *out = s.release();
     return CVX_OK;
 }

@@ -38,7 +38,7 @@ struct DeviceScene {
     uint32_t depth;         // BVH depth (launch choices only)
     uint32_t slab_sel;  // TreeFacts::select
     // The wide records of the node pairs (traverse.cuh), for the select form; null
-    // where the tree does not allow them (TreeFacts::wide).
+    // where the tree does not allow them (TreeFacts::wide) or the device had no room.
     const float4* wide;
 };
 
