@@ -103,9 +103,19 @@ bool cvx::injected_allocation_failure() {
 
 void cvx::touch_pages(void* p, size_t bytes) {
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    volatile char* c = static_cast<char*>(p);
-    for (size_t i = 0; i < bytes; i += page) c[i] = 0;
-    if (bytes) c[bytes - 1] = 0;
+    if (bytes == 0) return;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) cudaGetLastError();
+    else if (a.type != cudaMemoryTypeUnregistered) return;
+    unsigned char* const c = static_cast<unsigned char*>(p);
+    // A byte exchanged for itself: a write access that changes nothing, even
+    // where another thread writes the same byte meanwhile.
+    auto touch = [](unsigned char* at) {
+        unsigned char v = __atomic_load_n(at, __ATOMIC_RELAXED);
+        __atomic_compare_exchange_n(at, &v, v, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED);
+    };
+    for (size_t i = 0; i < bytes; i += page) touch(c + i);
+    touch(c + bytes - 1);
 }
 
 struct cvx_scene {

@@ -816,8 +816,14 @@ struct cvx_server {
                     continue;
                 }
                 cudaEventRecord(fl[e].done, stream_of(e));
-                for (auto& q : start[e])  // the pages of the images this wave completes, while it runs
-                    if (q->host_rgba && q->next_sample + q->wave_k == q->r.spp) touch_pages(q->host_rgba, q->npx * 4);
+                for (auto& q : start[e]) {  // the pages of the images this wave completes, while it runs
+                    bool wanted = q->host_rgba && q->next_sample + q->wave_k == q->r.spp;
+                    if (wanted) {
+                        std::lock_guard<std::mutex> lk(mu);
+                        wanted = !q->cancelled;
+                    }
+                    if (wanted) touch_pages(q->host_rgba, q->npx * 4);
+                }
                 fl[e].busy = true;
                 fl[e].reqs = std::move(start[e]);
                 if (n_busy++ == 0) busy_from = now();

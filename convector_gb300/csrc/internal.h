@@ -18,8 +18,9 @@ int32_t set_error(int32_t status, const std::string& msg);
 // allocation is to fail as if the device were out of memory.
 bool injected_allocation_failure();
 
-// Writes a zero to every page of an output buffer that is about to be filled
-// whole. Pages the process has not used yet (a fresh large allocation) cost the
+// Makes the pages of an output buffer present, whose contents stay as they are
+// (the call that is to fill it may yet fail); buffers that CUDA allocated or
+// registered need none of it. Pages the process has not used yet (a fresh large allocation) cost the
 // driver's copies and the device's stores several times what they cost the CPU
 // (3.8 MB on 64 KB pages: copy 29 us touched, 361 us fresh; touching 156 us, or
 // 1 us where they are in use), and the CPU can do it while the kernels run.
