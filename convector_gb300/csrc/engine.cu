@@ -808,6 +808,7 @@ struct cvx_server {
                                 start[e].push_back(q);
                             }
             }
+            bool started[kMaxEngines] = {};
             for (int e = 0; e <= n_wf; e++) {
                 if (start[e].empty()) continue;
                 int32_t st = submit_wave(e, start[e]);
@@ -816,7 +817,17 @@ struct cvx_server {
                     continue;
                 }
                 cudaEventRecord(fl[e].done, stream_of(e));
-                for (auto& q : start[e]) {  // the pages of the images this wave completes, while it runs
+                fl[e].busy = true;
+                fl[e].reqs = std::move(start[e]);
+                started[e] = true;
+                if (n_busy++ == 0) busy_from = now();
+            }
+            if (n_busy == 0) continue;
+            // The pages of the images that the new waves complete, while they run: after
+            // every engine has its wave, which fresh pages (150 us per 3.8 MB) would delay.
+            for (int e = 0; e <= n_wf; e++) {
+                if (!started[e]) continue;
+                for (auto& q : fl[e].reqs) {
                     bool wanted = q->host_rgba && q->next_sample + q->wave_k == q->r.spp;
                     if (wanted) {
                         std::lock_guard<std::mutex> lk(mu);
@@ -824,11 +835,7 @@ struct cvx_server {
                     }
                     if (wanted) touch_pages(q->host_rgba, q->npx * 4);
                 }
-                fl[e].busy = true;
-                fl[e].reqs = std::move(start[e]);
-                if (n_busy++ == 0) busy_from = now();
             }
-            if (n_busy == 0) continue;
             // Wait for an engine to finish, or for new work an idle engine could take.
             for (;;) {
                 bool ready = false;
