@@ -414,7 +414,8 @@ class Scene:
         return Scene(Bvh.from_meshes(meshes), light_pick=light_pick)
 
     def set_query_launch(self, blocks_per_sm):
-        """Resident blocks per SM of the nearest-hit kernel (0: default)."""
+        """Resident blocks per SM of the nearest-hit kernel (0: default, with
+        kernels of their own for queries of up to 262,144 rays)."""
         _check(lib().cvx_scene_set_query_launch(self._h, blocks_per_sm))
 
     def set_query_stack(self, shared_entries):

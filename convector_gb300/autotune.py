@@ -129,9 +129,11 @@ def autotuned_renderer(scene, width, height, rng_order=RNG_GROUP, allow_packet=T
     return Renderer(scene, width, height, **best)
 
 
-# (name, traversal, blocks per SM, shared stack entries) of the query candidates
-QUERY_SHAPES = [("packet8/0", TRAVERSE_PACKET, 0, 8)] + [
-    ("single/%d%s" % (bps, "" if st == 8 else "/s%d" % st), TRAVERSE_SINGLE, bps, st)
+# (name, traversal, blocks per SM, shared stack entries) of the query candidates.
+# 8 blocks per SM are the default shape: left unset (0), so that small queries
+# of the tuned scene keep their own kernels.
+QUERY_SHAPES = [("packet8/0", TRAVERSE_PACKET, 0, 0)] + [
+    ("single/%d%s" % (bps, "" if st == 8 else "/s%d" % st), TRAVERSE_SINGLE, bps if bps != 8 else 0, st)
     for bps, st in ((8, 8), (8, 0), (8, 4), (8, 12), (10, 8), (12, 8))]
 
 

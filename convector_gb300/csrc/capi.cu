@@ -432,13 +432,14 @@ int32_t cvx_intersect_nearest_device(cvx_scene* s, const float* rays, uint32_t n
 
 // The whole call of a small host query in one launch: the kernel reads the
 // caller's rays and writes the caller's hits and a page-locked status word over
-// the CPU-GPU link. Two pageable copies, a copied status and the waits for three
+// the CPU-GPU link (queries that direct_query allows). Two pageable copies, a copied status and the waits for three
 // streams were half of such a call (1 ray: 63 -> 28 us, 1021 rays of the
 // icosphere in packets 131 -> 78 us with the kernel's own gain, 65,536 rays 343 ->
 // 261 us). From about 200,000 rays on the copies win (262,144 rays, single, of the
 // icosphere 887 and 842 us; 524,288: 1721 and 1774).
 constexpr uint32_t kQueryChunks = 4;  // of the pipeline below, each with a status word
 constexpr uint32_t kDirectHostRays = 131072;
+static_assert(kDirectHostRays <= kDirectRays, "intersect_direct launches the direct kernels");
 static int32_t intersect_direct(cvx_scene* s, const float* ox, const float* oy, const float* oz, const float* dx,
                                 const float* dy, const float* dz, uint32_t n, float far_dist, uint32_t traversal,
                                 float* t_out, int32_t* tri_out) {
@@ -452,7 +453,7 @@ static int32_t intersect_direct(cvx_scene* s, const float* ox, const float* oy, 
     const RayCols cols{{ox, oy, oz, dx, dy, dz}};
     StreamSync sync(q);
     CK(launch_intersect(s->view(), cols, n, far_dist, traversal == CVX_TRAVERSE_PACKET, t_out, tri_out, nullptr,
-                        s->h_qerr, 0, s->blocks_per_sm, q, s->query_stack),
+                        s->h_qerr, 0, 0, q),
        "intersect launch");
     CK(cudaStreamSynchronize(q), "intersect");
     if (*reinterpret_cast<volatile uint32_t*>(s->h_qerr))
@@ -483,7 +484,8 @@ int32_t cvx_intersect_nearest(cvx_scene* s, const float* ox, const float* oy, co
     };
     bool apart = word_aligned(t_out) && word_aligned(tri_out) && !overlap(t_out, tri_out);
     for (const float* c : {ox, oy, oz, dx, dy, dz}) apart = apart && !overlap(c, t_out) && !overlap(c, tri_out);
-    if (in_place && apart && n <= kDirectHostRays) return intersect_direct(s, ox, oy, oz, dx, dy, dz, n, far_dist, traversal, t_out, tri_out);
+    if (in_place && apart && n <= kDirectHostRays && direct_query(n, s->blocks_per_sm))
+        return intersect_direct(s, ox, oy, oz, dx, dy, dz, n, far_dist, traversal, t_out, tri_out);
     if (s->scratch_n < n || (!in_place && !s->d_rays)) {
         cudaFree(s->d_rays);
         cudaFree(s->d_t);

@@ -342,7 +342,6 @@ __global__ void __launch_bounds__(128, kPacketBlocksPerSm) k_intersect_packets(S
 // 198; 70-level tube 241 -> 163, 421 -> 255, 640 -> 497, 839 -> 787; single rays,
 // room 52 -> 42, 68 -> 51, 91 -> 70, 112 -> 102, tube 234 -> 186, 218 -> 165, 312
 // -> 287, 419 -> 470. `err` may be page-locked host memory (it is stored to).
-constexpr uint32_t kDirectRays = 262144;
 __global__ void __launch_bounds__(64) k_intersect_warp(DeviceScene s, const RayCols rays, uint32_t n, float far_dist,
                                                        float* __restrict__ t_out, int32_t* __restrict__ tri_out,
                                                        uint32_t* err) {
@@ -1024,9 +1023,8 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
                              float* t_out, int32_t* tri_out, uint32_t* counters, uint32_t* err, uint32_t block,
                              uint32_t blocks_per_sm, cudaStream_t st, uint32_t shared_stack) {
     // Calls that do not fill the GPU several times over: one packet per warp, or
-    // one ray per lane, with nothing claimed (kDirectRays).
-    if (!counters && n <= kDirectRays && blocks_per_sm == 0 &&
-        (shared_stack == kQueryStackDefault || shared_stack == kQueryStackShared)) {
+    // one ray per lane, with nothing claimed.
+    if (!counters && direct_query(n, blocks_per_sm)) {
         if (packet) k_intersect_warp<<<(n + 15u) / 16u, 64, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
         else k_intersect_lanes<<<(n + 31u) / 32u, 32, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
         return cudaGetLastError();

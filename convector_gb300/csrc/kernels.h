@@ -32,10 +32,17 @@ inline RayCols soa_cols(const float* rays, uint32_t n) {  // one (6, n) device a
     return r;
 }
 
+// Whether a query takes the direct kernels (one packet per warp, one ray per lane):
+// up to kDirectRays rays, unless a launch shape of the persistent kernels is set
+// (times at k_intersect_warp). They store to `err`, which may then be page-locked
+// host memory, and use no counter behind it; the persistent kernels claim from
+// err[1], which must be device memory. They have no stack in shared memory.
+constexpr uint32_t kDirectRays = 262144;
+inline bool direct_query(uint32_t n, uint32_t blocks_per_sm) { return n <= kDirectRays && blocks_per_sm == 0; }
 // shared_stack: stack entries of each lane kept in shared memory by the
-// select-form single-ray kernel at 8 blocks per SM (0, 4, 8 or 12; not chosen: 0;
-// other launch shapes keep 8).
-constexpr uint32_t kQueryStackDefault = ~0u;
+// persistent single-ray kernel at 8 blocks per SM (0, 4, 8 or 12; other launch
+// shapes keep 8).
+constexpr uint32_t kQueryStackDefault = 0;
 cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t n, float far_dist, bool packet,
                              float* t_out, int32_t* tri_out, uint32_t* counters, uint32_t* err, uint32_t block,
                              uint32_t blocks_per_sm, cudaStream_t st, uint32_t shared_stack = kQueryStackDefault);

@@ -159,10 +159,12 @@ uint32_t cvx_scene_num_direct_samples(const cvx_scene* scene);
 int32_t cvx_scene_set_light_pick(cvx_scene* scene, uint32_t light_pick);
 /* Launch shape of this scene's nearest-hit queries: resident 128-thread
  * blocks per SM (0: default 8; the single-ray kernel is built for 8, 10 and
- * 12, trading registers for occupancy). Results do not depend on it. */
+ * 12, trading registers for occupancy). While it is not set, queries of up to
+ * 262,144 rays run without resident blocks, one packet per warp or one ray per
+ * lane. Results do not depend on it. */
 int32_t cvx_scene_set_query_launch(cvx_scene* scene, uint32_t blocks_per_sm);
-/* Stack depth of this scene's single-ray nearest-hit queries at the default
- * launch shape: how many of each lane's traversal stack entries are kept in
+/* Stack depth of this scene's single-ray nearest-hit queries at 8 resident
+ * blocks per SM: how many of each lane's traversal stack entries are kept in
  * shared memory (0, 4, 8 or 12; 0 if never set), the deeper ones in local memory.
  * Shared entries never miss a cache, but take shared memory from L1; the
  * best depth depends on the tree (convector_gb300.autotune.tune_query times
