@@ -108,9 +108,11 @@ struct PacketRay {
         const float c0 = b0.mask ? b0.tmin : inf, c1 = b1.mask ? b1.tmin : inf;
         // The reference pushes `first` then `second` and pops `second` first.
         const float t_first = first0 ? c0 : c1, t_second = first0 ? c1 : c0;
-        const bool kept = any(active & !geq(t_second, h.t));
+        // Either is culled when popped (aabb.rs:171-177), the first too if the second
+        // is not visited: then it is next at once.
+        const bool kept0 = any(active & !geq(t_first, h.t)), kept1 = any(active & !geq(t_second, h.t));
         if (!pair) return;
-        const bool v[2] = {first0 ? hit0 : hit1, (first0 ? hit1 : hit0) && kept};
+        const bool v[2] = {(first0 ? hit0 : hit1) && kept0, (first0 ? hit1 : hit0) && kept1};
         const uint32_t r[2] = {first0 ? r0 : r1, first0 ? r1 : r0};
         const float t[2] = {t_first, t_second};
         push<2>(v, r, t, stack, overflow);

@@ -54,3 +54,25 @@ def test_scene_without_room_for_the_wide_records(gpu, orc):
         t, tri = scene.intersect_nearest(o, d, traversal=traversal)
         ot, otri = osc.intersect(o, d, mode=traversal)
         assert (tri == otri).all() and (t.view(np.uint32) == ot.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("kind", ["loose", "tight, on box corners"])
+def test_packets_in_step_cull_either_child_of_a_pair(gpu, orc, kind):
+    """A million packet rays over the pairs: a scene with loose roots, and rays that start on box corners (whose
+    packets take pairs for the steps with tied zeros). A pair's first child is culled like its second."""
+    b = gpu.Bvh.build(scenes.spheres_and_boxes(3000, 5, obj=False)[0])
+    f = b.nodes.view(np.float32)
+    n = (1 << 20) + 5
+    o, d = scenes.random_rays(n, seed=n)
+    if kind == "loose":
+        f[0:2, 0:3] -= np.float32(0.5)
+        f[0:2, 3:6] += np.float32(0.5)
+    else:
+        k = np.random.default_rng(1).integers(0, f.shape[0], n // 8 + 1).repeat(8)[:n]
+        axis = np.random.default_rng(2).integers(0, 3, n)
+        o[np.arange(n), axis] = f[k, axis]
+    scene, osc = gpu.Scene(b), orc.OracleScene(b.triangles, b.nodes)
+    ot, otri = osc.intersect(o, d, mode=gpu.TRAVERSE_PACKET)
+    t, tri = scene.intersect_nearest(o, d, traversal=gpu.TRAVERSE_PACKET)
+    assert (tri == otri).all(), np.nonzero(tri != otri)[0][:10]
+    assert (t.view(np.uint32) == ot.view(np.uint32)).all()
