@@ -108,11 +108,15 @@ void cvx::touch_pages(void* p, size_t bytes) {
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) cudaGetLastError();
     else if (a.type != cudaMemoryTypeUnregistered) return;
     unsigned char* const c = static_cast<unsigned char*>(p);
-    // A byte exchanged for itself: a write access that changes nothing, even
-    // where another thread writes the same byte meanwhile.
+    // A byte exchanged for itself: a store that changes nothing, even where another
+    // thread writes the same byte meanwhile. A zero is tried first, as a fresh page
+    // holds: read first, it would take two faults (display frame of 1280x736 101 -> 107
+    // us). Pages in use need the store too (without it the copies into them are slow:
+    // 32 batched images, 53 MB, 7.3 -> 14.1 ms).
     auto touch = [](unsigned char* at) {
-        unsigned char v = __atomic_load_n(at, __ATOMIC_RELAXED);
-        __atomic_compare_exchange_n(at, &v, v, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED);
+        unsigned char v = 0;
+        if (!__atomic_compare_exchange_n(at, &v, (unsigned char)0, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED))
+            __atomic_compare_exchange_n(at, &v, v, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED);
     };
     for (size_t i = 0; i < bytes; i += page) touch(c + i);
     touch(c + bytes - 1);
