@@ -488,7 +488,8 @@ int32_t cvx_intersect_nearest(cvx_scene* s, const float* ox, const float* oy, co
     };
     bool apart = word_aligned(t_out) && word_aligned(tri_out) && !overlap(t_out, tri_out);
     for (const float* c : {ox, oy, oz, dx, dy, dz}) apart = apart && !overlap(c, t_out) && !overlap(c, tri_out);
-    if (in_place && apart && n <= kDirectHostRays && direct_query(n, s->blocks_per_sm))
+    if (in_place && apart && n <= kDirectHostRays &&
+        direct_query(s->view(), n, traversal == CVX_TRAVERSE_PACKET, s->blocks_per_sm))
         return intersect_direct(s, ox, oy, oz, dx, dy, dz, n, far_dist, traversal, t_out, tri_out);
     if (s->scratch_n < n || (!in_place && !s->d_rays)) {
         cudaFree(s->d_rays);

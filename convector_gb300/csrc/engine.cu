@@ -118,7 +118,11 @@ int32_t WaveEngine::set_scenes(cvx_scene* const* scenes, uint32_t n) {
     ECK(cudaMemcpy(d_scenes_, v.data(), n * sizeof(DeviceScene), cudaMemcpyHostToDevice), "upload scene table");
     n_scenes_ = n;
     scene_depth_.resize(n);
-    for (uint32_t i = 0; i < n; i++) scene_depth_[i] = v[i].depth;
+    scene_wide_.resize(n);
+    for (uint32_t i = 0; i < n; i++) {
+        scene_depth_[i] = v[i].depth;
+        scene_wide_[i] = v[i].wide != nullptr;
+    }
     return CVX_OK;
 }
 
@@ -126,28 +130,28 @@ static bool same_out(const WaveOutputs& a, const WaveOutputs& b) { return std::m
 
 static cudaError_t launch_any(bool fused, const Job* jobs, const WaveHeader* hdr, const DeviceScene* scenes,
                               const WaveState& st, const WaveOutputs& out, bool packet, uint32_t bps,
-                              uint32_t refill_from, bool deep, cudaStream_t stream) {
-    return fused ? launch_wave_fused(jobs, hdr, scenes, out, packet, bps, deep, stream)
+                              uint32_t refill_from, bool deep, bool wide, cudaStream_t stream) {
+    return fused ? launch_wave_fused(jobs, hdr, scenes, out, packet, bps, deep, wide, stream)
                  : launch_wave(jobs, hdr, scenes, st, out, packet, bps, refill_from, deep, stream);
 }
 
-// deep: a scene of this wave is deeper than 40 levels (the traversal's claim
-// threshold; captured graphs are kept per value).
-int32_t WaveEngine::launch(const WaveOutputs& out, bool deep, cudaStream_t stream) {
+// deep: a scene of this wave is deeper than 40 levels; wide: one has wide records
+// (which kernels run; captured graphs are kept per value).
+int32_t WaveEngine::launch(const WaveOutputs& out, bool deep, bool wide, cudaStream_t stream) {
     if (!use_graph_) {
-        ECK(launch_any(fused_, d_jobs_, d_hdr_, d_scenes_, st_, out, packet_, blocks_per_sm_, refill_from_, deep, stream),
+        ECK(launch_any(fused_, d_jobs_, d_hdr_, d_scenes_, st_, out, packet_, blocks_per_sm_, refill_from_, deep, wide, stream),
             "wave launch");
         return CVX_OK;
     }
     for (auto& g : graphs_)
-        if (same_out(g.out, out) && g.deep == deep) {
+        if (same_out(g.out, out) && g.deep == deep && g.wide == wide) {
             ECK(cudaGraphLaunch(g.exec, stream), "graph launch");
             return CVX_OK;
         }
     cudaGraph_t graph;
     ECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     cudaError_t e =
-        launch_any(fused_, d_jobs_, d_hdr_, d_scenes_, st_, out, packet_, blocks_per_sm_, refill_from_, deep, stream);
+        launch_any(fused_, d_jobs_, d_hdr_, d_scenes_, st_, out, packet_, blocks_per_sm_, refill_from_, deep, wide, stream);
     cudaError_t e2 = cudaStreamEndCapture(stream, &graph);
     if (e != cudaSuccess) return cuda_err(e, "capture wave");
     if (e2 != cudaSuccess) return cuda_err(e2, "end capture");
@@ -159,7 +163,7 @@ int32_t WaveEngine::launch(const WaveOutputs& out, bool deep, cudaStream_t strea
         cudaGraphExecDestroy(graphs_.front().exec);
         graphs_.erase(graphs_.begin());
     }
-    graphs_.push_back(Graph{out, deep, exec});
+    graphs_.push_back(Graph{out, deep, wide, exec});
     ECK(cudaGraphLaunch(exec, stream), "graph launch");
     return CVX_OK;
 }
@@ -182,6 +186,7 @@ int32_t WaveEngine::submit(const std::vector<Job>& jobs_in, WaveOutputs out, cud
     if (jobs_in.size() > max_jobs_) return set_error(CVX_ERR_CAPACITY, "too many jobs for one wave");
     uint64_t total = 0, deep_total = 0;
     uint32_t depth = 0;
+    bool wide = false;
     for (size_t i = 0; i < jobs_in.size(); i++) {
         Job j = jobs_in[i];
         if (j.scene >= n_scenes_) return set_error(CVX_ERR_INVALID, "job scene outside the scene table");
@@ -189,6 +194,7 @@ int32_t WaveEngine::submit(const std::vector<Job>& jobs_in, WaveOutputs out, cud
             return set_error(CVX_ERR_INVALID, "job image size out of range");
         const uint32_t dj = scene_depth_[j.scene];
         depth = dj > depth ? dj : depth;
+        wide = wide || scene_wide_[j.scene];
         j.n_groups = groups_of(j.w, j.h);
         if (dj >= kRefillMinDepth) deep_total += j.n_groups;
         if (total + j.n_groups > max_groups_) return set_error(CVX_ERR_CAPACITY, "wave exceeds the ray-queue capacity");
@@ -234,7 +240,7 @@ int32_t WaveEngine::submit(const std::vector<Job>& jobs_in, WaveOutputs out, cud
     ECK(cudaMemsetAsync(d_err_, 0, 8, stream), "reset status");
     if (want_job_rays) ECK(cudaMemsetAsync(d_job_rays_, 0, jobs_in.size() * 8, stream), "reset counters");
     ECK(cudaEventRecord(e0_, stream), "event");
-    int32_t st = launch(out, deep, stream);
+    int32_t st = launch(out, deep, wide, stream);
     if (st) return st;
     ECK(cudaEventRecord(e1_, stream), "event");
     ECK(cudaMemcpyAsync(&h_read_->rays, d_rays_, 8, cudaMemcpyDeviceToHost, stream), "read counters");

@@ -67,7 +67,7 @@ class WaveEngine {
     bool takes_sample_slots() const { return fused_ && !packet_ && refill_mode_ == CVX_REFILL_ALL; }
 
    private:
-    int32_t launch(const WaveOutputs& out, bool deep, cudaStream_t stream);
+    int32_t launch(const WaveOutputs& out, bool deep, bool wide, cudaStream_t stream);
     struct Readback {
         unsigned long long rays;
         uint32_t err;
@@ -78,7 +78,7 @@ class WaveEngine {
     bool last_want_ = false, fused_ = false;
     struct Graph {
         WaveOutputs out;
-        bool deep;
+        bool deep, wide;
         cudaGraphExec_t exec;
     };
     WaveState st_{};
@@ -93,6 +93,7 @@ class WaveEngine {
     uint32_t* d_group_em_ = nullptr;  // per group of a wave: the path refill's emitter counts
     uint32_t group_em_cap_ = 0;
     std::vector<uint32_t> scene_depth_;
+    std::vector<bool> scene_wide_;
     uint32_t n_scenes_ = 0, scene_cap_ = 0, max_groups_ = 0, max_jobs_ = 0, blocks_per_sm_ = 0, refill_from_ = 1,
              refill_mode_ = 0;
     bool packet_ = false, use_graph_ = false;

@@ -113,7 +113,8 @@ __global__ void k_prep_lights(const cvx_triangle* __restrict__ tris, const uint3
 // Nearest hit over SoA rays (Bvh::intersect_nearest, bvh.rs:659): eight
 // consecutive rays are one reference packet, or each is traced by itself
 // (k_intersect_packets, k_intersect_warp; k_intersect_refill, k_intersect_lanes
-// below). k_intersect_counts also counts the boxes and triangles of packets.
+// below). k_intersect_octets walks the pairs with a packet per octet, and counts
+// the boxes and triangles of packets (COUNT).
 
 // Next unit (group or packet) index for the calling octet (one atomic by its lane 0).
 __device__ __forceinline__ uint32_t octet_claim(uint32_t* counter, unsigned omask, int k) {
@@ -122,7 +123,8 @@ __device__ __forceinline__ uint32_t octet_claim(uint32_t* counter, unsigned omas
     return __shfl_sync(omask, g, (int)(threadIdx.x & 24u));
 }
 
-__global__ void __launch_bounds__(256) k_intersect_counts(DeviceScene s, const RayCols rays, uint32_t n,
+template <bool COUNT>
+__global__ void __launch_bounds__(256) k_intersect_octets(DeviceScene s, const RayCols rays, uint32_t n,
                                                           float far_dist, float* __restrict__ t_out,
                                                           int32_t* __restrict__ tri_out,
                                                           uint32_t* __restrict__ counters, uint32_t* __restrict__ err) {
@@ -140,12 +142,23 @@ __global__ void __launch_bounds__(256) k_intersect_counts(DeviceScene s, const R
         F3 d = f3(__ldg(rays.c[3] + src), __ldg(rays.c[4] + src), __ldg(rays.c[5] + src));
         Hit h{far_dist, 0.0f, 0.0f, -1};
         Counters c{0u, 0u};
-        if (!traverse<true>(s, o, d, active, omask, h, tab, &c)) atomicOr(err, kErrStackOverflow);
+        bool ok;
+        // The select-form slab test for a packet whose 8 rays all allow it,
+        // decided once per packet outside the traversal loop (4M random rays:
+        // 3.05 -> 2.92 ms; the same results).
+        if (!COUNT && s.slab_sel &&
+            oct_all(omask, select_form_recip(f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab)))))
+            ok = traverse<true, true>(s, o, d, active, omask, h, tab, nullptr);
+        else
+            ok = traverse<true>(s, o, d, active, omask, h, tab, COUNT ? &c : nullptr);
+        if (!ok) atomicOr(err, kErrStackOverflow);
         if (active) {
             t_out[i] = h.t;
             tri_out[i] = h.tri;
-            counters[i] = c.aabb;
-            counters[n + i] = c.tri;
+            if (COUNT) {
+                counters[i] = c.aabb;
+                counters[n + i] = c.tri;
+            }
         }
     }
 }
@@ -163,6 +176,7 @@ struct SoaRays {
     float* t_out;
     int32_t* tri_out;
     uint32_t* counters;
+    uint32_t slab_sel;  // DeviceScene::slab_sel
     __device__ __forceinline__ bool load(uint32_t r, F3& o, F3& d, float& far, const float4*& nd,
                                          const float4*& gm) const {
         nd = nodes;
@@ -280,7 +294,10 @@ struct StagedSoaClaim {
 // limit check per record 608, 468, 146. Two, three, four records per round:
 // 615, 605, 719; 472, 475, 546; 145, 146, 168 us. Ending a round early when few
 // lanes can walk on costs more in votes than it saves (748-794 us with pairs).
-constexpr int kQuerySteps = 2;
+// Pairs (Form::kPairs and kX86), with the leaf of a step tested by the next one:
+// 1, 3, 4 steps 0.798, 0.784, 0.777 ms per 4M rays of the icosphere, tube 1.538,
+// 1.503, 1.499 (six: within noise).
+constexpr int kQuerySteps = 2, kQueryPairSteps = 4;
 // Each lane's traversal stack lies in local memory. A scene may keep the first 4, 8
 // or 12 entries in shared memory instead (cvx_scene_set_query_stack, which the query
 // autotuner sets per scene). Eight shared entries were the better default while
@@ -290,11 +307,11 @@ constexpr int kQuerySteps = 2;
 // The other launch shapes keep 8.
 constexpr int kQueryStackShared = 8;
 
-// SELECT: the select-form slab test and postponed leaves for the rays that
-// meet the conditions (on scenes that do); the others are marked kDeferredRay
-// and traced by k_intersect_deferred.
+// FORM kWide or, for scenes that allow the select form but have no wide records,
+// kPairs: the rays that the form does not allow are marked kDeferredRay and traced
+// by k_intersect_deferred.
 // SHARED: stack entries of each lane in shared memory (the rest in local).
-template <int MINB, bool COUNT, int CLAIM, bool SELECT, int SHARED = kQueryStackShared>
+template <int MINB, bool COUNT, int CLAIM, Form FORM, int SHARED = kQueryStackShared>
 __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uint32_t* __restrict__ next_ray,
                                                                 uint32_t* __restrict__ err) {
     // The reciprocal table is read three times per ray: from global memory
@@ -303,7 +320,8 @@ __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uin
     __shared__ uint2 sstack[4][SHARED > 0 ? SHARED : 1][32];
     StagedSoaClaim claim{src, next_ray, stage[threadIdx.x >> 5], 0u, 0u, 0u, 0};
     claim.init(threadIdx.x & 31);
-    bool ok = traverse_refill<COUNT, false, CLAIM, SHARED, SELECT, kQuerySteps, SELECT && CLAIM == 8>(
+    constexpr bool kWide = FORM == Form::kWide;
+    bool ok = traverse_refill<COUNT, false, CLAIM, SHARED, FORM, kWide ? kQuerySteps : kQueryPairSteps, kWide && CLAIM == 8>(
         src, claim, g_tables, &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
     if (!ok) atomicOr(err, kErrStackOverflow);
 }
@@ -321,14 +339,21 @@ __global__ void __launch_bounds__(128, MINB) k_intersect_refill(SoaRays src, uin
 // round's second leaf tested at once and the stack in local memory: 290, 598, 1164
 // us; 5, 6, 8 blocks 288, 287, 307 us (room), 601, 594, 642 (icosphere).
 constexpr int kPacketBlocksPerSm = 7;
-template <int STEPS>
+// Scenes without wide records, us at 131,072, 1M and 4M rays, a packet per octet
+// (k_intersect_octets) against pairs in step, six per round (four: the same; one
+// and two 1-5 % more): room with loose roots 102/120, 334/343, 1220/1151; icosphere
+// 228/307, 806/725, 2988/2405; tube 526/547, 1479/1230, 5265/3949; a room under a
+// chain of 80 levels 190/332, 912/961, 3513/3549. Pairs in step from 2^20 rays.
+constexpr uint32_t kPairPacketRays = 1u << 20;
+constexpr int kPairPacketSteps = 6;
+template <int STEPS, Form FORM>
 __global__ void __launch_bounds__(128, kPacketBlocksPerSm) k_intersect_packets(SoaRays src,
                                                                                uint32_t* __restrict__ next_ray,
                                                                                uint32_t* __restrict__ err) {
     __shared__ float stage[4][2][6][32];
     StagedSoaClaim claim{src, next_ray, stage[threadIdx.x >> 5], 0u, 0u, 0u, 0};
     claim.init(threadIdx.x & 31);
-    bool ok = traverse_packets<STEPS>(src, claim, g_tables);
+    bool ok = traverse_packets<STEPS, FORM>(src, claim, g_tables);
     if (!ok) atomicOr(err, kErrStackOverflow);
 }
 
@@ -341,7 +366,11 @@ __global__ void __launch_bounds__(128, kPacketBlocksPerSm) k_intersect_packets(S
 // -> 124, 181 -> 182; packets, 19-level room 59 -> 46, 94 -> 63, 165 -> 123, 212 ->
 // 198; 70-level tube 241 -> 163, 421 -> 255, 640 -> 497, 839 -> 787; single rays,
 // room 52 -> 42, 68 -> 51, 91 -> 70, 112 -> 102, tube 234 -> 186, 218 -> 165, 312
-// -> 287, 419 -> 470. `err` may be page-locked host memory (it is stored to).
+// -> 287, 419 -> 470. Packets on scenes without wide records, a packet per octet
+// -> this, at 4,096, 32,768, 65,536, 131,072 rays: room with loose roots 96 -> 58,
+// 89 -> 72, 87 -> 82, 102 -> 120; icosphere 146 -> 112, 190 -> 163, 210 -> 201, 228 ->
+// 307; under a chain of 80 levels (room) 165 -> 92, 164 -> 131, 167 -> 196, 191 -> 328.
+// `err` may be page-locked host memory (it is stored to).
 __global__ void __launch_bounds__(64) k_intersect_warp(DeviceScene s, const RayCols rays, uint32_t n, float far_dist,
                                                        float* __restrict__ t_out, int32_t* __restrict__ tri_out,
                                                        uint32_t* err) {
@@ -389,7 +418,7 @@ __global__ void __launch_bounds__(32) k_intersect_lanes(DeviceScene s, const Ray
     if (overflow) *reinterpret_cast<volatile uint32_t*>(err) = kErrStackOverflow;
 }
 
-// After k_intersect_refill<SELECT>: the rays it left (index word kDeferredRay:
+// After k_intersect_refill: the rays it left (index word kDeferredRay:
 // a reciprocal infinite or below 0.75 in magnitude) with the x86-form slab
 // test. Such rays are rare (axis-parallel or very long directions), so the
 // scan over the index words is most of the work: each thread reads
@@ -501,8 +530,8 @@ __device__ __forceinline__ void flush_rays(const FrameArgs& a, uint32_t rays) {
     if ((threadIdx.x & 31u) == 0u && v) atomicAdd(a.rays, v);
 }
 
-// An octet renders whole groups: single rays, and the debug view (PACKET: of
-// packets; their frames take k_render_packets).
+// An octet renders whole groups: single rays, the debug view, and packets of the
+// scenes that k_render_packets leaves to it.
 template <bool PACKET>
 __global__ void __launch_bounds__(128, 8) k_render_group(FrameArgs a) {
     __shared__ ApproxTables tab;
@@ -532,8 +561,8 @@ __global__ void __launch_bounds__(128, 8) k_render_group(FrameArgs a) {
         x = fmaf(unit_from(rng.next()), scale, x);
         y = fmaf(unit_from(rng.next()), scale, y);
         PixelOut p;
-        if (PACKET || a.debug) ok &= render_pixels_debug<PACKET>(a.s, a.cam, x, y, omask, tab, p, rays);
-        else ok &= render_pixels<false>(a.s, a.cam, x, y, rng, omask, tab, p, rays);
+        if (a.debug) ok &= render_pixels_debug<PACKET>(a.s, a.cam, x, y, omask, tab, p, rays);
+        else ok &= render_pixels<PACKET>(a.s, a.cam, x, y, rng, omask, tab, p, rays);
         store_pixel(a, gx + (uint32_t)(k & 3), gy + (uint32_t)(k >> 2), p);
     }
     if (!ok) atomicOr(a.err, kErrStackOverflow);
@@ -675,15 +704,41 @@ constexpr int kDeepFrameClaim = 12;
 constexpr int kDeepFrameSteps = 2;
 // DEEP: a tree deeper than 40 levels (the constants above).
 // MULTI: a.samples samples in one launch (FramePaths<true>).
-template <bool DEEP, bool COUNT, bool MULTI = false>
+// FORM kPairs: a scene without wide records, and the counting form. Three steps
+// per round; deep trees wait for 8 lanes, keep the first 16 stack entries of each
+// lane in shared memory and read the tables from global memory (tube, ms per sample:
+// local stack 3.07-3.11, 16 entries 2.99; at claim 8 one, two, three, four steps
+// 3.15, 2.98, 2.93, 3.07). Icosphere and tube with loose roots, 1280x736: 1.42 and
+// 2.92 ms; in the kWide kernel's x86 steps 1.48 and 3.18.
+constexpr int kPairFrameSteps = 3, kDeepPairFrameClaim = 8, kDeepPairFrameStack = 16;
+template <bool DEEP, bool COUNT, Form FORM, bool MULTI = false>
 __global__ void __launch_bounds__(128, kRefillFrameBlocksPerSm) k_render_refill(FrameArgs a) {
     FramePaths<MULTI> P{a, (a.w + 15u) / 16u, (a.h + 3u) / 4u, 0u};
-    __shared__ ApproxTables tab;
-    load_tables(tab);
     bool ok;
-    if constexpr (DEEP) ok = path_refill<kDeepFrameClaim, kDeepFrameSteps, COUNT, true, true>(P, tab);
-    else ok = path_refill<16, kRefillFrameSteps, COUNT, true>(P, tab);
+    if constexpr (FORM == Form::kPairs && DEEP) {
+        __shared__ uint2 sstack[4][kDeepPairFrameStack][32];
+        ok = path_refill<kDeepPairFrameClaim, kPairFrameSteps, COUNT, FORM, false, kDeepPairFrameStack>(
+            P, g_tables, &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
+    } else {
+        __shared__ ApproxTables tab;
+        load_tables(tab);
+        if constexpr (FORM == Form::kPairs) ok = path_refill<16, kPairFrameSteps, COUNT, FORM>(P, tab);
+        else if constexpr (DEEP) ok = path_refill<kDeepFrameClaim, kDeepFrameSteps, COUNT, FORM, true>(P, tab);
+        else ok = path_refill<16, kRefillFrameSteps, COUNT, FORM>(P, tab);
+    }
     if (!ok) atomicOr(a.err, kErrStackOverflow);
+}
+
+template <Form FORM>
+static void launch_refill(const FrameArgs& a, uint32_t blocks, cudaStream_t st) {
+    const bool deep = a.s.depth > 40;
+    if (a.samples > 1) {
+        if (deep) k_render_refill<true, false, FORM, true><<<blocks, 128, 0, st>>>(a);
+        else k_render_refill<false, false, FORM, true><<<blocks, 128, 0, st>>>(a);
+    } else {
+        if (deep) k_render_refill<true, false, FORM><<<blocks, 128, 0, st>>>(a);
+        else k_render_refill<false, false, FORM><<<blocks, 128, 0, st>>>(a);
+    }
 }
 
 // Frames in packet traversal, per-group RNG order: an octet holds one 8-pixel
@@ -694,12 +749,25 @@ __global__ void __launch_bounds__(128, kRefillFrameBlocksPerSm) k_render_refill(
 // per SM (80 registers and more, no spill; 6 and 7 blocks: room 1.14, 1.21 ms,
 // icosphere 2.77, 2.76 ms, the small one 0.61, 0.64 ms); trees deeper than 40
 // levels one record and 6 blocks (6.34 ms; two records 6.81-6.85).
-template <bool DEEP>
+// Scenes without wide records (kPairs), one group per octet against this, us at
+// 320x184, 640x368, 900x516, 1280x736, 1920x1080: room with loose roots 608/395,
+// 697/528, 809/757, 1210/1362, 2495/2844; icosphere 981/657, 1402/1106, 2019/1823,
+// 3610/3316, 7550/6867; tube 3259/2381, 3976/2888, 5609/4292, 8787/7210, 16709/14228;
+// the icosphere under a chain of 60 levels 1244/811, 2011/1669, 3063/2875, 5629/5399,
+// 11833/11379; the room under one of 80 levels 957/606, 1227/1210, 2052/2130,
+// 3888/4058, 8209/8655. Six pairs per round (one to four: 1439, 1402, 1364, 1362 us for
+// the room at 1280x736; eight: the same).
+constexpr int kPairGroupSteps = 6;
+inline bool packets_in_step(const DeviceScene& s, uint32_t pixels) {
+    if (s.wide) return true;
+    return s.depth < 25u ? pixels <= 600000u : s.depth <= kWideMaxDepth || pixels <= 300000u;
+}
+template <bool DEEP, Form FORM>
 __global__ void __launch_bounds__(128, DEEP ? 6 : 5) k_render_packets(FrameArgs a) {
     __shared__ ApproxTables tab;
     load_tables(tab);
     FramePaths<false> P{a, (a.w + 15u) / 16u, (a.h + 3u) / 4u, 0u};
-    bool ok = group_refill<DEEP ? 1 : 2>(P, tab);
+    bool ok = group_refill<FORM == Form::kPairs ? kPairGroupSteps : DEEP ? 1 : 2, FORM>(P, tab);
     if (!ok) atomicOr(a.err, kErrStackOverflow);
 }
 
@@ -1012,10 +1080,10 @@ template <int CLAIM>
 static void launch_select_stack(uint32_t shared, uint32_t blocks, const SoaRays& src, uint32_t* err,
                                 cudaStream_t st) {
     switch (shared) {
-        case 4: k_intersect_refill<8, false, CLAIM, true, 4><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
-        case 12: k_intersect_refill<8, false, CLAIM, true, 12><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
-        case 8: k_intersect_refill<8, false, CLAIM, true, 8><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
-        default: k_intersect_refill<8, false, CLAIM, true, 0><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
+        case 4: k_intersect_refill<8, false, CLAIM, Form::kWide, 4><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
+        case 12: k_intersect_refill<8, false, CLAIM, Form::kWide, 12><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
+        case 8: k_intersect_refill<8, false, CLAIM, Form::kWide, 8><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
+        default: k_intersect_refill<8, false, CLAIM, Form::kWide, 0><<<blocks, 128, 0, st>>>(src, err + 1, err); break;
     }
 }
 
@@ -1024,7 +1092,7 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
                              uint32_t blocks_per_sm, cudaStream_t st, uint32_t shared_stack) {
     // Calls that do not fill the GPU several times over: one packet per warp, or
     // one ray per lane, with nothing claimed.
-    if (!counters && direct_query(n, blocks_per_sm)) {
+    if (!counters && direct_query(s, n, packet, blocks_per_sm)) {
         if (packet) k_intersect_warp<<<(n + 15u) / 16u, 64, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
         else k_intersect_lanes<<<(n + 31u) / 32u, 32, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, err);
         return cudaGetLastError();
@@ -1037,20 +1105,23 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
         uint32_t blocks = (uint32_t)num_sms() * bps;
         uint32_t need = (n + 127u) / 128u;
         if (blocks > need) blocks = need;
-        SoaRays src{s.nodes, s.wide, s.geom, rays, n, far_dist, t_out, tri_out, counters};
+        SoaRays src{s.nodes, s.wide, s.geom, rays, n, far_dist, t_out, tri_out, counters, s.slab_sel};
         bool deep = s.depth > 40;
-        const bool sel = s.wide && !counters;
-        if (counters) k_intersect_refill<8, true, 16, false><<<blocks, 128, 0, st>>>(src, err + 1, err);
+        const bool sel = s.slab_sel && !counters;
+        if (counters) k_intersect_refill<8, true, 16, Form::kX86><<<blocks, 128, 0, st>>>(src, err + 1, err);
         else if (!sel) {  // x86-form slab test throughout
-            if (deep) k_intersect_refill<8, false, 8, false><<<blocks, 128, 0, st>>>(src, err + 1, err);
-            else k_intersect_refill<8, false, 16, false><<<blocks, 128, 0, st>>>(src, err + 1, err);
+            if (deep) k_intersect_refill<8, false, 8, Form::kX86><<<blocks, 128, 0, st>>>(src, err + 1, err);
+            else k_intersect_refill<8, false, 16, Form::kX86><<<blocks, 128, 0, st>>>(src, err + 1, err);
+        } else if (!s.wide) {
+            if (deep) k_intersect_refill<8, false, 8, Form::kPairs><<<blocks, 128, 0, st>>>(src, err + 1, err);
+            else k_intersect_refill<8, false, 16, Form::kPairs><<<blocks, 128, 0, st>>>(src, err + 1, err);
         } else if (deep) {
-            if (bps >= 12) k_intersect_refill<12, false, 8, true><<<blocks, 128, 0, st>>>(src, err + 1, err);
-            else if (bps >= 10) k_intersect_refill<10, false, 8, true><<<blocks, 128, 0, st>>>(src, err + 1, err);
+            if (bps >= 12) k_intersect_refill<12, false, 8, Form::kWide><<<blocks, 128, 0, st>>>(src, err + 1, err);
+            else if (bps >= 10) k_intersect_refill<10, false, 8, Form::kWide><<<blocks, 128, 0, st>>>(src, err + 1, err);
             else launch_select_stack<8>(shared_stack, blocks, src, err, st);
         } else {
-            if (bps >= 12) k_intersect_refill<12, false, 16, true><<<blocks, 128, 0, st>>>(src, err + 1, err);
-            else if (bps >= 10) k_intersect_refill<10, false, 16, true><<<blocks, 128, 0, st>>>(src, err + 1, err);
+            if (bps >= 12) k_intersect_refill<12, false, 16, Form::kWide><<<blocks, 128, 0, st>>>(src, err + 1, err);
+            else if (bps >= 10) k_intersect_refill<10, false, 16, Form::kWide><<<blocks, 128, 0, st>>>(src, err + 1, err);
             else launch_select_stack<16>(shared_stack, blocks, src, err, st);
         }
         if (sel) {
@@ -1061,12 +1132,13 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
     }
     cudaError_t e = cudaMemsetAsync(err + 1, 0, 4, st);  // packet counter
     if (e != cudaSuccess) return e;
-    if (!counters) {
+    if (!counters && (s.wide || n >= kPairPacketRays)) {
         uint32_t blocks = (uint32_t)num_sms() * kPacketBlocksPerSm, need = (n + 127u) / 128u;
         if (blocks > need) blocks = need;
-        SoaRays src{s.nodes, s.wide, s.geom, rays, n, far_dist, t_out, tri_out, nullptr};
-        if (s.depth > 40) k_intersect_packets<1><<<blocks, 128, 0, st>>>(src, err + 1, err);
-        else k_intersect_packets<2><<<blocks, 128, 0, st>>>(src, err + 1, err);
+        SoaRays src{s.nodes, s.wide, s.geom, rays, n, far_dist, t_out, tri_out, nullptr, s.slab_sel};
+        if (!s.wide) k_intersect_packets<kPairPacketSteps, Form::kPairs><<<blocks, 128, 0, st>>>(src, err + 1, err);
+        else if (s.depth > 40) k_intersect_packets<1, Form::kWide><<<blocks, 128, 0, st>>>(src, err + 1, err);
+        else k_intersect_packets<2, Form::kWide><<<blocks, 128, 0, st>>>(src, err + 1, err);
         return cudaGetLastError();
     }
     if (block == 0) block = 128;
@@ -1074,7 +1146,8 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
     uint32_t need = ((n + 7u) & ~7u) / block + 1u;
     uint32_t blocks = (uint32_t)num_sms() * blocks_per_sm;
     if (blocks > need) blocks = need;
-    k_intersect_counts<<<blocks, block, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, counters, err);
+    if (counters) k_intersect_octets<true><<<blocks, block, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, counters, err);
+    else k_intersect_octets<false><<<blocks, block, 0, st>>>(s, rays, n, far_dist, t_out, tri_out, nullptr, err);
     return cudaGetLastError();
 }
 
@@ -1098,15 +1171,12 @@ cudaError_t launch_render(const DeviceScene& s, const DeviceCamera& cam, uint32_
         if (blocks > need) blocks = need;
         if (work) {
             if (samples > 1) return cudaErrorInvalidValue;
-            if (s.depth > 40) k_render_refill<true, true><<<blocks, 128, 0, st>>>(a);
-            else k_render_refill<false, true><<<blocks, 128, 0, st>>>(a);
-        } else if (samples > 1) {
-            if (s.depth > 40) k_render_refill<true, false, true><<<blocks, 128, 0, st>>>(a);
-            else k_render_refill<false, false, true><<<blocks, 128, 0, st>>>(a);
-        } else if (s.depth > 40) {
-            k_render_refill<true, false><<<blocks, 128, 0, st>>>(a);
+            if (s.depth > 40) k_render_refill<true, true, Form::kPairs><<<blocks, 128, 0, st>>>(a);
+            else k_render_refill<false, true, Form::kPairs><<<blocks, 128, 0, st>>>(a);
+        } else if (s.wide) {
+            launch_refill<Form::kWide>(a, blocks, st);
         } else {
-            k_render_refill<false, false><<<blocks, 128, 0, st>>>(a);
+            launch_refill<Form::kPairs>(a, blocks, st);
         }
         if (gbuf) {
             uint32_t fb = (ngroups + 255u) / 256u, cap = (uint32_t)num_sms() * 8u;
@@ -1132,11 +1202,12 @@ cudaError_t launch_render(const DeviceScene& s, const DeviceCamera& cam, uint32_
         uint32_t need = (units * 8 + block - 1) / block;
         uint32_t blocks = (uint32_t)num_sms() * 16u;
         if (blocks > need) blocks = need;
-        if (packet && !debug) {
-            const bool deep = s.depth > 40;
+        if (packet && !debug && packets_in_step(s, w * h)) {
+            const bool deep = s.wide && s.depth > 40;
             blocks = std::min((uint32_t)num_sms() * (deep ? 6u : 5u), (units * 8u + 127u) / 128u);
-            if (deep) k_render_packets<true><<<blocks, 128, 0, st>>>(a);
-            else k_render_packets<false><<<blocks, 128, 0, st>>>(a);
+            if (!s.wide) k_render_packets<false, Form::kPairs><<<blocks, 128, 0, st>>>(a);
+            else if (deep) k_render_packets<true, Form::kWide><<<blocks, 128, 0, st>>>(a);
+            else k_render_packets<false, Form::kWide><<<blocks, 128, 0, st>>>(a);
         } else if (packet) k_render_group<true><<<blocks, block, 0, st>>>(a);
         else k_render_group<false><<<blocks, block, 0, st>>>(a);
     }

@@ -33,12 +33,15 @@ inline RayCols soa_cols(const float* rays, uint32_t n) {  // one (6, n) device a
 }
 
 // Whether a query takes the direct kernels (one packet per warp, one ray per lane):
-// up to kDirectRays rays, unless a launch shape of the persistent kernels is set
-// (times at k_intersect_warp). They store to `err`, which may then be page-locked
-// host memory, and use no counter behind it; the persistent kernels claim from
-// err[1], which must be device memory. They have no stack in shared memory.
-constexpr uint32_t kDirectRays = 262144;
-inline bool direct_query(uint32_t n, uint32_t blocks_per_sm) { return n <= kDirectRays && blocks_per_sm == 0; }
+// up to kDirectRays rays (packets on a scene without wide records up to
+// kDirectPairRays), unless a launch shape of the persistent kernels is set (times
+// at k_intersect_warp). They store to `err`, which may then be page-locked host
+// memory, and use no counter behind it; the others claim from err[1], which must be
+// device memory. They have no stack in shared memory.
+constexpr uint32_t kDirectRays = 262144, kDirectPairRays = 32768;
+inline bool direct_query(const DeviceScene& s, uint32_t n, bool packet, uint32_t blocks_per_sm) {
+    return n <= (packet && !s.wide ? kDirectPairRays : kDirectRays) && blocks_per_sm == 0;
+}
 // shared_stack: stack entries of each lane kept in shared memory by the
 // persistent single-ray kernel at 8 blocks per SM (0, 4, 8 or 12; other launch
 // shapes keep 8).
@@ -99,7 +102,7 @@ cudaError_t launch_wave(const Job* jobs, const WaveHeader* hdr, const DeviceScen
 // The fused (megakernel) form of a wave: one persistent launch.
 // deep: a scene of the wave is deeper than 40 levels (claim threshold 8, else 16)
 cudaError_t launch_wave_fused(const Job* jobs, const WaveHeader* hdr, const DeviceScene* scenes,
-                              const WaveOutputs& out, bool packet, uint32_t blocks_per_sm, bool deep,
+                              const WaveOutputs& out, bool packet, uint32_t blocks_per_sm, bool deep, bool wide,
                               cudaStream_t stream);
 cudaError_t launch_resolve_multi(const ResolveItem* items, uint32_t n_items, const float* accum, uint32_t* rgba,
                                  cudaStream_t stream);

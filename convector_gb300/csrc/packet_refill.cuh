@@ -65,12 +65,12 @@ struct PacketRay {
     }
 
     // One step of each packet that is `on` (the whole warp calls this): at most
-    // one pop, and the wide record of its next node (SELECT, walking on past one
-    // waiting leaf) or that node's pair in the x86 form (a waiting leaf stops the
-    // packet).
-    template <bool SELECT, class Stack>
+    // one pop, and the wide record of its next node (kWide, walking on past one
+    // waiting leaf) or that node's pair (a waiting leaf stops the packet).
+    template <Form FORM, class Stack>
     __device__ __forceinline__ void walk(bool on, Stack& stack, bool& overflow) {
-        const bool pop = on && cur == kNone && sp > 0 && (SELECT || leaf == 0u);
+        constexpr bool kPast = FORM == Form::kWide;
+        const bool pop = on && cur == kNone && sp > 0 && (kPast || leaf == 0u);
         const uint2 e = top;
         if (pop) top = stack.load(--sp);
         const bool kept = any(active & !geq(__uint_as_float(e.y), h.t));
@@ -82,21 +82,26 @@ struct PacketRay {
                 cur_t = __uint_as_float(e.y);
             }
         }
-        const bool next = on && (cur & 31u) == 0u && (SELECT || leaf == 0u);
-        if constexpr (SELECT) wide_step(next, stack, overflow);
-        else pair_step(next, stack, overflow);
+        const bool next = on && (cur & 31u) == 0u && (kPast || leaf == 0u);
+        if constexpr (FORM == Form::kWide) wide_step(next, stack, overflow);
+        else pair_step<FORM == Form::kPairs>(next, stack, overflow);
     }
 
-    // The node pair of each packet with `pair`, in the x86 form.
-    template <class Stack>
+    // The node pair of each packet with `pair`, in the select form or the x86 form.
+    template <bool SELECT, class Stack>
     __device__ __forceinline__ void pair_step(bool pair, Stack& stack, bool& overflow) {
         BoxT b0{0.0f, 0.0f, false}, b1{0.0f, 0.0f, false};
         uint32_t r0 = 0u, r1 = 0u;
         if (pair) {
             const float4* np = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + cur);
             const float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
-            b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
-            b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
+            if constexpr (SELECT) {
+                b0 = box_test_sel(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
+                b1 = box_test_sel(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
+            } else {
+                b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o, inv);
+                b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o, inv);
+            }
             r0 = __float_as_uint(q3.x);
             r1 = __float_as_uint(q3.y);
         }
@@ -138,7 +143,7 @@ struct PacketRay {
             vis[k] = any(active & (c[k] < h.t)) & hit;
         }
         const bool in0 = all(ge0(p.t[0] - p.t[1])), in1 = all(ge0(p.t[2] - p.t[3])), ch = all(ge0(p.tc0 - p.tc1));
-        if (__builtin_expect(__any_sync(kFullWarp, zero), 0)) pair_step(zero, stack, overflow);
+        if (__builtin_expect(__any_sync(kFullWarp, zero), 0)) pair_step<false>(zero, stack, overflow);
         if (!rec || zero) return;
         const bool va0 = in0 ? vis[0] : vis[1], va1 = in0 ? vis[1] : vis[0];
         const bool vb0 = in1 ? vis[2] : vis[3], vb1 = in1 ? vis[3] : vis[2];
@@ -206,29 +211,43 @@ struct PacketRay {
         return cur == kNone && sp == 0 && leaf == 0u;
     }
     // One round of the warp: STEPS wide records of each packet, with the leaves
-    // they lead to tested once (sel: every packet `on` allows the select form),
-    // or pair by pair in the x86 form. Returns true when the packet is finished.
-    template <int STEPS, class Stack>
+    // they lead to tested once (kWide), or STEPS pairs with each leaf tested at
+    // once (kPairs); in the x86 form unless every packet `on` allows FORM (sel).
+    // Returns true when the packet is finished.
+    template <int STEPS, Form FORM, class Stack>
     __device__ __forceinline__ bool round(bool on, bool sel, Stack& stack, bool& overflow) {
         bool fin = false;
         if (!__any_sync(kFullWarp, on)) return false;  // (and then there may be no wide records)
         if (__all_sync(kFullWarp, !on || sel)) {
+            if constexpr (FORM == Form::kWide) {
 #pragma unroll 1
-            for (int st = 0; st < STEPS; st++) walk<true>(on, stack, overflow);
-            fin = test_leaf(on);
-            // Two records may lead to two leaves, of which the second stopped its packet:
-            // tested now instead of after the next round (1M packets: room 311 -> 299
-            // us, icosphere 632 -> 620; frames -0.6 and -1 %). With one record per round a
-            // second test costs 1.5 %.
-            if (STEPS > 1 && __any_sync(kFullWarp, on && leaf != 0u)) fin = test_leaf(on);
-        } else {
-#pragma unroll 1
-            for (int st = 0; st < STEPS; st++) {
-                walk<false>(on && !fin, stack, overflow);
-                fin = test_leaf(on && !fin);
+                for (int st = 0; st < STEPS; st++) walk<Form::kWide>(on, stack, overflow);
+                fin = test_leaf(on);
+                // Two records may lead to two leaves, of which the second stopped its packet:
+                // tested now instead of after the next round (1M packets: room 311 -> 299
+                // us, icosphere 632 -> 620; frames -0.6 and -1 %). With one record per round a
+                // second test costs 1.5 %.
+                if (STEPS > 1 && __any_sync(kFullWarp, on && leaf != 0u)) fin = test_leaf(on);
+            } else {
+                pairs<STEPS, FORM>(on, fin, stack, overflow);
             }
+        } else {
+            pairs<STEPS, Form::kX86>(on, fin, stack, overflow);
         }
         return fin;
+    }
+    template <int STEPS, Form FORM, class Stack>
+    __device__ __forceinline__ void pairs(bool on, bool& fin, Stack& stack, bool& overflow) {
+#pragma unroll 1
+        for (int st = 0; st < STEPS; st++) {
+            walk<FORM>(on && !fin, stack, overflow);
+            fin = test_leaf(on && !fin);
+        }
+    }
+    // Whether the packet, whose lanes call this with the rest of the warp, allows FORM.
+    template <Form FORM>
+    __device__ __forceinline__ bool allows(bool scene_allows) const {
+        return all(form_allows<FORM>(o, inv)) && scene_allows;
     }
 };
 
@@ -236,7 +255,7 @@ struct PacketRay {
 // consecutive rays; src as in traverse_refill, with one scene). A finished packet
 // is replaced at once. The lanes of a last, partial packet beyond its rays are
 // inactive copies of its first lane's ray.
-template <int STEPS, class Src, class Claim>
+template <int STEPS, Form FORM, class Src, class Claim>
 __device__ __forceinline__ bool traverse_packets(const Src& src, Claim& claim, const ApproxTables& tab) {
     const int lane = threadIdx.x & 31;
     PacketRay ray;
@@ -269,11 +288,11 @@ __device__ __forceinline__ bool traverse_packets(const Src& src, Claim& claim, c
                     ray.start(mine ? in.o : o0, mine ? in.d : d0, mine, src.far_dist, src.nodes, src.wide, src.geom, tab);
                 }
             }
-            const bool all_sel = PacketRay::all(select_form_ray(ray.o, ray.inv));
-            if (want) sel = src.wide && all_sel;
+            const bool all_sel = ray.allows<FORM>(FORM == Form::kWide ? src.wide != nullptr : src.slab_sel != 0u);
+            if (want) sel = all_sel;
         }
         if (__all_sync(kFullWarp, done)) break;
-        if (ray.round<STEPS>(have, sel, stack, overflow) && have) {
+        if (ray.round<STEPS, FORM>(have, sel, stack, overflow) && have) {
             if (ray.active) src.store(r_id, ray.h, 0u, 0u);
             have = false;
         }
@@ -288,7 +307,7 @@ __device__ __forceinline__ bool traverse_packets(const Src& src, Claim& claim, c
 // it saves: icosphere 2.77 -> 2.97 ms, tube 6.81 -> 7.57 ms.) Paths: as in
 // path_refill, path numbers being claimed 8 at a time (a group's lanes);
 // mark_emitter is not used.
-template <int STEPS, class Paths>
+template <int STEPS, Form FORM, class Paths>
 __device__ __forceinline__ bool group_refill(Paths& P, const ApproxTables& tab) {
     typedef typename Paths::PathRef PathRef;
     const int lane = threadIdx.x & 31;
@@ -369,14 +388,14 @@ __device__ __forceinline__ bool group_refill(Paths& P, const ApproxTables& tab) 
         }
         if (__all_sync(kFullWarp, done)) break;
         if (__any_sync(kFullWarp, started)) {
-            const bool all_sel = PacketRay::all(select_form_ray(ray.o, ray.inv));
+            const bool all_sel = ray.allows<FORM>(true);
             if (started) {
                 const DeviceScene s = P.scene(ref);
-                sel = all_sel && s.wide != nullptr;
+                sel = all_sel && (FORM == Form::kWide ? s.wide != nullptr : s.slab_sel != 0u);
                 tracing = true;
             }
         }
-        if (ray.round<STEPS>(tracing, sel, stack, overflow)) tracing = false;
+        if (ray.round<STEPS, FORM>(tracing, sel, stack, overflow)) tracing = false;
     }
     P.finish(ref);
     return !overflow;

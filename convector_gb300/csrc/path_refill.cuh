@@ -45,16 +45,17 @@
 
 namespace cvx {
 
-// SELECT_ROUNDS: a round walks STEPS wide records with the select-form slab test
-// and tests the leaves they led to once, at its end (RefillRay::walk), when
-// every tracing lane's ray allows it (a warp-uniform choice, so neither form's
-// code runs for the other's lanes); otherwise it takes STEPS steps in the x86
-// form. Each lane's results are the same either way.
-// POOL_LEAVES: such a round's leaves are tested by the whole warp (RefillRay::
-// test_leaves).
-template <int CLAIM_MIN, int STEPS, bool COUNT = false, bool SELECT_ROUNDS = false, bool POOL_LEAVES = false,
-          class Paths>
-__device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab) {
+// FORM kWide: a round walks STEPS wide records and tests the leaves they led to
+// once, at its end (RefillRay::walk), when every tracing lane's ray allows it (a
+// warp-uniform choice, so neither form's code runs for the other's lanes);
+// otherwise, and with kX86, it takes STEPS steps in the x86 form. kPairs: STEPS
+// steps in the select form or the x86 form, by the same choice. Each lane's
+// results are the same either way.
+// POOL_LEAVES (with kWide): such a round's leaves are tested by the whole warp
+// (RefillRay::test_leaves).
+template <int CLAIM_MIN, int STEPS, bool COUNT, Form FORM, bool POOL_LEAVES = false, int SHARED_STACK = 0, class Paths>
+__device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab, uint2* shared_stack = nullptr) {
+    static_assert(!(COUNT && FORM == Form::kWide), "the wide records do not count the reference's boxes");
     typedef typename Paths::PathRef PathRef;
     __shared__ uint8_t owners[4][32];  // RefillRay::test_leaves, blocks of four warps
     uint8_t* const owner = owners[threadIdx.x >> 5];
@@ -62,7 +63,8 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab) {
     const uint32_t npaths = P.n_paths();
     RefillRay ray;
     uint2 local_stack[kStackSlots];
-    LocalStack stack{local_stack};
+    typename std::conditional<SHARED_STACK == 0, LocalStack, SharedLocalStack<SHARED_STACK>>::type stack =
+        make_stack<SHARED_STACK>(shared_stack, local_stack);
     ray.top = make_uint2(0u, 0u);
     ray.sp = 0;
     ray.cur = RefillRay::kNone;
@@ -79,7 +81,11 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab) {
     F3 color = f3(1.0f, 1.0f, 1.0f);
     uint32_t bounce = 0;
     bool tracing = false, has_path = false, done = false, overflow = false;
-    bool ray_sel = false;  // the current ray allows the select-form slab test (SELECT_ROUNDS)
+    bool ray_sel = false;  // the current ray's scene and the ray allow FORM
+    auto allowed = [&](const DeviceScene& s) {
+        if (FORM == Form::kX86) return false;
+        return (FORM == Form::kWide ? s.wide != nullptr : s.slab_sel != 0u) && form_allows<FORM>(ray.no, ray.inv);
+    };
     uint64_t work_boxes = 0, work_tris = 0, work_shades = 0;
     for (;;) {
         bool want = !tracing && !done;
@@ -126,7 +132,7 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab) {
             } else {
                 bounce++;
                 ray.start(n.o, n.d, 1.0e5f, s.nodes, s.wide, s.geom, tab);
-                ray_sel = SELECT_ROUNDS && s.wide && select_form_ray(ray.no, ray.inv);
+                ray_sel = allowed(s);
                 tracing = true;
                 P.count_ray(ref);
             }
@@ -148,7 +154,7 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab) {
                     if (P.begin(p, ref, o, d, rng, tab)) {  // else: a group outside its image; take another path
                         const DeviceScene s = P.scene(ref);
                         ray.start(o, d, 1.0e5f, s.nodes, s.wide, s.geom, tab);
-                        ray_sel = SELECT_ROUNDS && s.wide && select_form_ray(ray.no, ray.inv);
+                        ray_sel = allowed(s);
                         color = f3(1.0f, 1.0f, 1.0f);
                         bounce = 0u;
                         has_path = true;
@@ -159,20 +165,27 @@ __device__ __forceinline__ bool path_refill(Paths& P, const ApproxTables& tab) {
             }
         }
         if (__all_sync(0xffffffffu, done)) break;
-        if (SELECT_ROUNDS && !COUNT && __all_sync(0xffffffffu, !tracing || ray_sel)) {
-            if (tracing) {
+        const bool all_sel = FORM != Form::kX86 && __all_sync(0xffffffffu, !tracing || ray_sel);
+        if constexpr (FORM == Form::kWide) {
+            if (all_sel) {
+                if (tracing) {
 #pragma unroll 1
-                for (int st = 0; st < STEPS; st++) ray.walk(stack, overflow);
+                    for (int st = 0; st < STEPS; st++) ray.walk(stack, overflow);
+                }
+                bool finished;
+                if constexpr (POOL_LEAVES) finished = ray.test_leaves<Paths::kOneScene>(owner, tracing);
+                else finished = tracing && ray.test_leaf();
+                if (finished) tracing = false;
+                continue;
             }
-            bool finished;
-            if constexpr (POOL_LEAVES) finished = ray.test_leaves<Paths::kOneScene>(owner, tracing);
-            else finished = tracing && ray.test_leaf();
-            if (finished) tracing = false;
-        } else {
-            if (SELECT_ROUNDS && !COUNT) ray.settle();
+            ray.settle();
+        } else if (all_sel) {
             for (int st = 0; st < STEPS && tracing; st++)
-                if (ray.step<COUNT, true>(stack, overflow)) tracing = false;
+                if (ray.step<COUNT, true, FORM == Form::kPairs>(stack, overflow)) tracing = false;
+            continue;
         }
+        for (int st = 0; st < STEPS && tracing; st++)
+            if (ray.step<COUNT, true>(stack, overflow)) tracing = false;
     }
     if constexpr (COUNT) P.work(work_boxes, work_tris, work_shades);
     P.finish(ref);

@@ -17,11 +17,12 @@ struct TreeFacts {
     uint32_t depth = 0;  // roots at depth 1
     std::vector<uint8_t> reached_pairs;
     bool reached(uint32_t pair) const { return reached_pairs[pair] != 0; }
-    // Every bound is at most kSelectMax in magnitude, lo <= hi on each axis and
-    // none is -0: the select-form slab test (box_test_sel) gives box_test's bits.
+    // Every bound is finite, lo <= hi on each axis and none is -0: the select-form
+    // slab test (box_test_sel) gives box_test's bits.
     bool select = false;
-    // Besides, every node's bounds are exactly the enclosure of its children's, as
-    // the build makes them, and the tree is within the limits of the wide records.
+    // Besides, every bound is at most kSelectMax in magnitude, every node's bounds
+    // are exactly the enclosure of its children's, as the build makes them, and the
+    // tree is within the limits of the wide records.
     bool wide = false;
 };
 
@@ -49,15 +50,16 @@ inline const char* check_tree(const cvx_bvh_node* nodes, uint32_t n_nodes, uint3
         }
     }
     out->depth = depth;
-    bool select = true;
+    bool select = true, bounded = true;
     for (uint32_t i = 0; i < n_nodes && select; i++)
         for (int c = 0; c < 3 && out->reached(i / 2); c++) {
             const float lo = nodes[i].origin[c], hi = nodes[i].far_[c];
-            if (!(std::fabs(lo) <= kSelectMax) || !(std::fabs(hi) <= kSelectMax) || !(lo <= hi) ||
-                (lo == 0.0f && std::signbit(lo)) || (hi == 0.0f && std::signbit(hi)))
+            if (!std::isfinite(lo) || !std::isfinite(hi) || !(lo <= hi) || (lo == 0.0f && std::signbit(lo)) ||
+                (hi == 0.0f && std::signbit(hi)))
                 select = false;
+            if (!(std::fabs(lo) <= kSelectMax) || !(std::fabs(hi) <= kSelectMax)) bounded = false;
         }
-    bool tight = select;
+    bool tight = select && bounded;
     for (uint32_t i = 0; i < n_nodes && tight; i++) {
         if (nodes[i].len != 0 || !out->reached(i / 2)) continue;
         const cvx_bvh_node &c0 = nodes[nodes[i].index], &c1 = nodes[nodes[i].index + 1];

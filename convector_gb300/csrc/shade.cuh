@@ -289,7 +289,7 @@ __device__ __forceinline__ bool render_pixels(const DeviceScene& s, const Device
         // chosen once per bounce outside the traversal loop (room frame in
         // packet traversal 1.32 -> 1.21 ms; the same image).
         if (PACKET && s.slab_sel &&
-            oct_all(omask, select_form_ray(o, f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab)))))
+            oct_all(omask, select_form_recip(f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab)))))
             ok &= traverse<true, true>(s, o, d, active, omask, h, tab, nullptr);
         // A single-ray lane over the wide records, two per round with the leaf
         // they lead to tested after them (RefillRay::walk; three per round 650
@@ -313,7 +313,7 @@ __device__ __forceinline__ bool render_pixels(const DeviceScene& s, const Device
         // Likewise a single-ray lane whose reciprocals allow it (room frame in
         // octet groups 0.82 -> 0.74 ms, 256-scene batch 53.4 -> 51.9 ms).
         else if (!PACKET && active && s.slab_sel &&
-                 select_form_ray(o, f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab))))
+                 select_form_recip(f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab))))
             ok &= traverse<false, true>(s, o, d, active, __activemask(), h, tab, nullptr);
         else if (PACKET || active)
             ok &= traverse<PACKET>(s, o, d, active, PACKET ? omask : __activemask(), h, tab, nullptr);

@@ -52,7 +52,7 @@ __device__ __forceinline__ BoxT box_test(float lx, float ly, float lz, float hx,
 // the two plane distances (one select for each compare-and-select). It gives
 // the bits of box_test when every bound is finite, lo <= hi and no bound is -0
 // (DeviceScene::slab_sel), and the reciprocals are finite with |1/d| >= 0.75
-// (select_form_ray). With a positive reciprocal, rounding keeps
+// (select_form_recip). With a positive reciprocal, rounding keeps
 // (lo - o) / d <= (hi - o) / d; x86 min takes the first and max the second, and
 // on equal values the second, which then has the same bits: a zero difference
 // is +0 without -0 bounds, and a non-zero one does not round to a zero at
@@ -213,9 +213,14 @@ struct WideT {
     }
 };
 
-// Rays that may take the select form: reciprocals and origin as above, and
-// bounded (with the bounds, DeviceScene::slab_sel), so that no plane distance
-// overflows.
+// Rays that may take the select form on the pair records: reciprocals as at
+// box_test_sel.
+__device__ __forceinline__ bool select_form_recip(F3 inv) {
+    return isfinite(inv.x) && isfinite(inv.y) && isfinite(inv.z) && fabsf(inv.x) >= 0.75f &&
+           fabsf(inv.y) >= 0.75f && fabsf(inv.z) >= 0.75f;
+}
+// And on the wide records: reciprocals and origin bounded too (as the bounds are,
+// TreeFacts::wide), so that no plane distance overflows.
 __device__ __forceinline__ bool select_form_ray(F3 o, F3 inv) {
     auto in = [](float x) { return fabsf(x) >= 0.75f && fabsf(x) <= kSelectMax; };
     return in(inv.x) && in(inv.y) && in(inv.z) && fabsf(o.x) <= kSelectMax && fabsf(o.y) <= kSelectMax &&
@@ -284,7 +289,7 @@ struct Counters {
 // In SINGLE mode an inactive lane must not call this. Returns false on stack
 // overflow (the hit is then incomplete). SELECT: the select-form slab test
 // (box_test_sel), for a scene with DeviceScene::slab_sel and rays whose
-// reciprocals meet select_form_ray (in PACKET mode: all 8 lanes').
+// reciprocals meet select_form_recip (in PACKET mode: all 8 lanes').
 template <bool PACKET, bool SELECT = false>
 __device__ __forceinline__ bool traverse(const DeviceScene& s, F3 o, F3 d, bool active, unsigned omask, Hit& h,
                                          const ApproxTables& tab, Counters* cnt) {
@@ -375,11 +380,21 @@ __device__ __forceinline__ void cp_async_wait_one_pending() { asm volatile("cp.a
 // that ray's result itself).
 enum : int { kClaimNone = 0, kClaimRay = 1, kClaimDone = 2 };
 
+// How a refill traversal tests boxes: node pairs with the x86 slab test, node
+// pairs with the select form (for scenes with DeviceScene::slab_sel), or wide
+// records (for scenes that have them). The last two leave a ray that does not
+// meet select_form_recip or select_form_ray to the first.
+enum class Form { kX86, kPairs, kWide };
+template <Form FORM>
+__device__ __forceinline__ bool form_allows(F3 o, F3 inv) {
+    return FORM == Form::kWide ? select_form_ray(o, inv) : FORM == Form::kPairs ? select_form_recip(inv) : true;
+}
+
 struct RayIn {
     F3 o, d;
     float far;
     const float4* nodes;
-    const float4* wide;  // SELECT only
+    const float4* wide;  // Form::kWide only
     const float4* geom;
 };
 
@@ -456,8 +471,9 @@ struct RefillRay {
     //
     // Returns true when the ray is finished (its stack is empty): h is then
     // its nearest hit. Sets `overflow` (and finishes the ray) when the stack
-    // would overflow.
-    template <bool COUNT, bool LEAF_AFTER_PAIR, class Stack>
+    // would overflow. SELECT: the slab test in select form (box_test_sel; the
+    // scene and the ray must meet its conditions).
+    template <bool COUNT, bool LEAF_AFTER_PAIR, bool SELECT = false, class Stack>
     __device__ __forceinline__ bool step(Stack& stack, bool& overflow) {
         if (cur == kNone) {
             // Pop until an entry survives the cull test (aabb.rs:171-177).
@@ -489,8 +505,14 @@ struct RefillRay {
             // the child pair (64 bytes per pair).
             const float4* np = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(nodes) + cur);
             float4 q0 = __ldg(np), q1 = __ldg(np + 1), q2 = __ldg(np + 2), q3 = __ldg(np + 3);
-            const BoxT b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o(), inv);
-            const BoxT b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o(), inv);
+            BoxT b0, b1;
+            if constexpr (SELECT) {
+                b0 = box_test_sel(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o(), inv);
+                b1 = box_test_sel(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o(), inv);
+            } else {
+                b0 = box_test(q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, o(), inv);
+                b1 = box_test(q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, o(), inv);
+            }
             bool first0 = !sneg(b0.tmin - b1.tmin);
             bool hit0 = b0.mask & !sneg(b0.tmax);
             bool hit1 = b1.mask & !sneg(b1.tmax);
@@ -535,7 +557,7 @@ struct RefillRay {
     // runs once per round for all lanes that reached a leaf in it, not at nearly
     // every step for one or two lanes.
     //
-    // A wide record holds the boxes of a pair's four grandchildren (WidePair):
+    // A wide record holds the boxes of a pair's four grandchildren (WidePlanes):
     // one step does what step() does for the pair and for both its children.
     // The triangles tested and their order are those of step():
     //  * Bounds nest (checked at scene creation), and the differences, products,
@@ -750,15 +772,14 @@ __device__ __forceinline__ typename std::conditional<N == 0, LocalStack, SharedL
 // CLAIM_MIN: lanes without a ray wait until that many want one; results do
 // not depend on it (each ray's traversal is independent of when it starts).
 // Returns false if a ray overflowed the stack (its hit is then incomplete).
-// SELECT: every ray whose reciprocals meet select_form_ray is traversed with
-// the select-form slab test and postponed leaves (RefillRay::walk); the others
-// are handed to src.defer(r) untraced (the caller traces them afterwards with
-// the x86 form). STEPS: node pairs (SELECT) or traversal steps per round of the
-// warp's votes (a lane whose ray ends within a round waits for the next
-// round's claim).
-// POOL_LEAVES (with SELECT): a round's leaves are tested by the whole warp
+// FORM kWide: rays walk the wide records, with postponed leaves (RefillRay::
+// walk); kPairs: step() in the select form. A ray that the form does not allow is
+// handed to src.defer(r) untraced (the caller traces it afterwards in the x86
+// form). STEPS: wide records or traversal steps per round of the warp's votes (a
+// lane whose ray ends within a round waits for the next round's claim).
+// POOL_LEAVES (with kWide): a round's leaves are tested by the whole warp
 // (RefillRay::test_leaves).
-template <bool COUNT, bool LEAF_AFTER_PAIR, int CLAIM_MIN, int SHARED_STACK = 0, bool SELECT = false, int STEPS = 1,
+template <bool COUNT, bool LEAF_AFTER_PAIR, int CLAIM_MIN, int SHARED_STACK = 0, Form FORM = Form::kX86, int STEPS = 1,
           bool POOL_LEAVES = false, class Src, class Claim>
 __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, const ApproxTables& tab,
                                                 uint2* shared_stack = nullptr) {
@@ -797,8 +818,8 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
                     r_id = r;
                     ray.start(in.o, in.d, in.far, in.nodes, in.wide, in.geom, tab);
                     have = true;
-                    if constexpr (SELECT) {
-                        if (!select_form_ray(ray.no, ray.inv)) {
+                    if constexpr (FORM != Form::kX86) {
+                        if (!form_allows<FORM>(ray.no, ray.inv)) {
                             src.defer(r);
                             have = false;
                         }
@@ -809,7 +830,7 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
             }
         }
         if (__all_sync(0xffffffffu, done)) break;
-        if constexpr (SELECT) {
+        if constexpr (FORM == Form::kWide) {
             if (have) {
 #pragma unroll
                 for (int st = 0; st < STEPS; st++) ray.walk(stack, overflow);
@@ -823,7 +844,7 @@ __device__ __forceinline__ bool traverse_refill(const Src& src, Claim& claim, co
             }
         } else {
             for (int st = 0; st < STEPS && have; st++) {
-                if (ray.step<COUNT, LEAF_AFTER_PAIR>(stack, overflow)) {
+                if (ray.step<COUNT, LEAF_AFTER_PAIR, FORM == Form::kPairs>(stack, overflow)) {
                     src.store(r_id, ray.h, ray.na, ray.nt);
                     have = false;
                 }

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(128, 10) k_wf_traverse_single(const Job* __res
                                                             int bounce, WaveOutputs out) {
     QueueStore store{st};
     QueueClaim claim{jobs, scenes, st, st.queue[bounce & 1], st.counts[bounce] * 8u, &st.counts[6 + bounce]};
-    if (!traverse_refill<false, true, CLAIM, 0, false, kWaveTraverseSteps>(store, claim, g_tables_wf))
+    if (!traverse_refill<false, true, CLAIM, 0, Form::kX86, kWaveTraverseSteps>(store, claim, g_tables_wf))
         atomicOr(out.err, kErrStackOverflow);
 }
 
@@ -531,18 +531,43 @@ constexpr int kRefillWaveSteps = 2;
 // DEEP: a wave with a tree deeper than 40 levels: lanes wait for 12 to shade, and a
 // warp's leaves are tested together
 // (16 mixed requests 148.8 -> 139.8 ms; 144.1 with 8 lanes).
-template <bool DEEP, bool SLOTS = false>
+// FORM kX86: a wave none of whose scenes has wide records. Two steps per round;
+// deep waves wait for 8 lanes, keep the first 16 stack entries of each lane in
+// shared memory and read the tables from global memory. (In the kWide kernel such
+// scenes take the same steps, in more registers.)
+constexpr int kDeepWaveStackShared = 16;
+template <bool DEEP, Form FORM, bool SLOTS = false>
 __global__ void __launch_bounds__(128, kRefillWaveBlocksPerSm) k_wave_refill(const Job* __restrict__ jobs,
                                                                           const WaveHeader* __restrict__ hdr,
                                                                           const DeviceScene* __restrict__ scenes,
                                                                           WaveOutputs out) {
     WavePaths<SLOTS> P{jobs, scenes, out, hdr->n_jobs, hdr->n_groups, 0u, 0u};
-    __shared__ ApproxTables tab;
-    load_tables_wf(tab);
     bool ok;
-    if constexpr (DEEP) ok = path_refill<12, kRefillWaveSteps, false, true, true>(P, tab);
-    else ok = path_refill<16, kRefillWaveSteps, false, true>(P, tab);
+    if constexpr (FORM == Form::kX86 && DEEP) {
+        __shared__ uint2 sstack[4][kDeepWaveStackShared][32];
+        ok = path_refill<8, 2, false, FORM, false, kDeepWaveStackShared>(
+            P, g_tables_wf, &sstack[threadIdx.x >> 5][0][threadIdx.x & 31]);
+    } else {
+        __shared__ ApproxTables tab;
+        load_tables_wf(tab);
+        if constexpr (FORM == Form::kX86) ok = path_refill<16, 2, false, FORM>(P, tab);
+        else if constexpr (DEEP) ok = path_refill<12, kRefillWaveSteps, false, FORM, true>(P, tab);
+        else ok = path_refill<16, kRefillWaveSteps, false, FORM>(P, tab);
+    }
     if (!ok) atomicOr(out.err, kErrStackOverflow);
+}
+
+template <Form FORM>
+static void launch_wave_refill(const Job* jobs, const WaveHeader* hdr, const DeviceScene* scenes,
+                               const WaveOutputs& out, bool deep, cudaStream_t stream) {
+    const uint32_t grid = (uint32_t)sm_count() * kRefillWaveBlocksPerSm;
+    if (out.samples) {  // sample slots (several samples of an image share the wave)
+        if (deep) k_wave_refill<true, FORM, true><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
+        else k_wave_refill<false, FORM, true><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
+    } else {
+        if (deep) k_wave_refill<true, FORM><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
+        else k_wave_refill<false, FORM><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
+    }
 }
 
 // After k_wave_refill: the groups of the wave whose 8 lanes all hit an
@@ -564,18 +589,12 @@ __global__ void __launch_bounds__(256) k_wave_emitter_groups(const Job* __restri
 }
 
 cudaError_t launch_wave_fused(const Job* jobs, const WaveHeader* hdr, const DeviceScene* scenes,
-                              const WaveOutputs& out, bool packet, uint32_t blocks_per_sm, bool deep,
+                              const WaveOutputs& out, bool packet, uint32_t blocks_per_sm, bool deep, bool wide,
                               cudaStream_t stream) {
     if (!packet && out.group_em) {
-        uint32_t grid = (uint32_t)sms() * kRefillWaveBlocksPerSm;
-        if (out.samples) {  // sample slots: no gbuffer (several samples of an image share the wave)
-            if (out.gbuf) return cudaErrorInvalidValue;
-            if (deep) k_wave_refill<true, true><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
-            else k_wave_refill<false, true><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
-            return cudaGetLastError();
-        }
-        if (deep) k_wave_refill<true><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
-        else k_wave_refill<false><<<grid, 128, 0, stream>>>(jobs, hdr, scenes, out);
+        if (out.samples && out.gbuf) return cudaErrorInvalidValue;
+        if (wide) launch_wave_refill<Form::kWide>(jobs, hdr, scenes, out, deep, stream);
+        else launch_wave_refill<Form::kX86>(jobs, hdr, scenes, out, deep, stream);
         if (out.gbuf) k_wave_emitter_groups<<<(uint32_t)sms() * 4u, 256, 0, stream>>>(jobs, hdr, out);
         return cudaGetLastError();
     }

@@ -72,3 +72,17 @@ def test_stack_settings_agree(gpu, orc, bvh, stack, blocks):
     t, tri = scene.intersect_nearest(o, d, traversal=gpu.TRAVERSE_SINGLE)
     ot, otri = osc.intersect(o, d, mode=gpu.TRAVERSE_SINGLE)
     assert (tri == otri).all() and (t.view(np.uint32) == ot.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("n,traversal,kernel", [(20000, 0, "k_intersect_warp"), (50000, 0, "k_intersect_octets"),
+                                                (1 << 20, 0, "k_intersect_packets<6"),
+                                                (300000, 1, "k_intersect_refill<8, false, 16, (cvx::Form)1")])
+def test_kernels_of_a_scene_without_wide_records(gpu, n, traversal, kernel):
+    b = gpu.Bvh.build(scenes.spheres_and_boxes(3000, 5, obj=False)[0])
+    f = b.nodes.view(np.float32)
+    f[0:2, 0:3] -= np.float32(0.5)
+    f[0:2, 3:6] += np.float32(0.5)
+    scene = gpu.Scene(b)
+    o, d = scenes.random_rays(n, seed=1)
+    names = _kernels(lambda: scene.intersect_nearest(o, d, traversal=traversal))
+    assert any(kernel in k for k in names), names

@@ -79,6 +79,7 @@ def test_unreached_nodes_are_not_followed(check, built, index, length, bound):
 def test_forms(check, built):
     nodes, n, depth = built
     for at, value, want in ((0, -5.0, "select 1 wide 0"),            # a root wider than its children
+                            (0, -1.0e30, "select 1 wide 0"),         # beyond the wide records' bound
                             (0, 1.0e30, "select 0 wide 0"),          # lo above hi
                             (3, np.inf, "select 0 wide 0")):
         v = nodes.copy()
