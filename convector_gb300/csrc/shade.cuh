@@ -311,9 +311,11 @@ __device__ __forceinline__ bool render_pixels(const DeviceScene& s, const Device
             h = ray.h;
         }
         // Likewise a single-ray lane whose reciprocals allow it (room frame in
-        // octet groups 0.82 -> 0.74 ms, 256-scene batch 53.4 -> 51.9 ms).
+        // octet groups 0.82 -> 0.74 ms, 256-scene batch 53.4 -> 51.9 ms). The stricter
+        // condition of the wide records: select_form_recip alone costs frames with
+        // records 10 us at 320x184 by the registers.
         else if (!PACKET && active && s.slab_sel &&
-                 select_form_recip(f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab))))
+                 select_form_ray(o, f3(x_rcp(d.x, tab), x_rcp(d.y, tab), x_rcp(d.z, tab))))
             ok &= traverse<false, true>(s, o, d, active, __activemask(), h, tab, nullptr);
         else if (PACKET || active)
             ok &= traverse<PACKET>(s, o, d, active, PACKET ? omask : __activemask(), h, tab, nullptr);
