@@ -1,10 +1,12 @@
 // The device half of the C-ABI (include/convector_gpu.h): scene upload,
 // nearest-hit queries and frame rendering.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
+#include <cerrno>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -103,23 +105,19 @@ bool cvx::injected_allocation_failure() {
 
 void cvx::touch_pages(void* p, size_t bytes) {
     static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* c = static_cast<char*>(p);
+    for (size_t i = 0; i < bytes; i += page) c[i] = 0;
+    if (bytes) c[bytes - 1] = 0;
+}
+
+void cvx::populate_pages(void* p, size_t bytes) {
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14)
     if (bytes == 0) return;
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) cudaGetLastError();
-    else if (a.type != cudaMemoryTypeUnregistered) return;
-    unsigned char* const c = static_cast<unsigned char*>(p);
-    // A byte exchanged for itself: a store that changes nothing, even where another
-    // thread writes the same byte meanwhile. A zero is tried first, as a fresh page
-    // holds: read first, it would take two faults (display frame of 1280x736 101 -> 107
-    // us). Pages in use need the store too (without it the copies into them are slow:
-    // 32 batched images, 53 MB, 7.3 -> 14.1 ms).
-    auto touch = [](unsigned char* at) {
-        unsigned char v = 0;
-        if (!__atomic_compare_exchange_n(at, &v, (unsigned char)0, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED))
-            __atomic_compare_exchange_n(at, &v, v, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED);
-    };
-    for (size_t i = 0; i < bytes; i += page) touch(c + i);
-    touch(c + bytes - 1);
+    const uintptr_t from = (uintptr_t)p / page * page, to = ((uintptr_t)p + bytes + page - 1) / page * page;
+    const int err = errno;
+    madvise(reinterpret_cast<void*>(from), to - from, kPopulateWrite);  // where refused: only slower copies
+    errno = err;
 }
 
 struct cvx_scene {

@@ -418,7 +418,7 @@ extern "C" int32_t cvx_batch_render(cvx_batch* b, const cvx_view* views, uint32_
             int32_t st = b->fused.submit(jobs[0], out, b->stream2, false);
             if (!st) st = b->engine.submit(jobs[1], out, b->stream, false);
             for (uint32_t i = 0; i < n && !touched; i++)
-                if (rgba[i]) touch_pages(rgba[i], (size_t)views[i].width * views[i].height * 4);
+                if (rgba[i]) populate_pages(rgba[i], (size_t)views[i].width * views[i].height * 4);
             touched = true;
             int32_t st0 = b->fused.collect(b->stream2, &r[0], nullptr, &t[0]);
             int32_t st1 = b->engine.collect(b->stream, &r[1], nullptr, &t[1]);
@@ -839,7 +839,7 @@ struct cvx_server {
                         std::lock_guard<std::mutex> lk(mu);
                         wanted = !q->cancelled;
                     }
-                    if (wanted) touch_pages(q->host_rgba, q->npx * 4);
+                    if (wanted) populate_pages(q->host_rgba, q->npx * 4);
                 }
             }
             // Wait for an engine to finish, or for new work an idle engine could take.

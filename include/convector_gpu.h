@@ -10,7 +10,10 @@
  * Ownership and threading: the caller owns every host buffer it passes;
  * handles own their device memory. A handle must be used by one thread at a
  * time; distinct handles may be used concurrently. Calls that take host
- * buffers are synchronous. Nothing here falls back to the CPU: without a
+ * buffers are synchronous. A query, frame or display call that returns an error
+ * may have written its output buffers in part; a batch call or request that ends
+ * with CVX_ERR_DEVICE, or is cancelled, leaves its images as they were. Nothing here
+ * falls back to the CPU: without a
  * usable CUDA device the GPU entry points return CVX_ERR_CUDA.
  *
  * Devices: a scene or display belongs to the device current in the calling
