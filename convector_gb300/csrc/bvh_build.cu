@@ -1170,10 +1170,15 @@ struct Lists {
 int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     if (n == 0) return set_error(CVX_ERR_INVALID, "cannot build a BVH of zero triangles");
     if (n > kMaxTris) return set_error(CVX_ERR_CAPACITY, "device BVH build: more than 2^26 triangles");
+    std::vector<float> tx, tt;
+    float ty;
+    tsah_tables(n, tx, tt, &ty);
+    std::unique_ptr<cvx_bvh> bvh(new cvx_bvh());
     cudaStream_t st = nullptr;
     BK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
     // Host arrays of uploads in flight, kept until the stream has been waited for
-    // (the guard, which goes first, waits on every way out).
+    // (the guard, which goes before them and before what is declared above, waits on
+    // every way out).
     std::vector<std::shared_ptr<void>> keep;
     struct StreamGuard {
         cudaStream_t s;
@@ -1190,9 +1195,6 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
         return CVX_OK;
     };
 
-    std::vector<float> tx, tt;
-    float ty;
-    tsah_tables(n, tx, tt, &ty);
     const uint32_t max_nodes = 2 * n;
     const uint32_t max_slots = n / (kSmall + 1) + 1;
 
@@ -1474,12 +1476,14 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
                                        out_nodes, (float4*)out_tris, order_tmp, misc + 3,
                                        misc + 1);
     BK(cudaGetLastError(), "crystallize");
-    // The result's memory, while the kernels run.
-    std::unique_ptr<cvx_bvh> bvh(new cvx_bvh());
+    // The result's memory, while the kernels run. There are one (room, tube) to two
+    // (icosphere) nodes per triangle: room for the most there can be, which is not
+    // resident until it is used, and the pages of five for four triangles.
     bvh->nodes.reserve(max_nodes);
+    bvh->nodes.resize(std::min<size_t>(max_nodes, (size_t)n + n / 4));
     bvh->triangles.resize(n);
     bvh->source_index.resize(n);
-    touch_pages(bvh->nodes.data(), (size_t)max_nodes * sizeof(cvx_bvh_node));
+    touch_pages(bvh->nodes.data(), bvh->nodes.size() * sizeof(cvx_bvh_node));
     touch_pages(bvh->triangles.data(), (size_t)n * sizeof(cvx_triangle));
     touch_pages(bvh->source_index.data(), (size_t)n * 4);
     uint32_t flags[4], root_c0 = 0, root_inner = 0, root_tris = 0;
@@ -1490,9 +1494,9 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     BK(cudaMemcpyAsync(&root_tris, cr.tris, 4, cudaMemcpyDeviceToHost, st), "download");
     BK(cudaMemcpyAsync(&root_ratio, cr.ratio, 4, cudaMemcpyDeviceToHost, st), "download");
     BK(cudaStreamSynchronize(st), "crystallize");
-    next_id = flags[2];
     if (flags[1] & 8u) return set_error(CVX_ERR_DEVICE, "device BVH build: malformed interim tree");
     if (flags[1]) return set_error(CVX_ERR_DEVICE, "device BVH build: internal range check failed");
+    next_id = flags[2];
     if (next_id > max_nodes) return set_error(CVX_ERR_DEVICE, "device BVH build: node overflow");
     if (!root_c0)
         return set_error(CVX_ERR_INVALID,
@@ -1500,8 +1504,9 @@ int32_t bvh_build_device(const cvx_triangle* tris, uint32_t n, cvx_bvh** out) {
     if (root_tris != n) return set_error(CVX_ERR_DEVICE, "device BVH build lost triangles");
     if (2u * root_inner != next_id - 1u)
         return set_error(CVX_ERR_DEVICE, "device BVH build: unreachable interim nodes");
-    const size_t m = 2 * (size_t)root_inner;
+    const size_t m = 2 * (size_t)root_inner, touched = bvh->nodes.size();
     bvh->nodes.resize(m);
+    if (m > touched) touch_pages(bvh->nodes.data() + touched, (m - touched) * sizeof(cvx_bvh_node));
     BK(cudaMemcpyAsync(bvh->nodes.data(), out_nodes, m * sizeof(cvx_bvh_node), cudaMemcpyDeviceToHost, st),
        "download");
     BK(cudaMemcpyAsync(bvh->triangles.data(), out_tris, (size_t)n * sizeof(cvx_triangle), cudaMemcpyDeviceToHost,
