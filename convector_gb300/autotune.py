@@ -44,6 +44,8 @@ def candidates(rng_order=RNG_GROUP, allow_packet=True):
     travs = [TRAVERSE_SINGLE, TRAVERSE_PACKET] if allow_packet else [TRAVERSE_SINGLE]
     for trav in travs:
         for block in (64, 128):  # the fused kernels are compiled for at most 128 threads per block
+            if block == 64 and rng_order != RNG_GROUP and trav == TRAVERSE_PACKET:
+                continue  # four warps a patch, whatever the block size
             out.append(dict(rng_order=rng_order, traversal=trav, mode=MODE_MEGAKERNEL, block_size=block,
                             refill_mode=REFILL_NONE))
     if rng_order == RNG_GROUP:  # single launch with paths per lane (its block is fixed at 128)

@@ -1133,7 +1133,8 @@ cudaError_t launch_intersect(const DeviceScene& s, const RayCols& rays, uint32_t
     cudaError_t e = cudaMemsetAsync(err + 1, 0, 4, st);  // packet counter
     if (e != cudaSuccess) return e;
     if (!counters && (s.wide || n >= kPairPacketRays)) {
-        uint32_t blocks = (uint32_t)num_sms() * kPacketBlocksPerSm, need = (n + 127u) / 128u;
+        uint32_t blocks = (uint32_t)num_sms() * (blocks_per_sm ? blocks_per_sm : (uint32_t)kPacketBlocksPerSm),
+                 need = (n + 127u) / 128u;
         if (blocks > need) blocks = need;
         SoaRays src{s.nodes, s.wide, s.geom, rays, n, far_dist, t_out, tri_out, nullptr, s.slab_sel};
         if (!s.wide) k_intersect_packets<kPairPacketSteps, Form::kPairs><<<blocks, 128, 0, st>>>(src, err + 1, err);
@@ -1204,10 +1205,10 @@ cudaError_t launch_render(const DeviceScene& s, const DeviceCamera& cam, uint32_
         if (blocks > need) blocks = need;
         if (packet && !debug && packets_in_step(s, w * h)) {
             const bool deep = s.wide && s.depth > 40;
-            blocks = std::min((uint32_t)num_sms() * (deep ? 6u : 5u), (units * 8u + 127u) / 128u);
-            if (!s.wide) k_render_packets<false, Form::kPairs><<<blocks, 128, 0, st>>>(a);
-            else if (deep) k_render_packets<true, Form::kWide><<<blocks, 128, 0, st>>>(a);
-            else k_render_packets<false, Form::kWide><<<blocks, 128, 0, st>>>(a);
+            blocks = std::min((uint32_t)num_sms() * ((deep ? 6u : 5u) * 128u / block), need);
+            if (!s.wide) k_render_packets<false, Form::kPairs><<<blocks, block, 0, st>>>(a);
+            else if (deep) k_render_packets<true, Form::kWide><<<blocks, block, 0, st>>>(a);
+            else k_render_packets<false, Form::kWide><<<blocks, block, 0, st>>>(a);
         } else if (packet) k_render_group<true><<<blocks, block, 0, st>>>(a);
         else k_render_group<false><<<blocks, block, 0, st>>>(a);
     }

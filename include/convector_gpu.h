@@ -257,7 +257,8 @@ typedef struct cvx_render_config {
     uint32_t rng_order;     /* CVX_RNG_* */
     uint32_t traversal;     /* CVX_TRAVERSE_* */
     uint32_t mode;          /* CVX_MODE_* */
-    uint32_t block_size;    /* megakernel, octet groups: threads per block, 32, 64, 96 or 128 (0: 128) */
+    uint32_t block_size;    /* megakernel: threads per block, 32, 64, 96 or 128 (0: 128), where octets hold
+                               groups or patches; paths per lane and packets in the patch order take 128 */
     uint32_t use_graph;     /* wavefront: capture the bounce loop in a CUDA graph */
     uint32_t blocks_per_sm; /* wavefront: persistent blocks per SM (0: 12) */
     uint32_t refill_mode;   /* CVX_REFILL_* */

@@ -86,3 +86,56 @@ def test_kernels_of_a_scene_without_wide_records(gpu, n, traversal, kernel):
     o, d = scenes.random_rays(n, seed=1)
     names = _kernels(lambda: scene.intersect_nearest(o, d, traversal=traversal))
     assert any(kernel in k for k in names), names
+
+
+def _shapes(call, tmp_path, kernel):
+    """(grid, block) of the launches of `kernel` during the call."""
+    import json
+    import torch
+    call()
+    for _ in range(3):
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+            call()
+            torch.cuda.synchronize()
+        p.export_chrome_trace(str(tmp_path / "trace.json"))
+        with open(tmp_path / "trace.json") as f:
+            events = json.load(f)["traceEvents"]
+        found = [(e["args"]["grid"][0], e["args"]["block"][0]) for e in events
+                 if kernel in e.get("name", "") and "grid" in e.get("args", {})]
+        if found:
+            return found
+    pytest.skip("no activity records")
+
+
+def test_launch_shape_of_packet_queries(gpu, bvh, tmp_path):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    scene = gpu.Scene(bvh)
+    o, d = scenes.random_rays(300000, seed=1)
+    t, tri = scene.intersect_nearest(o, d)
+    for blocks in (4, 10):
+        scene.set_query_launch(blocks)
+        shapes = _shapes(lambda: scene.intersect_nearest(o, d), tmp_path, "k_intersect_packets")
+        assert shapes == [(blocks * sms, 128)], shapes
+        t2, tri2 = scene.intersect_nearest(o, d)
+        assert (tri == tri2).all() and (t.view(np.uint32) == t2.view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("block", [32, 64, 96, 128])
+def test_block_size_of_packet_frames(gpu, bvh, tmp_path, block):
+    scene = gpu.Scene(bvh)
+    scenes.default_camera(scene.camera)
+    w, h = 333, 181
+    ref = gpu.Renderer(scene, w, h, rng_order=gpu.RNG_GROUP, traversal=gpu.TRAVERSE_PACKET).render_frame_u8(3)
+    r = gpu.Renderer(scene, w, h, rng_order=gpu.RNG_GROUP, traversal=gpu.TRAVERSE_PACKET, block_size=block)
+    out = r.render_frame_u8(3)
+    assert (out[0] == ref[0]).all() and (out[1] == ref[1]).all()
+    shapes = _shapes(lambda: r.render_frame_u8(3), tmp_path, "k_render_packets")
+    assert [b for _, b in shapes] == [block], shapes
+
+
+def test_autotuner_times_each_launch_once(gpu):
+    from convector_gb300 import autotune
+    for order in (gpu.RNG_PATCH, gpu.RNG_GROUP):
+        packets = [c for c in autotune.candidates(order) if c["traversal"] == gpu.TRAVERSE_PACKET and "block_size" in c]
+        assert len(packets) == (1 if order == gpu.RNG_PATCH else 2)
