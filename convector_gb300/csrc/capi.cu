@@ -731,7 +731,7 @@ int32_t cvx_renderer_set_debug_view(cvx_renderer* r, uint32_t enable) {
 }
 
 // The listed patches with the reference's per-patch generator, in one launch
-// (one octet per patch); only the patches' pixels are copied to the caller's
+// (four warps a patch in packet traversal, else an octet); only the patches' pixels are copied to the caller's
 // full-frame buffers.
 static int32_t run_patches(cvx_renderer* r, uint32_t pw, const uint32_t* xy, uint32_t n, uint32_t frame,
                            bool accumulate, uint32_t* rgba, uint32_t* gbuf) {
@@ -815,11 +815,11 @@ int32_t cvx_accumulate_frame_f32(cvx_renderer* r, uint32_t frame, uint32_t* gbuf
 
 // Frames per launch of cvx_accumulate_frames_f32. The paths of up to
 // kMaxLaunchFrames frames share one path-refill launch, so the launch's drain
-// (lanes running out of paths while the last ones finish: 1.1 of 2.9 ms of a
+// (lanes running out of paths while the last ones finish: 0.65 of 1.98 ms of a
 // one-frame launch on the 870k-triangle tube) is paid once per launch instead
-// of once per frame. Measured per 1280x736 tube sample at 1, 2, 4, 8, 16
-// frames per launch: 2.94, 2.61, 2.40, 2.30, 2.25 ms (room: 0.709, 0.650,
-// 0.614, 0.596, 0.588 ms), about 2.20 + 0.82 / frames. The colour buffers of
+// of once per frame. Measured per 1280x736 tube sample at 1, 2, 4, 8, 16, 32
+// frames per launch: 1.98, 1.64, 1.48, 1.40, 1.36, 1.34 ms (room: 0.491, 0.444,
+// 0.418, 0.404, 0.397, 0.393 ms), about 1.32 + 0.65 / frames. The colour buffers of
 // all frames of a launch but the last take at most kSampleBufferBytes.
 constexpr uint32_t kMaxLaunchFrames = 32;
 constexpr size_t kSampleBufferBytes = (size_t)512 << 20;
@@ -836,8 +836,8 @@ int32_t cvx_accumulate_frames_f32(cvx_renderer* r, uint32_t first_frame, uint32_
     per_launch = (uint32_t)std::min<uint64_t>(per_launch, (1ull << 31) / paths);  // 32-bit path numbers
     // Shared launches use the path-refill kernel whatever the refill mode: its
     // frames have the bits of the octet-group kernel's, and with the drain
-    // shared it is the faster form on every scene measured (room 0.588 against
-    // 0.744 ms per 1280x736 sample for one octet per group).
+    // shared it is the faster form on every scene measured (room 0.393 against
+    // 0.66 ms per 1280x736 sample for one octet per group).
     const bool shared_launch = !r->engine && !r->debug && r->cfg.traversal == CVX_TRAVERSE_SINGLE &&
                                r->cfg.rng_order == CVX_RNG_GROUP && per_launch > 1;
     if (!shared_launch) {  // one launch per frame

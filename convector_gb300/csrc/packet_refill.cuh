@@ -158,9 +158,8 @@ struct PacketRay {
 
     // The boxes to visit, from the last to the first: each becomes the next
     // node, and the one before it is pushed, by selects (as branches, frames: room
-    // 1.127 -> 1.119 ms, icosphere 2.76 -> 2.72, 320x184 of it 0.57 -> 0.53; a push that
-    // may go to shared memory is better as a branch). Then a leaf goes to wait, if
-    // none does.
+    // 1.127 -> 1.119 ms, icosphere 2.76 -> 2.72, 320x184 of it 0.57 -> 0.53). Then a
+    // leaf goes to wait, if none does.
     template <int N, class Stack>
     __device__ __forceinline__ void push(const bool (&v)[N], const uint32_t (&r)[N], const float (&t)[N], Stack& stack,
                                          bool& overflow) {

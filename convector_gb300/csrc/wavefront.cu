@@ -341,8 +341,8 @@ cudaError_t set_stack_limit_wave(int entries) {
 // wavefront kernels. A group's samples (Job::more) follow one another on its octet,
 // so each pixel's are added in their order.
 template <bool PACKET>
-// 8 resident blocks per SM (64 registers, small spill): batches of small
-// scenes render 12 % faster than at the compiler's 80 registers (6 blocks).
+// 8 resident blocks per SM (64 registers; 212 bytes of spill stores and 244 of loads,
+// 116 each for packets): 5 to 8 blocks 6.13-6.18 ms for 32 open scenes.
 __global__ void __launch_bounds__(128, 8) k_wave_fused(const Job* __restrict__ jobs, const WaveHeader* __restrict__ hdr,
                                                     const DeviceScene* __restrict__ scenes, WaveOutputs out) {
     __shared__ ApproxTables tab;
@@ -517,20 +517,19 @@ struct WavePaths {
 
 // A fused wave in per-lane path refill form (path_refill); launch shape and
 // loop form as the frame kernel's (k_render_refill).
-// 7 resident blocks per SM (72 registers and a small spill): 6 (80 registers,
-// no spill) served the 415-request mix at 2,014 against 2,083 Mrays/s.
-// With postponed leaves (below) again: 6 blocks 2,744 against 2,869 Mrays/s.
+// 7 resident blocks per SM (72 registers; 120 bytes of spill stores and 92 of loads):
+// 6 served the 415-request mix at 2,744 against 2,869 Mrays/s.
 constexpr int kRefillWaveBlocksPerSm = 7;
 // Wide records a lane walks per round (RefillRay::walk), whose leaves are tested
 // once at its end. Five node pairs per round against x86-form rounds of two
 // steps, a served 1280x736 request of 16 samples: room 11.2 -> 9.5 ms, 82k
-// icosphere 20.7 -> 17.3 ms, 870k tube 38.2 -> 31.4 ms, although the spill grows
-// from 82-94 to 112-120 bytes. Records instead of pairs, 16 mixed requests: 159
-// -> 149 ms (three and four per round 147, 153).
+// icosphere 20.7 -> 17.3 ms, 870k tube 38.2 -> 31.4 ms. Two records as in the frame
+// kernel of the same loop: 16 mixed requests do not resolve the choice, as one state
+// gives 99 to 109 ms from process to process (one record 109-111, three 92-98).
 constexpr int kRefillWaveSteps = 2;
 // DEEP: a wave with a tree deeper than 40 levels: lanes wait for 12 to shade, and a
-// warp's leaves are tested together
-// (16 mixed requests 148.8 -> 139.8 ms; 144.1 with 8 lanes).
+// warp's leaves are tested together, as in the frame kernel (mixed requests: 8 lanes
+// 118-127 ms, 12 99-109, 16 105-117).
 // FORM kX86: a wave none of whose scenes has wide records. Two steps per round;
 // deep waves wait for 8 lanes, keep the first 16 stack entries of each lane in
 // shared memory and read the tables from global memory. (In the kWide kernel such

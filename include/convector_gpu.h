@@ -161,10 +161,11 @@ uint32_t cvx_scene_num_direct_samples(const cvx_scene* scene);
  * triangles); 1 (default): `(bits * n) >> 32`, identical to it when n == 8. */
 int32_t cvx_scene_set_light_pick(cvx_scene* scene, uint32_t light_pick);
 /* Launch shape of this scene's nearest-hit queries: resident 128-thread
- * blocks per SM (0: default 8; the single-ray kernel is built for 8, 10 and
- * 12, trading registers for occupancy). While it is not set, queries of up to
- * 262,144 rays run without resident blocks, one packet per warp or one ray per
- * lane. Results do not depend on it. */
+ * blocks per SM (0: default, 8 for single rays and 7 for packets; the single-ray
+ * kernel over wide records is built for 8, 10 and 12, trading registers for
+ * occupancy). While it is not set, small queries (up to 262,144 rays) run without
+ * resident blocks, one packet per warp or one ray per lane. Results do not depend
+ * on it. */
 int32_t cvx_scene_set_query_launch(cvx_scene* scene, uint32_t blocks_per_sm);
 /* Stack depth of this scene's single-ray nearest-hit queries at 8 resident
  * blocks per SM: how many of each lane's traversal stack entries are kept in
@@ -343,9 +344,9 @@ int32_t cvx_renderer_stats(cvx_renderer* r, uint64_t* rays, float* ms);
 int32_t cvx_renderer_count_work(cvx_renderer* r, uint32_t frame_number, uint64_t* out);
 
 /* ---- device: batched rendering -----------------------------------------
- * Many images of many resident scenes in shared wavefronts: sample s of
- * every view goes into wave s, so each view accumulates its samples in order
- * and its image equals the one cvx_accumulate_frame_f32 + cvx_resolve_u8
+ * Many images of many resident scenes in shared wavefronts: every wave holds
+ * the next sample of each view (in the octet form, up to 16 of them), so each view
+ * accumulates its samples in order and its image equals the one cvx_accumulate_frame_f32 + cvx_resolve_u8
  * give for it alone. No reference counterpart: the reference renders one
  * frame of one scene (main.rs:124-217). */
 typedef struct cvx_view {
